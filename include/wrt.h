@@ -58,10 +58,12 @@ typedef enum wrt_sampler {
 } wrt_sampler;
 
 typedef enum wrt_kernel {
-  WRT_KERNEL_AUTO = 0,   /* the staged kernel (both samplers; volumes of edge >= 4),
+  WRT_KERNEL_AUTO = 0,   /* the staged kernels (both samplers; volumes of edge >= 4),
                             else the plain one */
   WRT_KERNEL_PLAIN = 1,  /* one warp per plane, gathers through L1 */
-  WRT_KERNEL_STAGED = 2  /* volume layers staged in shared memory, persistent CTAs:
+  WRT_KERNEL_STAGED = 2  /* the row-sum profiles where they cover and suit the request
+                            (working memory of up to ~750 MB in the context), else
+                            volume layers staged in shared memory, persistent CTAs:
                             trilinear from the layer pairs (FP32 or BF16 storage),
                             nearest from the z-major cell layers (FP32 storage) */
 } wrt_kernel;
@@ -293,7 +295,8 @@ typedef struct wrt_forward_req {
  * of all requests are ordered by cost and shared by all SMs.  The launch
  * sequence (table upload, output reset, request set-up, plane kernel,
  * finalize) is a CUDA graph captured once per context and replayed with a new
- * request table.  Asynchronous on the context's stream.  Each result is
+ * request table; requests that suit the row-sum profiles share the launches of
+ * those instead.  Asynchronous on the context's stream.  Each result is
  * bitwise identical to what wrt_radon_forward_device gives for the same
  * request alone.  Batch transforms of the reference's loop nest
  * radon_grid/src/radon_grid.c:229-264, one per request. */
@@ -311,7 +314,9 @@ void *wrt_ctx_stream(wrt_ctx *ctx);
 int wrt_tune_plane_kernel(wrt_ctx *ctx, const wrt_volume *vol, const wrt_grid *grid,
                           const wrt_plane_opts *opts, double *dev_out, int *best,
                           float *best_ms);
-/* Number of tile configurations; their shapes; force one (-1: default). */
+/* Number of tile configurations; their shapes; force one (-1: default, the
+ * row-sum profiles or the staged kernel's default tile by the request's sizes).
+ * The last one is the row-sum profiles, for every request they cover. */
 int wrt_plane_kernel_config_count(void);
 int wrt_plane_kernel_config_describe(int index, int *threads, int *rows_per_group,
                                      int *shifts_per_lane);

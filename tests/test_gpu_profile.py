@@ -1,0 +1,76 @@
+"""Plane integrals by the row-sum profiles (csrc/k_profile.cu) against the FP64
+oracle, at the sizes where their rules change: the smallest edge, odd and even
+edges (a sample line on a cell boundary for phis on an axis), edges around the
+one from which phi and phi + pi share tables, phis on and off the axes, one
+latitude (every row of a plane at one t), lattices that end inside the cube,
+volumes that reach its faces, several units of t and groups of layers."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import rel_l2, rel_max, wrt
+from wrt_b200.phantom import ellipsoid_phantom
+
+pytestmark = pytest.mark.gpu
+
+# the FP32 tolerance of every plane kernel's parity test
+TOL_L2, TOL_MAX = 1e-5, 1e-4
+
+CASES = [  # n, (nphi, ntheta, nshift), L, volume
+    (8, (8, 4, 9), 8, "noise"), (9, (6, 3, 33), 18, "noise"),
+    (9, (4, 1, 5), 9, "noise"), (24, (7, 5, 31), 24, "noise"),
+    (33, (12, 5, 40), 33, "phantom"), (39, (8, 3, 32), 39, "noise"),
+    (40, (8, 3, 32), 40, "noise"), (41, (10, 3, 21), 41, "phantom"),
+    (41, (8, 5, 21), 20, "noise"), (64, (6, 4, 65), 128, "noise"),
+    (65, (8, 3, 17), 65, "phantom"), (97, (4, 2, 9), 97, "noise"),
+]
+
+
+def _volume(kind, n):
+    if kind == "phantom":
+        return ellipsoid_phantom(n, 8, 100 + n)
+    return np.random.default_rng(n).standard_normal((n, n, n)).astype(np.float32).astype(np.float64)
+
+
+@pytest.fixture()
+def profiles(ctx):
+    wrt.set_plane_kernel_config(ctx, len(wrt.plane_kernel_configs()) - 1)
+    yield ctx
+    wrt.set_plane_kernel_config(ctx, -1)
+
+
+@pytest.mark.parametrize("sampler", [O.TRILINEAR, O.NEAREST])
+@pytest.mark.parametrize("n,grid,L,kind", CASES)
+def test_matches_oracle(profiles, n, grid, L, kind, sampler):
+    vol = _volume(kind, n)
+    got = profiles.radon_grid(vol, *grid, sampler=sampler, half_extent=L)
+    ref = O.radon_forward(vol, *grid, sampler=sampler, half_extent=L)
+    assert rel_l2(got, ref) < TOL_L2
+    assert rel_max(got, ref) < TOL_MAX
+    again = profiles.radon_grid(vol, *grid, sampler=sampler, half_extent=L)
+    assert np.array_equal(got, again)
+
+
+def test_batch_and_bf16_equal_alone(profiles):
+    reqs, keep = [], []
+    for k, (n, grid, L, kind) in enumerate(CASES[4:9]):
+        v = wrt.Volume(profiles, n, storage=wrt.STORAGE_BF16 if k % 2 else wrt.STORAGE_F32)
+        v.upload(_volume(kind, n))
+        g = wrt.Grid(profiles, *grid)
+        out = wrt.DeviceBuffer(profiles, g.nplanes * 8)
+        keep.append((v, g, out, L))
+        reqs.append((v, g, out.ptr, L))
+    wrt.radon_forward_batch(profiles, reqs)
+    profiles.synchronize()
+    batched = [out.download(np.empty(g.nplanes)) for (_, g, out, _) in keep]
+    for (v, g, out, L), got in zip(keep, batched):
+        wrt.radon_forward_device(profiles, v, g, out.ptr, half_extent=L)
+        assert np.array_equal(got, out.download(np.empty(g.nplanes)))
+
+
+def test_tight_budget_takes_the_staged_kernel():
+    vol = ellipsoid_phantom(48, 8, 5)
+    with wrt.Context(0, budget_bytes=12 << 20) as c:
+        got = c.radon_grid(vol, 32, 16, 64, sampler=wrt.TRILINEAR, half_extent=48)
+    ref = O.radon_forward(vol, 32, 16, 64, sampler=O.TRILINEAR, half_extent=48)
+    assert rel_l2(got, ref) < TOL_L2

@@ -12,6 +12,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
 #include <new>
 #include <vector>
 
@@ -279,6 +280,7 @@ int wrt_ctx_destroy(wrt_ctx *ctx) {
   if (ctx->dropin_vol) wrt_volume_destroy(ctx->dropin_vol);
   if (ctx->dropin_grid) wrt_grid_destroy(ctx->dropin_grid);
   laplace_release(ctx);
+  profile_lanes_release(&ctx->prof_lanes);
   for (int r = 0; r < WS_ROLES; ++r) ctx_free(ctx, ctx->ws[r], ctx->ws_bytes[r]);
   pinned_release(ctx);
   host_pool_destroy(ctx->host_pool);
@@ -649,8 +651,11 @@ namespace {
 
 // Staged-kernel launch of one request; see k_staged.cu.  Trilinear: the
 // volume's layer pairs; nearest: its z-major cell layers (FP32 storage).
+// phis / nphis: the planes of these phis only (the others are zeroed), all
+// when nphis is 0.
 int radon_forward_staged(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, int L,
-                         double *dev_out, bool nearest) {
+                         double *dev_out, bool nearest, const int *phis = nullptr,
+                         int nphis = 0) {
   int st = nearest ? volume_ensure_layers(vol) : volume_ensure_pairs(vol);
   if (st) return st;
   const int n = vol->n;
@@ -682,7 +687,8 @@ int radon_forward_staged(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, in
   StagedItem *d_items = nullptr;
   const int *d_nitems = nullptr;
   int nitems = 0;
-  st = staged_items_cached(ctx, n, th, r.crop_r2, r.ndir, &d_items, &d_nitems, &nitems, nearest);
+  st = staged_items_cached(ctx, n, th, r.crop_r2, r.ndir, &d_items, &d_nitems, &nitems, nearest,
+                           phis, nphis, grid->ntheta);
   if (st) return st;
   st = staged_scratch(ctx, sizeof(StagedReq));
   if (st) return st;
@@ -698,7 +704,73 @@ int radon_forward_staged(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, in
     if (st) return st;
   }
   const double delta = 1.0 / n;
+  if (nphis)
+    return plane_finalize_phis(ctx, dev_out, phis, nphis, grid->nphi, grid->ntheta, grid->nshift,
+                               delta * delta / r.scale);
   return plane_finalize(ctx, dev_out, (long long)nout, delta * delta / r.scale);
+}
+
+ProfReq profile_request(const wrt_ctx *ctx, const wrt_volume *vol, const wrt_grid *grid, int L,
+                        bool nearest, double *out) {
+  ProfReq r = {};
+  r.vol = vol->storage == WRT_STORAGE_BF16 ? (const void *)vol->d_vol16 : (const void *)vol->d_vol;
+  r.dir = grid->d_dir;
+  r.shift = grid->d_shift;
+  r.stats = vol->d_stats;
+  r.out = out;
+  r.counter = ctx->d_counter;
+  r.n = vol->n;
+  r.L = L;
+  r.nphi = grid->nphi;
+  r.ntheta = grid->ntheta;
+  r.nshift = grid->nshift;
+  r.storage = vol->storage;
+  r.nearest = nearest ? 1 : 0;
+  r.paired = profile_paired(vol->n, grid->nphi, L);
+  return r;
+}
+
+// The profiles' working memory of these requests in the context's workspace:
+// what they ask for, or the least that serves them; an error (cleared) when
+// the context's budget or the device holds neither.
+int profile_ws(wrt_ctx *ctx, const ProfReq *reqs, const float *crop, int nreq, void **ws,
+               size_t *bytes) {
+  const size_t want = profile_workspace_want(reqs, crop, nreq);
+  size_t least = 0;
+  for (int q = 0; q < nreq; ++q)
+    least = std::max(least, profile_workspace_least(reqs[q], crop[q]));
+  int st = ws_get(ctx, WS_PROFILE, want, ws);
+  if (st) st = ws_get(ctx, WS_PROFILE, least, ws);
+  if (st) {
+    ctx->err[0] = 0;
+    return st;
+  }
+  *bytes = std::min(want, ctx->ws_bytes[WS_PROFILE]);
+  return WRT_OK;
+}
+
+int radon_forward_profile(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, int L,
+                          double *dev_out, bool nearest, bool *done) {
+  const ProfReq r = profile_request(ctx, vol, grid, L, nearest, dev_out);
+  const float crop = nearest ? nearest_crop_r2(vol->r2, vol->n) : trilinear_crop_r2(vol->r2, vol->n);
+  void *ws = nullptr;
+  size_t bytes = 0;
+  *done = false;
+  if (profile_ws(ctx, &r, &crop, 1, &ws, &bytes)) return WRT_OK;  // no room: the staged kernel
+  *done = true;
+  if (nearest) {
+    // phis on an axis: half of every row's samples lie on a cell boundary for
+    // every t, so no table serves them
+    int phis[4], m = 0;
+    for (int p = 0; p < grid->nphi; ++p)
+      if ((fabs(cos(grid->phi[p])) < 1e-9 || fabs(sin(grid->phi[p])) < 1e-9) && m < 4)
+        phis[m++] = p;
+    if (m) {
+      int st = radon_forward_staged(ctx, vol, grid, L, dev_out, true, phis, m);
+      if (st) return st;
+    }
+  }
+  return profile_forward(ctx, ctx->stream, &ctx->prof_lanes, &r, &crop, 1, ws, bytes);
 }
 
 }  // namespace
@@ -726,8 +798,14 @@ int wrt_radon_forward_device(wrt_ctx *ctx, const wrt_volume *cvol, const wrt_gri
                 "BF16 volumes are sampled by the staged kernel (trilinear sampler) only");
   if (o.kernel == WRT_KERNEL_STAGED && !staged_ok)
     return fail(ctx, WRT_ERR_INVALID_ARGUMENT, "staged kernel: volume edge below 4");
-  if (o.kernel != WRT_KERNEL_PLAIN && staged_ok)
+  if (o.kernel != WRT_KERNEL_PLAIN && staged_ok) {
+    if (profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift, nearest)) {
+      bool done = false;
+      st = radon_forward_profile(ctx, vol, grid, L, dev_out, nearest, &done);
+      if (st || done) return st;
+    }
     return radon_forward_staged(ctx, vol, grid, L, dev_out, nearest);
+  }
   PlaneJob job = {};
   job.vol = vol->d_vol;
   job.n = vol->n;
@@ -752,7 +830,33 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
   if (st) return st;
   if (nreq == 0) return WRT_OK;
   BatchBuilder b;
+  // requests for the row-sum profiles, FP32 and BF16 volumes together
+  std::vector<ProfReq> prof;
+  std::vector<float> prof_crop;
+  std::vector<char> routed(nreq, 0);
   for (int r = 0; r < nreq; ++r) {
+    const wrt_volume *vol = reqs[r].volume;
+    const wrt_grid *grid = reqs[r].grid;
+    int th = 0, qp = 0;
+    if (!vol || !grid || !reqs[r].dev_out || vol->ctx != ctx || grid->ctx != ctx || vol->n < 4 ||
+        staged_smem_bytes(vol->n, &th, &qp) <= 0 || reqs[r].half_extent < 0 ||
+        reqs[r].half_extent > 8 * vol->n)
+      continue;  // refused below
+    const int L = reqs[r].half_extent ? reqs[r].half_extent : 2 * vol->n;
+    if (!profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift, false)) continue;
+    routed[r] = 1;
+    prof.push_back(profile_request(ctx, vol, grid, L, false, reqs[r].dev_out));
+    prof_crop.push_back(trilinear_crop_r2(vol->r2, vol->n));
+  }
+  void *prof_ws = nullptr;
+  size_t prof_bytes = 0;
+  if (!prof.empty() && profile_ws(ctx, prof.data(), prof_crop.data(), (int)prof.size(), &prof_ws,
+                                  &prof_bytes)) {
+    prof.clear();
+    std::fill(routed.begin(), routed.end(), 0);
+  }
+  for (int r = 0; r < nreq; ++r) {
+    if (routed[r]) continue;
     wrt_volume *vol = const_cast<wrt_volume *>(reqs[r].volume);
     const wrt_grid *grid = reqs[r].grid;
     if (!vol || !grid || !reqs[r].dev_out || vol->ctx != ctx || grid->ctx != ctx)
@@ -782,6 +886,11 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
     a.L = L;
     a.prep = 0;
     batch_add_forward(b, q, a, trilinear_crop_r2(vol->r2, n));
+  }
+  if (!prof.empty()) {
+    st = profile_forward(ctx, ctx->stream, &ctx->prof_lanes, prof.data(), prof_crop.data(),
+                         (int)prof.size(), prof_ws, prof_bytes);
+    if (st || b.fwd.empty()) return st;
   }
   if (!ctx->batch_slot) {
     BatchSlot *s = new (std::nothrow) BatchSlot();

@@ -120,6 +120,7 @@ __global__ void batch_volume_kernel(char *t) {
       if (amax > 0.0f) atomicMax(A[r].stats + 1, __float_as_uint(amax));
     }
     float2 *pairs = A[r].pairs;
+    if (!pairs) continue;  // statistics only
     const long long npairs = (long long)(n - 1) * n * pitch;
     for (long long k = tid; k < npairs; k += nth) {
       const int ix = (int)(k % pitch), iy = (int)((k / pitch) % n),
@@ -435,6 +436,14 @@ int batch_slot_launch(BatchSlot *s, BatchBuilder &b) {
   if (e != cudaSuccess) return cuda_fail(ctx, e, "batch event");
   s->launched = true;
   ctx->launches += kBatchKernels;
+  // the plane transforms by row-sum profiles (their volumes' statistics are
+  // the graph's work; the host does not know the support yet)
+  if (!b.prof.empty()) {
+    const std::vector<float> crop(b.prof.size(), 3.0f + 1e-5f);
+    st = profile_forward(ctx, s->stream, &s->prof_lanes, b.prof.data(), crop.data(),
+                         (int)b.prof.size(), s->prof_ws, s->prof_bytes);
+    if (st) return st;
+  }
   // the backprojections, behind the graph (which built their spline lines):
   // their direction constants travel as launch parameters
   for (const AdjReq &j : b.adj) {
@@ -448,6 +457,8 @@ void batch_slot_release(BatchSlot *s) {
   if (!s->ctx) return;
   if (s->launched) cudaEventSynchronize(s->done);
   drop_graph(s);
+  ctx_free(s->ctx, s->prof_ws, s->prof_bytes);
+  profile_lanes_release(&s->prof_lanes);
   if (s->h_table) cudaFreeHost(s->h_table);
   ctx_free(s->ctx, s->d_table, s->cap);
   ctx_free(s->ctx, s->d_next, sizeof(int));

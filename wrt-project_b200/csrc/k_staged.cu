@@ -726,6 +726,18 @@ __global__ void plane_finalize_kernel(double *out, long long count, double facto
   }
 }
 
+__global__ void plane_finalize_phis_kernel(double *out, int4 phis, int nphis, int nphi, int ntheta,
+                                           int nshift, double factor) {
+  const int per = nphis * ntheta;
+  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < (long long)nshift * per;
+       k += (long long)gridDim.x * blockDim.x) {
+    const int r = (int)(k % per), p = r / ntheta;
+    const int ip = p == 0 ? phis.x : p == 1 ? phis.y : p == 2 ? phis.z : phis.w;
+    const long long o = (k / per * nphi + ip) * ntheta + r % ntheta;
+    out[o] = (double)reinterpret_cast<const long long *>(out)[o] * factor;
+  }
+}
+
 }  // namespace
 
 namespace wrt {
@@ -781,13 +793,16 @@ int launch_cfg(wrt_ctx *ctx, cudaStream_t stream, const StagedReq *d_reqs,
 // was the fastest at 96^3, 128^3 and 256^3 on B200.
 const StagedConfig kStagedConfigs[] = {
     {1024, 8, 2}, {768, 8, 2}, {768, 4, 2}, {1024, 4, 2}, {768, 2, 2}, {1024, 1, 2}, {512, 8, 4},
+    // the row-sum profiles (k_profile.cu) where they cover the request, else the
+    // default tile: one row at a time per lane, lanes on shifts
+    {256, 32, 1},
 };
 const int kNumStagedConfigs = sizeof(kStagedConfigs) / sizeof(kStagedConfigs[0]);
 
 int plane_staged_launch(wrt_ctx *ctx, cudaStream_t stream, const StagedReq *d_reqs,
                         const StagedItem *d_items, const int *d_nitems, int max_smem,
                         int *d_next) {
-  const int c = (ctx->staged_config >= 0 && ctx->staged_config < kNumStagedConfigs)
+  const int c = (ctx->staged_config >= 0 && ctx->staged_config < kNumStagedConfigs - 1)
                     ? ctx->staged_config : 0;
   switch (c) {
     case 0: return launch_cfg<1024, 8, 2>(ctx, stream, d_reqs, d_items, d_nitems, max_smem, d_next);
@@ -811,6 +826,16 @@ int plane_finalize(wrt_ctx *ctx, double *out, long long count, double factor) {
   plane_finalize_kernel<<<blocks, 256, 0, ctx->stream>>>(out, count, factor);
   ctx->launches++;
   return check_launch(ctx, "plane_finalize_kernel");
+}
+
+int plane_finalize_phis(wrt_ctx *ctx, double *out, const int *phis, int nphis, int nphi,
+                        int ntheta, int nshift, double factor) {
+  const int4 p = make_int4(phis[0], phis[nphis > 1 ? 1 : 0], phis[nphis > 2 ? 2 : 0],
+                           phis[nphis > 3 ? 3 : 0]);
+  plane_finalize_phis_kernel<<<ctx->sm_count * 2, 256, 0, ctx->stream>>>(out, p, nphis, nphi,
+                                                                         ntheta, nshift, factor);
+  ctx->launches++;
+  return check_launch(ctx, "plane_finalize_phis_kernel");
 }
 
 // Work items of one request, largest estimated cost first.  Cost of a
@@ -861,19 +886,22 @@ struct ItemList {
   size_t bytes = 0;
 };
 struct StagedCache {
-  std::map<std::tuple<int, int, unsigned, int, bool>, ItemList> lists;
+  // n, tile rows, crop, directions, sampler, number of phis on an axis (0: all
+  // phis) and ntheta (with the directions they fix which phis those are)
+  std::map<std::tuple<int, int, unsigned, int, bool, int, int>, ItemList> lists;
 };
 }  // namespace
 
 // Device copy of the item list of one geometry: a 16-byte header holding the
 // item count (the kernel reads it from there), then the items.
 int staged_items_cached(wrt_ctx *ctx, int n, int tile_h, float crop_r2, int ndir,
-                        StagedItem **d_items, const int **d_nitems, int *nitems, bool nearest) {
+                        StagedItem **d_items, const int **d_nitems, int *nitems, bool nearest,
+                        const int *phis, int nphis, int ntheta) {
   if (!ctx->staged_cache) ctx->staged_cache = new StagedCache();
   StagedCache *c = static_cast<StagedCache *>(ctx->staged_cache);
   unsigned bits;
   memcpy(&bits, &crop_r2, sizeof(bits));
-  const auto key = std::make_tuple(n, tile_h, bits, ndir, nearest);
+  const auto key = std::make_tuple(n, tile_h, bits, ndir, nearest, nphis, ntheta);
   auto it = c->lists.find(key);
   if (it == c->lists.end()) {
     if (c->lists.size() > 64) {  // bounded: drop everything, rebuild on demand
@@ -882,7 +910,21 @@ int staged_items_cached(wrt_ctx *ctx, int n, int tile_h, float crop_r2, int ndir
       c->lists.clear();
     }
     std::vector<StagedItem> items;
-    staged_items(0, n, tile_h, crop_r2, ndir, kStagedDirChunk, items, nearest);
+    if (nphis) {
+      // a few phis only: chunks of 64 directions, so that they fill the SMs
+      std::vector<std::pair<double, StagedItem>> v;
+      for (int p = 0; p < nphis; ++p) {
+        const size_t v0 = v.size();
+        staged_items_costed(0, n, tile_h, crop_r2, ntheta, 64, 1.0, v, nearest);
+        for (size_t k = v0; k < v.size(); ++k) v[k].second.dir0 += phis[p] * ntheta;
+      }
+      std::stable_sort(v.begin(), v.end(),
+                       [](const std::pair<double, StagedItem> &a,
+                          const std::pair<double, StagedItem> &b) { return a.first > b.first; });
+      for (auto &c : v) items.push_back(c.second);
+    } else {
+      staged_items(0, n, tile_h, crop_r2, ndir, kStagedDirChunk, items, nearest);
+    }
     ItemList l;
     l.count = (int)items.size();
     l.bytes = 16 + sizeof(StagedItem) * items.size();

@@ -24,6 +24,8 @@
 #include <math.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -84,6 +86,9 @@ struct Request {
   double frame[9] = {};
   bool has_frame = false;
 };
+
+constexpr size_t kServerProfBytes = (size_t)768 << 20;
+constexpr size_t kServerProfLeast = (size_t)16 << 20;
 
 struct Slot {
   wrt::BatchSlot batch;
@@ -327,7 +332,7 @@ bool is_pinned(const void *p) {
 }
 
 // Adds an admitted request to the batch being built.
-void add_to_batch(wrt_server *s, Request *q, wrt::BatchBuilder &b) {
+void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::BatchBuilder &b) {
   const wrt_request &r = q->req;
   const GridTables *g = q->grid;
   const int n = r.ngrid;
@@ -413,6 +418,32 @@ void add_to_batch(wrt_server *s, Request *q, wrt::BatchBuilder &b) {
     a.pitch = (int)forward_pitch(n);
     a.L = L;
     a.prep = 1;
+    // the row-sum profiles, where they cover the request and the slot has
+    // their working memory (decided by sizes alone: a request's result does not
+    // depend on what else is running)
+    wrt::ProfReq p = {};
+    p.vol = vol;
+    p.dir = g->dir;
+    p.shift = g->shift;
+    p.stats = stats;
+    p.out = q->d_out;
+    p.n = n;
+    p.L = L;
+    p.nphi = r.nphi;
+    p.ntheta = r.ntheta;
+    p.nshift = r.nshift;
+    p.storage = WRT_STORAGE_F32;
+    p.paired = wrt::profile_paired(n, r.nphi, L);
+    if (wrt::profile_route(s->ctx, n, r.nphi, r.ntheta, r.nshift, false) &&
+        slot.prof_bytes >= wrt::profile_workspace_least(p, 3.0f + 1e-5f)) {
+      a.pairs = nullptr;
+      a.nout = 0;
+      sr.nshift = sr.ndir = 0;
+      b.fwd.push_back(sr);
+      b.aux.push_back(a);
+      b.prof.push_back(p);
+      return;
+    }
     wrt::batch_add_forward(b, sr, a, 3.0f + 1e-5f);
   } else {
     const size_t nplanes = (size_t)ndir * r.nshift;
@@ -513,7 +544,7 @@ void dispatch_loop(wrt_server *s) {
         e = cudaMemcpyAsync(q->d_tab, q->tab.data(), sizeof(double) * q->tab.size(),
                             cudaMemcpyHostToDevice, slot->stream);
       if (e != cudaSuccess && !st) st = wrt::cuda_fail(s->ctx, e, "server input upload");
-      add_to_batch(s, q, b);
+      add_to_batch(s, q, slot->batch, b);
     }
     if (!st) st = wrt::batch_slot_launch(&slot->batch, b);
     if (!st) {
@@ -638,6 +669,13 @@ int wrt_server_create(const wrt_server_opts *opts, wrt_server **out) {
       break;
     }
     st = wrt::batch_slot_init(ctx, &sl->batch, sl->stream);
+    // working memory of the row-sum profiles, beside the arena: a sixteenth of
+    // the budget per slot, at most kServerProfBytes; without it (small budgets,
+    // no memory left) the plane transforms take the staged kernel
+    const size_t want = std::min(budget / 16, kServerProfBytes) & ~(size_t)0xffff;
+    if (!st && want >= kServerProfLeast &&
+        wrt::ctx_alloc(ctx, &sl->batch.prof_ws, want) == WRT_OK)
+      sl->batch.prof_bytes = want;
     s->slots.push_back(std::move(sl));
   }
   if (st) {

@@ -36,6 +36,11 @@
 // ---------------------------------------------------------------- host side
 namespace wrt {
 struct HostPool;  // host threads of the staged copies (hostcopy.cu)
+constexpr int kProfLanes = 4;
+struct ProfLanes {  // side streams of the row-sum profiles (k_profile.cu)
+  cudaStream_t stream[kProfLanes - 1] = {};
+  cudaEvent_t fork = nullptr, done[kProfLanes - 1] = {};
+};
 }
 
 struct wrt_ctx {
@@ -62,8 +67,9 @@ struct wrt_ctx {
   void *batch_slot = nullptr;  // BatchSlot of wrt_radon_forward_batch (batch.cu)
   // grow-only working buffers, one per role (wrt::ws_get), freed with the
   // context: warm calls of the same or smaller sizes allocate nothing
-  void *ws[8] = {};
-  size_t ws_bytes[8] = {};
+  void *ws[10] = {};
+  size_t ws_bytes[10] = {};
+  wrt::ProfLanes prof_lanes;  // side streams of the plane transform's profiles
   void *fft_plans = nullptr;  // spectral Laplacian plans (k_laplace.cu)
   // the volume and sphere grid of the last drop-in (host-array) call, kept
   // for the next call of the same sizes
@@ -87,7 +93,8 @@ void ctx_free(wrt_ctx *ctx, void *p, size_t bytes);
 int check_launch(wrt_ctx *ctx, const char *what);
 // Working buffer of a role, at least `bytes` long (grown after the context's
 // stream has drained; contents are not kept).
-enum WsRole { WS_STAGE, WS_IN, WS_OUT, WS_LINES, WS_SPLINE, WS_COEF, WS_TABLE, WS_FFT, WS_ROLES };
+enum WsRole { WS_STAGE, WS_IN, WS_OUT, WS_LINES, WS_SPLINE, WS_COEF, WS_TABLE, WS_FFT, WS_PROFILE,
+              WS_ROLES };
 int ws_get(wrt_ctx *ctx, int role, size_t bytes, void **p);
 // Copies between caller (pageable) host arrays and the device, through the
 // context's pinned chunk buffers and host threads (hostcopy.cu): the upload
@@ -211,6 +218,9 @@ int plane_staged_launch_nearest(wrt_ctx *ctx, cudaStream_t stream, const StagedR
                                 const StagedItem *d_items, const int *d_nitems, int max_smem,
                                 int *d_next);
 int plane_finalize(wrt_ctx *ctx, double *out, long long count, double factor);
+// The same for the planes of up to four phis of [nshift][nphi][ntheta].
+int plane_finalize_phis(wrt_ctx *ctx, double *out, const int *phis, int nphis, int nphi,
+                        int ntheta, int nshift, double factor);
 // Work items of one request (layer x y-tile x direction chunk) with their
 // estimated cost (staged voxels inside the crop radius x directions x weight).
 void staged_items_costed(int req, int n, int tile_h, float crop_r2, int ndir, int dir_chunk,
@@ -218,11 +228,69 @@ void staged_items_costed(int req, int n, int tile_h, float crop_r2, int ndir, in
                          bool nearest = false);
 void staged_items(int req, int n, int tile_h, float crop_r2, int ndir, int dir_chunk,
                   std::vector<StagedItem> &out, bool nearest = false);
+// phis / nphis: only the directions of these phis (ntheta = ndir / nphi each),
+// all of them when nphis is 0.
 int staged_items_cached(wrt_ctx *ctx, int n, int tile_h, float crop_r2, int ndir,
                         StagedItem **d_items, const int **d_nitems, int *nitems,
-                        bool nearest = false);
+                        bool nearest = false, const int *phis = nullptr, int nphis = 0,
+                        int ntheta = 0);
 int staged_scratch(wrt_ctx *ctx, size_t req_bytes);
 void staged_release(wrt_ctx *ctx);
+
+// Row-sum profiles (k_profile.cu): plane integrals from tables of row sums.
+// Tables of the steps in flight, all lanes together; requests with at least
+// kProfLaneBytes of tables are dealt to kProfLanes streams.
+constexpr size_t kProfTableBytes = (size_t)512 << 20;
+constexpr size_t kProfLaneBytes = (size_t)64 << 20;
+struct ProfReq {            // one plane transform
+  const void *vol;          // v[ix][iy][iz], float or bf16
+  const double *dir;        // [ndir][9]
+  const double *shift;      // [nshift]
+  const unsigned *stats;    // device: [0] largest |x|^2 of a non-zero node (float bits)
+  double *out;              // [nshift][ndir]
+  unsigned long long *counter;
+  int n, L, nphi, ntheta, nshift, storage, nearest;
+  int paired;               // phi and phi + pi share their tables
+};
+struct ProfSeg {            // the units (consecutive phis, one range of t) of one request in a step
+  ProfReq r;
+  void *table, *rec;        // [unit][cap][n] coefficients; [unit][cap] piece records
+  unsigned *pos, *ids;      // [unit][cap + 16] piece starts; what starts there
+  unsigned *start;          // [unit][kUnitBins + 8] first piece of a bin
+  unsigned long long *keys; // [unit][cap]
+  int chunk, base0, nbase, first;
+  int cap, nsub, sub_bins;
+  int blk_rows;             // blocks of the rows role per unit
+};
+template <int S>
+struct ProfStep {
+  ProfSeg seg[S];
+  unsigned long long *list;  // count, then the planes marked in this step
+  int n;
+};
+// Whether phi and phi + pi share tables: their lattices differ by one end sample
+// (-L for L), which lies outside any crop ball for L >= 1.75 n, and outside that
+// of data in the unit ball for L >= n unless the grid is coarse.
+inline bool profile_paired(int n, int nphi, int L) {
+  return nphi % 2 == 0 && (L >= 1.75 * n || (L >= n && n >= 40));
+}
+// Whether the sizes of a request suit the profiles, and whether a request goes
+// there under the context's tile configuration (the same rule for a request
+// alone, in a batch and in the server).
+bool profile_covers(int n, int nphi, int ntheta, int nshift);
+size_t profile_workspace_least(const ProfReq &r, float crop);
+size_t profile_workspace_want(const ProfReq *reqs, const float *crop, int nreq);
+bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift, bool nearest);
+// The plane integrals of nreq requests (one sampler) on a stream.  crop[q]: a bound on the
+// squared crop radius (3 where the host does not know the volume's support yet;
+// it limits which empty ranges of t are visited and the room for pieces).  ws: at least profile_workspace_least for every
+// request.
+// lanes: streams for side-by-side steps, created on first use; the work is
+// forked from `stream` and joined to it again.
+int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const ProfReq *reqs,
+                    const float *crop, int nreq, void *ws, size_t ws_bytes);
+int profile_lanes_init(wrt_ctx *ctx, ProfLanes *l);
+void profile_lanes_release(ProfLanes *l);
 
 // Ray kernels (k_ray.cu).
 struct RayJob {
@@ -297,8 +365,10 @@ struct BatchBuilder {
   std::vector<AdjReq> adj;
   std::vector<RayJob> ray;
   std::vector<RedReq> red;
+  std::vector<ProfReq> prof;  // plane transforms by row-sum profiles
   std::vector<std::pair<double, StagedItem>> items;  // cost, item
   void clear() {
+    prof.clear();
     fwd.clear();
     aux.clear();
     adj.clear();
@@ -320,6 +390,11 @@ struct BatchSlot {
   cudaEvent_t done = nullptr;
   int config = -2;
   bool counting = false, launched = false;
+  // the row-sum profiles' working memory (set by the owner; null: requests take
+  // the staged kernel) and side streams
+  void *prof_ws = nullptr;
+  size_t prof_bytes = 0;
+  ProfLanes prof_lanes;
 };
 // Adds a forward request (staged kernel) to the builder: its descriptor, its
 // auxiliary record and its work items.  crop_items: crop radius^2 used to
