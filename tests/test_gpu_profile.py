@@ -74,3 +74,20 @@ def test_tight_budget_takes_the_staged_kernel():
         got = c.radon_grid(vol, 32, 16, 64, sampler=wrt.TRILINEAR, half_extent=48)
     ref = O.radon_forward(vol, 32, 16, 64, sampler=O.TRILINEAR, half_extent=48)
     assert rel_l2(got, ref) < TOL_L2
+
+
+# ---- backprojection from merged splines (csrc/k_backproj.cu): just beyond the
+# sizes of the allocation-free path; odd longitudes (nothing merged), longitudes
+# not a multiple of 32, odd latitudes, one voxel tile and several, few knots
+# with many longitudes
+@pytest.mark.parametrize("n,nphi,ntheta,nshift", [
+    (5, 64, 32, 129), (20, 33, 31, 257), (17, 130, 64, 33), (33, 96, 47, 61), (48, 70, 35, 110),
+])
+def test_backprojection_matches_oracle(ctx, n, nphi, ntheta, nshift):
+    radon = np.random.default_rng(n).standard_normal((nshift, nphi, ntheta))
+    got = ctx.radon3d_adjoint(radon, n)
+    assert np.array_equal(got, ctx.radon3d_adjoint(radon, n))
+    x = -1.0 + (2.0 * np.arange(n) + 1.0) / n
+    pick = np.random.default_rng(1).integers(0, n, (400, 3))
+    ref = O.adjoint_points(radon, x[pick[:, 1]], x[pick[:, 2]], x[pick[:, 0]])
+    assert rel_l2(got[pick[:, 0], pick[:, 1], pick[:, 2]], ref) < TOL_L2

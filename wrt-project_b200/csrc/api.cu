@@ -1161,6 +1161,36 @@ int wrt_radon3d_adjoint_device(wrt_ctx *ctx, const double *dev_radon, const wrt_
                : WRT_ERR_INVALID_ARGUMENT;
   int st = set_device(ctx);
   if (st) return st;
+  if (backproj_covers(grid->nphi, grid->ntheta, grid->nshift, ngrid)) {
+    const size_t want = backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, false);
+    void *ws = nullptr, *cp = nullptr;
+    st = ws_get(ctx, WS_PROFILE, want, &ws);
+    if (st)
+      st = ws_get(ctx, WS_PROFILE,
+                  backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, true), &ws);
+    if (!st) st = ws_get(ctx, WS_COEF, sizeof(double) * 2 * grid->nshift, &cp);
+    if (!st) {
+      std::vector<double> coef(2 * (size_t)grid->nshift);
+      spline_coefficients(grid->nshift, coef.data(), coef.data() + grid->nshift);
+      // a copy from pageable memory returns once the data is staged
+      st = h2d(ctx, cp, coef.data(), sizeof(double) * grid->nshift, "spline coefficients");
+      if (st) return st;
+      BackReq r = {};
+      r.radon = dev_radon;
+      r.cs = grid->d_cs;
+      r.dir = grid->d_dir;
+      r.dirw = grid->d_dirw;
+      r.cp = static_cast<const double *>(cp);
+      r.out = dev_out;
+      r.nphi = grid->nphi;
+      r.ntheta = grid->ntheta;
+      r.ns = grid->nshift;
+      r.n = ngrid;
+      return backproj_forward(ctx, ctx->stream, &ctx->prof_lanes, r, ws,
+                              std::min(want, ctx->ws_bytes[WS_PROFILE]));
+    }
+    ctx->err[0] = 0;  // no room for the tables: the direct kernel
+  }
   return adjoint_forward(ctx, dev_radon, grid->nphi, grid->ntheta, grid->nshift, grid->d_dirw,
                          grid->dirw.data(), ngrid, dev_out);
 }

@@ -444,6 +444,10 @@ int batch_slot_launch(BatchSlot *s, BatchBuilder &b) {
                          (int)b.prof.size(), s->prof_ws, s->prof_bytes);
     if (st) return st;
   }
+  for (const BackReq &q : b.back) {
+    st = backproj_forward(ctx, s->stream, &s->prof_lanes, q, s->prof_ws, s->prof_bytes);
+    if (st) return st;
+  }
   // the backprojections, behind the graph (which built their spline lines):
   // their direction constants travel as launch parameters
   for (const AdjReq &j : b.adj) {

@@ -447,6 +447,22 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
     wrt::batch_add_forward(b, sr, a, 3.0f + 1e-5f);
   } else {
     const size_t nplanes = (size_t)ndir * r.nshift;
+    if (wrt::backproj_covers(r.nphi, r.ntheta, r.nshift, n) &&
+        slot.prof_bytes >= wrt::backproj_workspace(r.nphi, r.ntheta, r.nshift, n, true)) {
+      wrt::BackReq q2 = {};
+      q2.radon = reinterpret_cast<const double *>(base);
+      q2.cs = g->cs;
+      q2.dir = g->dir;
+      q2.dirw = g->dirw;
+      q2.cp = g->cp;
+      q2.out = q->d_out;
+      q2.nphi = r.nphi;
+      q2.ntheta = r.ntheta;
+      q2.ns = r.nshift;
+      q2.n = n;
+      b.back.push_back(q2);
+      return;
+    }
     wrt::AdjReq j = {};
     j.radon = reinterpret_cast<const double *>(base);
     j.scratch = reinterpret_cast<double *>(base + al(8 * nplanes));

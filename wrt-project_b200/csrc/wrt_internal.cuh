@@ -292,6 +292,36 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
 int profile_lanes_init(wrt_ctx *ctx, ProfLanes *l);
 void profile_lanes_release(ProfLanes *l);
 
+// Backprojection from splines merged over the latitudes (k_backproj.cu).
+struct BackReq {
+  const double *radon;   // [is][iphi][itheta]
+  const double *cs;      // [ntheta][2] cos, sin theta
+  const double *dir;     // [ndir][9] FP64 directions
+  const double4 *dirw;   // [ndir] omega / h, dphi * w_theta
+  const double *cp;      // [ns] spline elimination factors
+  double *out;           // [iz][ix][iy]
+  int nphi, ntheta, ns, n;
+  // set by backproj_forward
+  int nbase, paired;     // longitudes tabulated; phi + pi merged into phi
+  double *Y, *M, *D;     // [theta][is][nbase]
+};
+constexpr size_t kBackTableBytes = (size_t)768 << 20;  // tables in flight
+struct BackStep {        // a group of z planes
+  BackReq r;
+  float4 *table;         // [z][cap][nbase]
+  void *rec;             // [z][cap]
+  unsigned *pos, *ids;   // [z][cap + 16]
+  unsigned *start;       // [z][nb + 8]
+  unsigned long long *keys;  // [z][cap]
+  int z0, cap, nb, nb_log2, nsub_log2, tiles;
+};
+// Whether a backprojection goes there (by sizes alone), its working memory (for
+// one z plane at a time, or what fills the device), and the launches.
+bool backproj_covers(int nphi, int ntheta, int ns, int n);
+size_t backproj_workspace(int nphi, int ntheta, int ns, int n, bool least);
+int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackReq r, void *ws,
+                     size_t ws_bytes);
+
 // Ray kernels (k_ray.cu).
 struct RayJob {
   const float *vol;
@@ -366,9 +396,11 @@ struct BatchBuilder {
   std::vector<RayJob> ray;
   std::vector<RedReq> red;
   std::vector<ProfReq> prof;  // plane transforms by row-sum profiles
+  std::vector<BackReq> back;  // backprojections by merged splines
   std::vector<std::pair<double, StagedItem>> items;  // cost, item
   void clear() {
     prof.clear();
+    back.clear();
     fwd.clear();
     aux.clear();
     adj.clear();
@@ -390,8 +422,8 @@ struct BatchSlot {
   cudaEvent_t done = nullptr;
   int config = -2;
   bool counting = false, launched = false;
-  // the row-sum profiles' working memory (set by the owner; null: requests take
-  // the staged kernel) and side streams
+  // working memory of the row-sum profiles and merged backprojections (set by
+  // the owner; null: requests take the staged and direct kernels), side streams
   void *prof_ws = nullptr;
   size_t prof_bytes = 0;
   ProfLanes prof_lanes;
