@@ -1074,11 +1074,9 @@ int wrt_ray_forward_device(wrt_ctx *ctx, const wrt_volume *cvol, const double *f
   st = ws_get(ctx, WS_TABLE, sizeof(double) * tab.size(), &dtab);
   // a copy from pageable memory returns once the data is staged
   if (!st) st = h2d(ctx, dtab, tab.data(), sizeof(double) * tab.size(), "ray grid");
-  // samples read the cell octets (one 32-byte sector each; built once per
-  // volume); in the reference frame the guard-band-free groups do, and single
-  // samples read the layer pairs (built once) as before
-  if (!st && identity) st = volume_ensure_pairs(vol);
-  if (!st) st = volume_ensure_octets(vol);
+  // in rotated frames samples read the cell octets (one 32-byte sector each;
+  // built once per volume); the z-slices read the volume itself
+  if (!st && !identity) st = volume_ensure_octets(vol);
   if (st) return st;
   RayJob job = {};
   job.vol = vol->d_vol;
@@ -1095,12 +1093,8 @@ int wrt_ray_forward_device(wrt_ctx *ctx, const wrt_volume *cvol, const double *f
   job.margin = sampler_margin(n, WRT_SAMPLER_TRILINEAR);
   job.out = dev_out;
   job.counter = ctx->d_counter;
-  if (identity) {
-    job.pairs = vol->d_pairs;
-    job.pitch = vol->pitch;
-  }
-  job.oct = vol->d_oct;
-  return ray_forward(ctx, job);
+  job.oct = identity ? nullptr : vol->d_oct;
+  return ray_forward(ctx, ctx->stream, job);
 }
 
 int wrt_ray_grid(wrt_ctx *ctx, const double *volume, int n, int nslices, int nshift, int nphi,

@@ -182,7 +182,8 @@ __global__ void batch_spline_kernel(const char *t) {
   }
 }
 
-// Every ray of every ray-transform request (ray_grid/src/integral.c:11-50):
+// Every ray of every ray-transform request in a rotated frame
+// (ray_grid/src/integral.c:11-50):
 // consecutive threads take consecutive rays (32 shifts of one layer and angle).
 __global__ void __launch_bounds__(256) batch_ray_kernel(const char *t) {
   const int nr = hdr(t)->nray;
@@ -195,10 +196,7 @@ __global__ void __launch_bounds__(256) batch_ray_kernel(const char *t) {
     const long long total = (long long)job.nslices * job.nshift * job.nphi;
     const float g = wrtd::ray_guard(job.n);
     for (long long k = dealt_first(tid, first, nth); k < total; k += nth) {
-      if (job.has_frame)
-        wrtd::ray_one<true>(job, k, g);
-      else
-        wrtd::ray_one<false>(job, k, g);
+      wrtd::ray_one(job, k, g);
     }
     first += total;
   }
@@ -442,6 +440,10 @@ int batch_slot_launch(BatchSlot *s, BatchBuilder &b) {
     const std::vector<float> crop(b.prof.size(), 3.0f + 1e-5f);
     st = profile_forward(ctx, s->stream, &s->prof_lanes, b.prof.data(), crop.data(),
                          (int)b.prof.size(), s->prof_ws, s->prof_bytes);
+    if (st) return st;
+  }
+  for (const RayJob &j : b.slices) {
+    st = ray_forward(ctx, s->stream, j);
     if (st) return st;
   }
   for (const BackReq &q : b.back) {

@@ -1,21 +1,17 @@
 // ray_dev.cuh -- the device body of the layer-by-layer ray integral
-// (ray_grid/src/integral.c:11-50), shared by the single-request kernel
-// (k_ray.cu) and the batched one (batch.cu).
+// (ray_grid/src/integral.c:11-50) in a rotated layer frame, shared by the
+// single-request kernel (k_ray.cu) and the batched one (batch.cu).
 //
 // Ray (z, s, phi): p(k) = (s cos phi, s sin phi, z) + delta*k*(cos(phi+pi/2),
 // sin(phi+pi/2), 0), delta = 1/(n-1), k in [-2n, 2n], weight delta, trilinear
-// sampler.  With a frame F every point is mapped to F p(k) (the layer scheme
-// about another axis; F = identity reproduces the reference).
+// sampler, every point mapped to F p(k) (the layer scheme about another axis;
+// the reference's own z-slices, F = identity, are k_ray.cu's slices kernel).
 //
 // One lane per ray; the kernels choose which rays share a warp (k_ray.cu: a
 // tile of consecutive shifts x consecutive angles of one layer).  Samples
 // farther than sqrt(crop_r2) from the origin or outside the cube are skipped
 // (their value is exactly 0).  Numerics: FP32 cell coordinates with the guard
-// band of wrt_internal.cuh.  In the reference frame the z coordinate of a ray
-// is one FP64 number for all its samples, so its cell and fraction are
-// computed once per ray with the reference's own arithmetic
-// (cube_trilinear_interp, radon_grid/src/interp.c:33-53) and used by every
-// FP32 sample of the ray.
+// band of wrt_internal.cuh.
 #pragma once
 #include "wrt_internal.cuh"
 
@@ -82,7 +78,6 @@ struct RayCell {
 };
 
 // Ray number `ray` (0 <= ray < nslices * nshift * nphi, shift fastest) of a job.
-template <bool FRAME>
 __device__ __forceinline__ void ray_one(const wrt::RayJob &job, long long ray, float guard) {
   const int is = (int)(ray % job.nshift);
   const int ip = (int)((ray / job.nshift) % job.nphi);
@@ -114,64 +109,32 @@ __device__ __forceinline__ void ray_one(const wrt::RayJob &job, long long ray, f
   }
   const double h = 0.5 * (n - 1);
   const double *F = job.frame;  // kernel parameter space
-  if (any && !FRAME) {
-    any = clip_axis(p0x, ax, klo, khi) && clip_axis(p0y, ay, klo, khi) && fabs(zslice) <= 1.0;
-  } else if (any) {
+  if (any) {
     double bx = rot_row(F, 0, p0x, p0y, p0z), by = rot_row(F, 1, p0x, p0y, p0z),
            bz = rot_row(F, 2, p0x, p0y, p0z);
     double tx = F[0] * ax + F[1] * ay, ty = F[3] * ax + F[4] * ay, tz = F[6] * ax + F[7] * ay;
     any = clip_axis(bx, tx, klo, khi) && clip_axis(by, ty, klo, khi) && clip_axis(bz, tz, klo, khi);
   }
   if (any) {
-    float ub, vb, wb, du, dv, dw;
-    int zc = 0;
-    float tzc = 0.0f;
-    if (!FRAME) {
-      ub = (float)((p0x + 1.0) * h);
-      vb = (float)((p0y + 1.0) * h);
-      du = (float)(ax * h);
-      dv = (float)(ay * h);
-      wb = 0.0f;
-      dw = 0.0f;
-      // z cell of the whole ray, reference arithmetic (interp.c:32-53)
-      const double dlt = 2.0 / (n - 1);
-      const double z1 = __dadd_rn(zslice, 1.0);
-      zc = (int)__ddiv_rn(z1, dlt);
-      double cz = __ddiv_rn(fmod(z1, dlt), dlt);
-      if (zc == n - 1) {
-        zc -= 1;
-        cz = 1.0;
-      }
-      tzc = (float)cz;
-    } else {
-      const double bx = rot_row(F, 0, p0x, p0y, p0z), by = rot_row(F, 1, p0x, p0y, p0z),
-                   bz = rot_row(F, 2, p0x, p0y, p0z);
-      ub = (float)((bx + 1.0) * h);
-      vb = (float)((by + 1.0) * h);
-      wb = (float)((bz + 1.0) * h);
-      du = (float)((F[0] * ax + F[1] * ay) * h);
-      dv = (float)((F[3] * ax + F[4] * ay) * h);
-      dw = (float)((F[6] * ax + F[7] * ay) * h);
-    }
+    const double bx = rot_row(F, 0, p0x, p0y, p0z), by = rot_row(F, 1, p0x, p0y, p0z),
+                 bz = rot_row(F, 2, p0x, p0y, p0z);
+    float ub = (float)((bx + 1.0) * h), vb = (float)((by + 1.0) * h), wb = (float)((bz + 1.0) * h);
+    const float du = (float)((F[0] * ax + F[1] * ay) * h);
+    const float dv = (float)((F[3] * ax + F[4] * ay) * h);
+    const float dw = (float)((F[6] * ax + F[7] * ay) * h);
     // FP64 reference evaluation of sample k (interp.c:25-60 at F p(k))
     auto exact_at = [&](int k) {
       const double dk = (double)k;
-      double px = __dadd_rn(p0x, __dmul_rn(ax, dk));
-      double py = __dadd_rn(p0y, __dmul_rn(ay, dk));
-      double pz = __dadd_rn(p0z, __dmul_rn(__dmul_rn(delta, 0.0), dk));
-      if (FRAME) {
-        const double wx = rot_row(F, 0, px, py, pz), wy = rot_row(F, 1, px, py, pz),
-                     wz = rot_row(F, 2, px, py, pz);
-        px = wx;
-        py = wy;
-        pz = wz;
-      }
-      return wrtd::exact_trilinear(job.vol, n, px, py, pz);
+      const double px = __dadd_rn(p0x, __dmul_rn(ax, dk));
+      const double py = __dadd_rn(p0y, __dmul_rn(ay, dk));
+      const double pz = __dadd_rn(p0z, __dmul_rn(__dmul_rn(delta, 0.0), dk));
+      return wrtd::exact_trilinear(job.vol, n, rot_row(F, 0, px, py, pz),
+                                   rot_row(F, 1, px, py, pz), rot_row(F, 2, px, py, pz));
     };
     // Every path locates a sample the same way and interpolates its 8
     // corners in one order (octet_lerp: x, then y, then z), whether the
-    // corners come from the cell octets, the layer pairs or the volume, so a
-    // ray's value does not depend on which of them the job carries.
+    // corners come from the cell octets or the volume, so a ray's value does
+    // not depend on which of them the job carries.
     // q' = q - 1/2 at k = 0 (one more rounding of at most half an ulp, well
     // inside the guard band's allowance for the FP32 coordinates)
     ub -= 0.5f;
@@ -189,20 +152,12 @@ __device__ __forceinline__ void ray_one(const wrt::RayJob &job, long long ray, f
       c.by = __float_as_uint(sy);
       c.tx = ex + 0.5f;
       c.ty = ey + 0.5f;
-      float m = fmaxf(fabsf(ex), fabsf(ey));
-      c.in = (c.bx - mb < um) & (c.by - mb < um);
-      if (FRAME) {
-        const float qz = fmaf(kf, dw, wb), sz = qz + kRayMagic;
-        const float ez = qz - (sz - kRayMagic);
-        c.bz = __float_as_uint(sz);
-        c.tz = ez + 0.5f;
-        m = fmaxf(m, fabsf(ez));
-        c.in &= c.bz - mb < um;
-      } else {
-        c.bz = mb + (unsigned)zc;  // the ray's z cell, reference arithmetic
-        c.tz = tzc;
-      }
-      c.band = m > halfband;
+      const float qz = fmaf(kf, dw, wb), sz = qz + kRayMagic;
+      const float ez = qz - (sz - kRayMagic);
+      c.bz = __float_as_uint(sz);
+      c.tz = ez + 0.5f;
+      c.in = (c.bx - mb < um) & (c.by - mb < um) & (c.bz - mb < um);
+      c.band = fmaxf(fmaxf(fabsf(ex), fabsf(ey)), fabsf(ez)) > halfband;
       return c;
     };
     // the 8 corners of an inside cell in octet order
@@ -210,13 +165,6 @@ __device__ __forceinline__ void ray_one(const wrt::RayJob &job, long long ray, f
       const unsigned ix = c.bx - mb, iy = c.by - mb, izc = c.bz - mb;
       if (job.oct) {
         ld_octet(job.oct, ((size_t)izc * (n - 1) + iy) * (n - 1) + ix, lo, hi);
-      } else if (!FRAME && job.pairs) {
-        // one z-layer pair: rows contiguous in x
-        const float2 *p = job.pairs + ((size_t)izc * n + iy) * job.pitch + ix;
-        const float2 a = __ldg(p), b = __ldg(p + job.pitch), d = __ldg(p + 1),
-                     e = __ldg(p + job.pitch + 1);
-        lo = make_float4(a.x, a.y, b.x, b.y);
-        hi = make_float4(d.x, d.y, e.x, e.y);
       } else {
         const float *p = job.vol + ((size_t)ix * n + iy) * n + izc;
         const size_t sx = (size_t)n * n;

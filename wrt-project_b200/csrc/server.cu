@@ -339,8 +339,8 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
   const int ndir = r.nphi * r.ntheta;
   char *base = static_cast<char *>(q->d_in);
   if (r.op == WRT_OP_RAY) {
-    // the volume is prepared (statistics, layer pairs) by the batch's volume
-    // kernel through a forward entry with no planes and no work items
+    // the volume's statistics come from the batch's volume kernel through a
+    // forward entry with no planes and no work items
     const size_t nn = (size_t)n;
     float *vol = reinterpret_cast<float *>(base);
     float2 *pairs = reinterpret_cast<float2 *>(base + al(4 * nn * nn * nn));
@@ -351,7 +351,7 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
                         nullptr, nullptr, nullptr, nullptr, nullptr, &sr);
     wrt::FwdAux a = {};
     a.vol = vol;
-    a.pairs = pairs;
+    a.pairs = nullptr;
     a.stats = stats;
     a.nout = 0;
     a.n = n;
@@ -373,11 +373,7 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
     job.r2bits = stats;
     job.margin = wrt::trilinear_margin(n);
     job.out = q->d_out;
-    if (!q->has_frame) {  // z-slices read the layer pairs
-      job.pairs = pairs;
-      job.pitch = (int)forward_pitch(n);
-    }
-    b.ray.push_back(job);
+    (q->has_frame ? b.ray : b.slices).push_back(job);
     return;
   }
   if (r.op == WRT_OP_REDUCE) {

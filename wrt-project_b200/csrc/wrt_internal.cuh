@@ -334,8 +334,6 @@ struct RayJob {
   const unsigned int *r2bits;
   double margin;
   double *out;          // [nslices][nshift][nphi]
-  const float2 *pairs;  // layer pairs [n-1][n][pitch] of the volume, or null
-  int pitch;
   unsigned long long *counter;  // optional: samples evaluated
   const float4 *oct;    // cell octets of the volume (rotated frames), or null
 };
@@ -393,7 +391,8 @@ struct BatchBuilder {
   std::vector<StagedReq> fwd;
   std::vector<FwdAux> aux;
   std::vector<AdjReq> adj;
-  std::vector<RayJob> ray;
+  std::vector<RayJob> ray;     // in rotated frames
+  std::vector<RayJob> slices;  // in the reference frame
   std::vector<RedReq> red;
   std::vector<ProfReq> prof;  // plane transforms by row-sum profiles
   std::vector<BackReq> back;  // backprojections by merged splines
@@ -401,6 +400,7 @@ struct BatchBuilder {
   void clear() {
     prof.clear();
     back.clear();
+    slices.clear();
     fwd.clear();
     aux.clear();
     adj.clear();
@@ -442,7 +442,7 @@ void staged_request(int n, int pitch, int ndir, int nshift, int L, int storage,
                     const void *pairs, const void *vol, const double *dir, const float *dir32,
                     const double *shift, const float *shift32, double *out, StagedReq *r);
 
-int ray_forward(wrt_ctx *ctx, const RayJob &job);
+int ray_forward(wrt_ctx *ctx, cudaStream_t stream, const RayJob &job);
 // Host tables of a ray job (ray_grid/src/init.c:163-176, integral.c:16-24):
 // tab[0..nshift) the shifts, then [nphi][4] cos phi, sin phi, cos(phi+pi/2),
 // sin(phi+pi/2).
