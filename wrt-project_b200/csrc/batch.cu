@@ -442,6 +442,12 @@ int batch_slot_launch(BatchSlot *s, BatchBuilder &b) {
                          (int)b.prof.size(), s->prof_ws, s->prof_bytes);
     if (st) return st;
   }
+  for (const RedReq &q : b.staged_red) {
+    st = reduction_staged(ctx, s->stream, q.rays, q.ngrid, q.ns_ray, q.nphi, q.shift, q.nshift, q.cs,
+                          q.ntheta, q.coef, q.scratch, reinterpret_cast<float *>(q.lines), nullptr,
+                          q.out);
+    if (st) return st;
+  }
   for (const RayJob &j : b.slices) {
     st = ray_forward(ctx, s->stream, j);
     if (st) return st;

@@ -142,6 +142,23 @@ cudaError_t launch_adjoint(cudaStream_t stream, const float4 *d_lines, int ndir,
 int reduction_forward(wrt_ctx *ctx, const double *d_rays, int ngrid, int nshift_ray, int nphi,
                       const double *d_shift, int nshift, const double *d_cs, int ntheta,
                       double *d_out) {
+  if (reduction_covers(ngrid, nshift_ray)) {
+    const size_t count = (size_t)ngrid * nphi * nshift_ray;
+    std::vector<double> coef(2 * (size_t)nshift_ray);
+    spline_coefficients(nshift_ray, coef.data(), coef.data() + nshift_ray);
+    void *cp = nullptr, *scratch = nullptr, *m = nullptr;
+    int st = ws_get(ctx, WS_COEF, sizeof(double) * coef.size(), &cp);
+    if (!st) st = ws_get(ctx, WS_SPLINE, sizeof(double) * count, &scratch);
+    if (!st) st = ws_get(ctx, WS_LINES, sizeof(float) * count, &m);
+    if (st) return st;
+    // a copy from pageable memory returns once the data is staged
+    cudaError_t e = cudaMemcpyAsync(cp, coef.data(), sizeof(double) * nshift_ray,
+                                    cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "spline coefficients");
+    return reduction_staged(ctx, ctx->stream, d_rays, ngrid, nshift_ray, nphi, d_shift, nshift, d_cs,
+                            ntheta, static_cast<const double *>(cp), static_cast<double *>(scratch),
+                            static_cast<float *>(m), ctx->d_counter, d_out);
+  }
   // lines (iz, iphi): element is at d_rays[(iz*ns_ray + is)*nphi + iphi]
   float4 *d_lines = nullptr;
   int st = prep_lines(ctx, d_rays, ngrid * nphi, nphi, (long long)nshift_ray * nphi, nphi, 1,

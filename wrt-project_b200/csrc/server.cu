@@ -392,7 +392,7 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
     rq.nphi = r.nphi;
     rq.nshift = r.nshift;
     rq.ntheta = r.ntheta;
-    b.red.push_back(rq);
+    (wrt::reduction_covers(n, (int)nsr) ? b.staged_red : b.red).push_back(rq);
     return;
   }
   if (r.op == WRT_OP_FORWARD) {

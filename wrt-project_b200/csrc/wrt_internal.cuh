@@ -393,13 +393,15 @@ struct BatchBuilder {
   std::vector<AdjReq> adj;
   std::vector<RayJob> ray;     // in rotated frames
   std::vector<RayJob> slices;  // in the reference frame
-  std::vector<RedReq> red;
+  std::vector<RedReq> red;     // by records gathered through L1
+  std::vector<RedReq> staged_red;  // with a longitude's splines in shared memory
   std::vector<ProfReq> prof;  // plane transforms by row-sum profiles
   std::vector<BackReq> back;  // backprojections by merged splines
   std::vector<std::pair<double, StagedItem>> items;  // cost, item
   void clear() {
     prof.clear();
     back.clear();
+    staged_red.clear();
     slices.clear();
     fwd.clear();
     aux.clear();
@@ -474,6 +476,14 @@ int reduction_forward(wrt_ctx *ctx, const double *d_rays, int ngrid, int nshift_
                       int nphi, const double *d_shift, int nshift,
                       const double *d_cs /* [ntheta][2]: cos, sin theta */, int ntheta,
                       double *d_out);
+// The same with one longitude's splines in shared memory (k_reduction.cu), where
+// they fit (by sizes alone): cp[ns_ray] elimination factors, scratch [ngrid*nphi*
+// ns_ray] doubles and m as many floats of working memory.
+bool reduction_covers(int ngrid, int ns_ray);
+int reduction_staged(wrt_ctx *ctx, cudaStream_t stream, const double *rays, int ngrid, int ns_ray,
+                     int nphi, const double *shift, int nshift, const double *cs, int ntheta,
+                     const double *cp, double *scratch, float *m, unsigned long long *counter,
+                     double *out);
 // d_dirw / h_dirw: the same direction table [nphi*ntheta] (omega/h, dphi*w) on
 // the device (spline weights) and on the host (per-launch constants).
 int adjoint_forward(wrt_ctx *ctx, const double *d_radon, int nphi, int ntheta, int nshift,
