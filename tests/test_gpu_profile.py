@@ -68,6 +68,30 @@ def test_batch_and_bf16_equal_alone(profiles):
         assert np.array_equal(got, out.download(np.empty(g.nplanes)))
 
 
+def test_batch_of_both_kernels(ctx):
+    # sizes on either side of the rule: the profiles run beside the staged kernel
+    sizes = [(16, (16, 8, 40), 16), (40, (8, 3, 32), 40), (24, (16, 8, 32), 24),
+             (65, (30, 15, 50), 65), (9, (6, 3, 33), 9), (31, (15, 9, 61), 31)]
+    reqs, keep = [], []
+    for n, grid, L in sizes:
+        v = wrt.Volume(ctx, n)
+        v.upload(_volume("noise", n))
+        g = wrt.Grid(ctx, *grid)
+        out = wrt.DeviceBuffer(ctx, g.nplanes * 8)
+        keep.append((v, g, out))
+        reqs.append((v, g, out.ptr, L))
+    got = []
+    for _ in range(2):
+        wrt.radon_forward_batch(ctx, reqs)
+        ctx.synchronize()
+        got.append([out.download(np.empty(g.nplanes)) for _, g, out in keep])
+    for (n, grid, L), a, b in zip(sizes, *got):
+        ref = O.radon_forward(_volume("noise", n), *grid, sampler=O.TRILINEAR, half_extent=L)
+        assert np.array_equal(a, b)
+        assert rel_l2(a, ref.ravel()) < TOL_L2
+        assert rel_max(a, ref.ravel()) < TOL_MAX
+
+
 def test_tight_budget_takes_the_staged_kernel():
     vol = ellipsoid_phantom(48, 8, 5)
     with wrt.Context(0, budget_bytes=12 << 20) as c:

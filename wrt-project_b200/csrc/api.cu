@@ -887,10 +887,22 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
     a.prep = 0;
     batch_add_forward(b, q, a, trilinear_crop_r2(vol->r2, n));
   }
+  auto profiles = [&](bool forked) {
+    return prof.empty() ? WRT_OK
+                        : profile_forward(ctx, ctx->stream, &ctx->prof_lanes, prof.data(),
+                                          prof_crop.data(), (int)prof.size(), prof_ws, prof_bytes,
+                                          forked);
+  };
+  if (b.fwd.empty()) return profiles(false);
   if (!prof.empty()) {
-    st = profile_forward(ctx, ctx->stream, &ctx->prof_lanes, prof.data(), prof_crop.data(),
-                         (int)prof.size(), prof_ws, prof_bytes);
-    if (st || b.fwd.empty()) return st;
+    // beside the staged kernel, and before it: its blocks hold their SM until
+    // the item list is empty, so they take what the profiles leave free
+    st = profile_lanes_init(ctx, &ctx->prof_lanes);
+    if (st) return st;
+    cudaError_t e = cudaEventRecord(ctx->prof_lanes.fork, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "profile fork");
+    st = profiles(true);
+    if (st) return st;
   }
   if (!ctx->batch_slot) {
     BatchSlot *s = new (std::nothrow) BatchSlot();
@@ -903,7 +915,12 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
     }
     ctx->batch_slot = s;
   }
-  return batch_slot_launch(static_cast<BatchSlot *>(ctx->batch_slot), b);
+  st = batch_slot_launch(static_cast<BatchSlot *>(ctx->batch_slot), b);
+  if (!prof.empty()) {
+    cudaError_t e = cudaStreamWaitEvent(ctx->stream, ctx->prof_lanes.done[0], 0);
+    if (e != cudaSuccess && !st) st = cuda_fail(ctx, e, "profile join");
+  }
+  return st;
 }
 
 int wrt_plane_kernel_config_count(void) { return kNumStagedConfigs; }

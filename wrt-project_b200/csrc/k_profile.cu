@@ -18,10 +18,11 @@
 // table reads instead of its ~2n samples.  At 128^3 with 64 latitudes, 256
 // shifts, a table of 2.8e4 x 128 records serves 4.7e6 rows of ~170 samples.
 //
-// A step handles as many units of work (as a rule of one request) as the tables' workspace holds, in three
+// A step handles as many units of work as the tables' workspace holds, in four
 // launches: the pieces of every unit are found and sorted, the tables summed
-// up, the rows evaluated.  A unit is one phi (or the pair phi, phi + pi, which
-// share their lines: t -> -t) and one range of kUnitBins bins of t.
+// up, the rows evaluated, and those that the tables do not decide once more.  A unit
+// is one phi (or the pair phi, phi + pi, which share their lines: t -> -t) and one
+// range of kUnitBins bins of t.
 //
 // Coordinates.  t in cells, tb = (t + t_off) * n bins (n bins per cell: 2 to 4
 // pieces per bin).  Positions within a unit are fixed point, 12.20 bits.
@@ -33,15 +34,16 @@
 // of a piece boundary (some sample within ~1e-8 cells of a cell boundary, where
 // the reference's rounding decides the cell) or with z within 1e-9 cells of a
 // node layer is summed sample by sample with the reference's FP64 arithmetic.
-// Plane sums are FP64 in a fixed order, one warp per plane and unit, units in
-// order: bitwise the same alone or in any batch.
+// Plane sums are FP64 in an order that the request's sizes fix: bitwise the same
+// alone or in any batch.
 //
 // What bounds it: nothing close to a byte or flop limit any more; the rows
 // launch waits for its gathers (random 32-byte reads, mostly from L2) and FP64
 // geometry, the build for its node loads.  128^3, 64 x 128 directions x 256
 // shifts, lattice [-n, n)^2: 53.7 ms by the staged kernel (lattice samples
 // through shared memory), 5.2 ms here; 256^3 BF16, 96 x 192 x 384: 750 and 64
-// ms; error against FP64 6.5e-8 (staged 8.9e-8).
+// ms; error against FP64 6.5e-8 (staged 8.9e-8).  Small requests wait for the four
+// launches one after another (24^3, 8 x 16 x 32: 109 and 80 us).
 #include <math.h>
 #include <string.h>
 
@@ -58,7 +60,7 @@ using wrt::ProfSeg;
 
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kThreads = 256;
-constexpr int kRowTiles = 1;  // groups of 32 planes per warp of the rows role
+constexpr int kMaxChunks = 6;  // ranges of t of one phi in a step
 constexpr double kMagicPos = 6442450944.0;            // 1.5 * 2^32: 20 fraction bits
 constexpr double kMagicInt = 6755399441055744.0;      // 1.5 * 2^52
 constexpr unsigned kBoundary = 2;  // 2^-20 bins: rows this near a piece end go exact
@@ -74,12 +76,16 @@ __device__ __forceinline__ Geo geo_of(const ProfReq &r, int base, int chunk) {
   return make_geo(r.n, r.nearest, r.L, __ldg(D + 7), -__ldg(D + 6), (double)crop_of(r), chunk);
 }
 
+__device__ __forceinline__ Geo geo_of_unit(const ProfSeg &s, int unit) {
+  return geo_of(s.r, s.base0 + unit % s.nbase, s.chunk + unit / s.nbase);
+}
+
 // ------------------------------------------------------------------ sort role
 // One block finds the unit's piece boundaries, counts them per bin, and writes
 // them in order of (position, identity): a bin's few entries are ranked by
 // counting, so the order does not depend on the atomics.
 __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
-  const Geo g = geo_of(s.r, s.base0 + unit, s.chunk);
+  const Geo g = geo_of_unit(s, unit);
   unsigned *pos = s.pos + (size_t)unit * (s.cap + 16);
   unsigned *ids = s.ids + (size_t)unit * (s.cap + 16);
   unsigned *start = s.start + (size_t)unit * (kUnitBins + 8);
@@ -299,7 +305,7 @@ constexpr int kRecTile = 128;
 template <bool NEAR, typename VT>
 __device__ __forceinline__ void role_build(const ProfSeg &s, int blk, const VT *vol, char *smem) {
   const int unit = blk / s.nsub, sub = blk % s.nsub;
-  const Geo g = geo_of(s.r, s.base0 + unit, s.chunk);
+  const Geo g = geo_of_unit(s, unit);
   if (NEAR && on_axis(g)) return;
   const int n = g.n, nl = max(0, g.jhi - g.jlo + 1);
   const double t0 = (g.tfirst + (double)sub * s.sub_bins) / n - g.toff;
@@ -607,45 +613,68 @@ __device__ __forceinline__ double slow_rows(const ProfSeg &s, const Geo &g, cons
   return add;
 }
 
-// One block per plane that the rows role has marked in a unit: its rows once
-// more, 32 to a warp, those that need more than the table worked out; the
-// warps' sums are added in order.  Around theta = pi/2 every plane can have such
-// a row and a few have nothing else, which is why they are spread over the
-// whole device instead of holding up the warp that met them.
+// The planes that the rows role has marked in their units: their rows once more,
+// those that need more than the table worked out.  A warp per plane, as a rule for
+// one or two such rows; at theta = pi/2, where all rows of a plane have one t and
+// can all lie on a boundary and each then takes a warp ~5 us, the block's warps
+// share the plane's rows and their sums are added in order (56^3, 11 x 22 x 78:
+// 171 us with 8 warps and 32 rows each, 48 us with 16 that take every 16th).
+constexpr int kSlowThreads = 512;
+// A mark: segment (5 bits), which of its ranges of t (kMaxChunks bits), phi (16), plane (37).
+constexpr int kMarkSeg = 59, kMarkChunk = 53, kMarkPhi = 37;
+static_assert(kMarkChunk + kMaxChunks <= kMarkSeg, "marks");
+
 template <int S>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kSlowThreads)
     profile_slow_kernel(const __grid_constant__ wrt::ProfStep<S> st) {
-  __shared__ double s_sum[kThreads / 32];
+  __shared__ double s_sum[kSlowThreads / 32];
   const unsigned long long *list = st.list + 1;
   const long long count = (long long)st.list[0];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (long long k = blockIdx.x; k < count; k += gridDim.x) {
-    const unsigned long long item = list[k];
-    const ProfSeg &s = st.seg[S == 1 ? 0 : (int)(item >> 56)];
-    const ProfReq &r = s.r;
-    const int unit = (int)(item >> 40 & 0xffffu);
-    const long long plane = (long long)(item & 0xffffffffffull);
-    const int ndir = r.nphi * r.ntheta;
-    const int d = (int)(plane % ndir), is = (int)(plane / ndir);
-    const Geo g = geo_of(r, s.base0 + unit, s.chunk);
-    const RowGeo q = row_geo(r, g, d);
-    const double crop = (double)crop_of(r), sh = __ldg(r.shift + is);
-    const double u0 = fma(sh, q.ub, q.uo), w0 = fma(sh, q.wb, q.wo);
-    const bool mirrored = d >= (s.base0 + unit + 1) * r.ntheta;
-    int lo;
-    const int len = row_range(r, g, q, crop, sh, u0, w0, &lo);
-    double sum = 0.0;
-    for (int x = warp * 32; x < len; x += kThreads)
-      sum += slow_rows(s, g, q, unit, d, is, lo + x + lane, x + lane < len, u0, w0, crop, mirrored);
-    sum = wrtd::warp_sum(sum);
-    if (lane == 0) s_sum[warp] = sum;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double v = 0.0;
-      for (int w = 0; w < kThreads / 32; ++w) v += s_sum[w];
-      r.out[plane] += v / ((double)r.n * r.n);
+  constexpr int kW = kSlowThreads / 32;
+  for (int pass = 0; pass < 2; ++pass) {
+    const bool together = pass == 1;
+    const long long first = together ? blockIdx.x : (long long)blockIdx.x * kW + warp;
+    const long long step = together ? gridDim.x : (long long)gridDim.x * kW;
+    for (long long k = first; k < count; k += step) {
+      const unsigned long long item = list[k];
+      const ProfSeg &s = st.seg[S == 1 ? 0 : (int)(item >> kMarkSeg)];
+      const ProfReq &r = s.r;
+      const int phi = (int)(item >> kMarkPhi & 0xffffu);
+      const long long plane = (long long)(item & ((1ull << kMarkPhi) - 1));
+      const int ndir = r.nphi * r.ntheta;
+      const int d = (int)(plane % ndir), is = (int)(plane / ndir);
+      if ((fabs(__ldg(r.dir + 9 * (size_t)d + 2)) < 1e-9) != together) continue;  // cos theta
+      const double crop = (double)crop_of(r), sh = __ldg(r.shift + is);
+      const bool mirrored = d >= (s.base0 + phi + 1) * r.ntheta;
+      double sum = 0.0;
+      for (int c = 0; c < s.nchunk; ++c) {
+        if (!(item >> (kMarkChunk + c) & 1u)) continue;
+        const Geo g = geo_of(r, s.base0 + phi, s.chunk + c);
+        const RowGeo q = row_geo(r, g, d);
+        const double u0 = fma(sh, q.ub, q.uo), w0 = fma(sh, q.wb, q.wo);
+        int lo;
+        const int len = row_range(r, g, q, crop, sh, u0, w0, &lo);
+        const int x0 = together ? warp + kW * lane : lane, dx = together ? kSlowThreads : 32;
+        for (int x = x0; x - x0 < len; x += dx)
+          sum += slow_rows(s, g, q, c * s.nbase + phi, d, is, lo + x, x < len, u0, w0, crop,
+                           mirrored);
+      }
+      sum = wrtd::warp_sum(sum);
+      const double scale = 1.0 / ((double)r.n * r.n);
+      if (!together) {
+        if (lane == 0) r.out[plane] += sum * scale;
+        continue;
+      }
+      if (lane == 0) s_sum[warp] = sum;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double v = 0.0;
+        for (int w = 0; w < kW; ++w) v += s_sum[w];
+        r.out[plane] += v * scale;
+      }
+      __syncthreads();
     }
-    __syncthreads();
   }
 }
 
@@ -755,35 +784,39 @@ template <bool NEAR>
 __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long *list,
                           char *smem) {
   const ProfReq &r = s.r;
-  const int unit = blk / s.blk_rows, tile = blk % s.blk_rows;
-  const int base = s.base0 + unit;
-  const Geo g = geo_of(r, base, s.chunk);
-  if (NEAR && on_axis(g)) return;
+  const int phi = blk / s.blk_rows, tile = blk % s.blk_rows, base = s.base0 + phi;
   const int tid = threadIdx.x, lane = tid & 31;
-  const unsigned *gstart = s.start + (size_t)unit * (kUnitBins + 8);
-  const unsigned *gpos = s.pos + (size_t)unit * (s.cap + 16);
-  unsigned *pos = reinterpret_cast<unsigned *>(smem);
-  const int total = gstart[kUnitBins];
-  unsigned short *start = reinterpret_cast<unsigned short *>(pos + s.cap + 16);
-  for (int k = tid; k < total + 16; k += kThreads) pos[k] = gpos[k];
-  for (int k = tid; k <= kUnitBins; k += kThreads) start[k] = (unsigned short)gstart[k];
-  __syncthreads();
-  const int n = r.n, W = g.W;
+  const int n = r.n, ndir = r.nphi * r.ntheta;
   const double crop = (double)crop_of(r);
-  const int ndir = r.nphi * r.ntheta;
   const int sgroups = (r.nshift + 31) / 32;
-  const int warps = sgroups * r.ntheta * (r.paired ? 2 : 1);
-  const char *table = static_cast<const char *>(s.table) +
-                      (size_t)unit * s.cap * n * (NEAR ? 4 : 16);
-  for (int rep = 0; rep < kRowTiles; ++rep) {
-    const int wi = (tile * kRowTiles + rep) * (kThreads / 32) + (tid >> 5);
-    if (wi >= warps) break;
-    const int half = wi / (sgroups * r.ntheta), q = wi - half * sgroups * r.ntheta;
-    // the thetas nearest pi/2 first: their warps have the most rows to walk
-    const int rank = q / sgroups, is0 = (q - rank * sgroups) * 32;
-    const int it = (r.ntheta - 1) / 2 + (rank & 1 ? (rank + 1) / 2 : -(rank / 2));
-    const int np = min(32, r.nshift - is0);
-    const int d = (base + half * (r.nphi / 2)) * r.ntheta + it;
+  const int wi = tile * (kThreads / 32) + (tid >> 5);
+  const bool live = wi < sgroups * r.ntheta * (r.paired ? 2 : 1);
+  const int half = wi / (sgroups * r.ntheta), ws = wi - half * sgroups * r.ntheta;
+  // the thetas nearest pi/2 first: their warps have the most rows to walk
+  const int rank = ws / sgroups, is0 = (ws - rank * sgroups) * 32;
+  const int it = (r.ntheta - 1) / 2 + (rank & 1 ? (rank + 1) / 2 : -(rank / 2));
+  const int np = live ? min(32, r.nshift - is0) : 0;
+  const int d = live ? (base + half * (r.nphi / 2)) * r.ntheta + it : 0;
+  double mine = 0.0;   // the sum of plane `lane`
+  unsigned marks = 0;  // ranges where a row of it is not decided by the table alone
+  bool some = false;   // it has rows here
+  for (int c = 0; c < s.nchunk; ++c) {
+    const Geo g = geo_of(r, base, s.chunk + c);
+    if (NEAR && on_axis(g)) return;
+    const int unit = c * s.nbase + phi;
+    const unsigned *gstart = s.start + (size_t)unit * (kUnitBins + 8);
+    const unsigned *gpos = s.pos + (size_t)unit * (s.cap + 16);
+    unsigned *pos = reinterpret_cast<unsigned *>(smem);
+    const int total = gstart[kUnitBins];
+    unsigned short *start = reinterpret_cast<unsigned short *>(pos + s.cap + 16);
+    if (c) __syncthreads();
+    for (int k = tid; k < total + 16; k += kThreads) pos[k] = gpos[k];
+    for (int k = tid; k <= kUnitBins; k += kThreads) start[k] = (unsigned short)gstart[k];
+    __syncthreads();
+    if (!live) continue;
+    const int W = g.W;
+    const char *table = static_cast<const char *>(s.table) +
+                        (size_t)unit * s.cap * n * (NEAR ? 4 : 16);
     const RowGeo w = row_geo(r, g, d);
     // ---- row ranges, lane = plane
     int lo = 1, len = 0;
@@ -795,9 +828,9 @@ __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long
       len = row_range(r, g, w, crop, sh, u0, w0, &lo);
     }
     const int most = (int)__reduce_max_sync(kAll, (unsigned)len);
-    if (!most && !s.first) continue;
-    bool flag = false;  // a row of plane `lane` that the table alone does not decide
-    double mine = 0.0;  // the sum of plane `lane`
+    if (!most) continue;
+    some |= len > 0;
+    bool flag = false;
     if (most <= kLongRows) {
       double di = (double)lo;
       for (int x = 0; x < most; x += 4, di += 4.0)
@@ -815,21 +848,12 @@ __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long
         acc = wrtd::warp_sum(acc);
         mark = __any_sync(kAll, mark);
         if (lane == p) {
-          mine = acc;
+          mine += acc;
           flag |= mark;
         }
       }
     }
-    if (lane < np) {
-      double *o = r.out + (size_t)(is0 + lane) * ndir + d;
-      const double v = mine / ((double)n * n);
-      if (s.first) *o = v;
-      else if (len > 0) *o += v;
-      if (flag)
-        list[1 + atomicAdd(list, 1ull)] = (unsigned long long)seg << 56 |
-                                          (unsigned long long)unit << 40 |
-                                          (unsigned long long)(is0 + lane) * ndir + d;
-    }
+    marks |= (flag ? 1u : 0u) << c;
     if (r.counter) {
       unsigned long long counted = 0;
       for (int x = 0; x < len; ++x)
@@ -837,6 +861,15 @@ __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long
       if (counted) atomicAdd(r.counter, counted);
     }
   }
+  if (lane >= np) return;
+  const unsigned long long plane = (unsigned long long)(is0 + lane) * ndir + d;
+  const double v = mine / ((double)n * n);
+  if (s.first) r.out[plane] = v;
+  else if (some) r.out[plane] += v;
+  if (marks)
+    list[1 + atomicAdd(list, 1ull)] = (unsigned long long)seg << kMarkSeg |
+                                      (unsigned long long)marks << kMarkChunk |
+                                      (unsigned long long)phi << kMarkPhi | plane;
 }
 
 // Samples that no table holds, one warp per plane (lanes on its rows), added to
@@ -881,8 +914,8 @@ __global__ void __launch_bounds__(kThreads)
   int b = (int)blockIdx.x;
   for (int k = 0; k < st.n; ++k) {
     const ProfSeg &s = st.seg[k];
-    if (b < s.nbase) return role_sort(s, b, smem);
-    b -= s.nbase;
+    if (b < s.nbase * s.nchunk) return role_sort(s, b, smem);
+    b -= s.nbase * s.nchunk;
   }
 }
 
@@ -893,7 +926,7 @@ __global__ void __launch_bounds__(kThreads, 3)
   int b = (int)blockIdx.x;
   for (int k = 0; k < st.n; ++k) {
     const ProfSeg &s = st.seg[k];
-    const int nb = s.nsub * s.nbase;
+    const int nb = s.nsub * s.nbase * s.nchunk;
     if (b < nb) {
       if (NEAR || s.r.storage != WRT_STORAGE_BF16)
         role_build<NEAR>(s, b, static_cast<const float *>(s.r.vol), smem);
@@ -960,6 +993,23 @@ struct Areas {
 };
 
 constexpr int kManySegs = 24;
+static_assert(kManySegs <= 32, "marks");
+
+// Ranges of t that are computed together: a small volume's all in one step (64^3
+// with 14 x 28 directions 600 -> 240 us), where a large one's fill the device one by
+// one (128^3 in groups of two 5.7 -> 6.4 ms).  By the size alone, because the order in
+// which a plane's sum is added up follows it.
+int chunk_group(int n) {
+  return n <= 64 ? 4 : 1;
+}
+
+// The ranges of t in which data within the crop bound has rows.
+void chunk_range(const ProfReq &r, float crop, int *c0, int *c1) {
+  const double h = 0.5 * (r.nearest ? r.n : r.n - 1), toff = prof_t_off(r.n, r.nearest);
+  const double tmax = std::min(std::sqrt((double)crop), 1.4142135623730952) * h + 1e-3;
+  *c0 = std::max(0, (int)std::floor((toff - tmax) * r.n / kUnitBins));
+  *c1 = (int)std::floor((toff + tmax) * r.n / kUnitBins) + 1;
+}
 
 template <bool NEAR, int S>
 cudaError_t launch_step(wrt_ctx *ctx, cudaStream_t stream, const std::vector<ProfSeg> &segs,
@@ -973,8 +1023,8 @@ cudaError_t launch_step(wrt_ctx *ctx, cudaStream_t stream, const std::vector<Pro
   for (int k = 0; k < st.n; ++k) {
     st.seg[k] = segs[k];
     cap = std::max(cap, segs[k].cap);
-    sort += segs[k].nbase;
-    build += (long long)segs[k].nsub * segs[k].nbase;
+    sort += segs[k].nbase * segs[k].nchunk;
+    build += (long long)segs[k].nsub * segs[k].nbase * segs[k].nchunk;
     rows += (long long)segs[k].blk_rows * segs[k].nbase;
     n = std::max(n, segs[k].r.n);
   }
@@ -993,7 +1043,7 @@ cudaError_t launch_step(wrt_ctx *ctx, cudaStream_t stream, const std::vector<Pro
   profile_sort_kernel<S><<<(unsigned)sort, kThreads, kUnitBins * 8, stream>>>(st);
   profile_build_kernel<NEAR, S><<<(unsigned)build, th_build, sm_build, stream>>>(st);
   profile_rows_kernel<NEAR, S><<<(unsigned)rows, kThreads, sm_rows, stream>>>(st);
-  profile_slow_kernel<S><<<ctx->sm_count * 2, kThreads, 0, stream>>>(st);
+  profile_slow_kernel<S><<<ctx->sm_count * 2, kSlowThreads, 0, stream>>>(st);
   ctx->launches += 4;
   return cudaGetLastError();
 }
@@ -1009,36 +1059,46 @@ bool profile_covers(int n, int nphi, int ntheta, int nshift) {
 }
 
 // A phi's tables cost ~2.5 n^2 pieces x n layers whatever is read from them, the
-// staged kernel its rows x samples, so what decides is rows per layer and piece,
-// ntheta nshift / n.  Measured against the staged kernel on 110 random sizes (n
-// 8 .. 176, 3 .. 64 latitudes, 8 .. 256 shifts): trilinear 0.5-1.0 of its speed
-// at 5-10, 0.8-1.5 at 12-20, 2-10 times beyond 30; nearest (whose phis on an axis
-// stay with the staged kernel) even at 30-40.  Small requests are launch-bound
-// either way: below 4000 planes the staged kernel's one launch wins.
+// staged kernel its rows x samples, so what decides is the rows per layer of a
+// table, ntheta nshift / n (half that where phi + pi has tables of its own); few phis
+// of a large volume leave most of the device idle while they are built.  Against
+// the staged kernel on 110 random sizes past the line (n 10 .. 176, 3 .. 64 latitudes,
+// 8 .. 256 shifts, 4000 planes up): 0.93 of its speed at worst, 1.05-2.5 times within a
+// fifth of the line, 2-4 times at twice; just below it 0.5-1.3 times for n > 100, up
+// to 2.5 for n < 60.  The nearest sampler's (whose phis on an axis stay with the staged
+// kernel) are even at 30-40.  Below 4000 planes both are launches: 0.7-1.6 times.
 bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift, bool nearest) {
   if (!profile_covers(n, nphi, ntheta, nshift)) return false;
   if (ctx->staged_config >= 0) return ctx->staged_config == kNumStagedConfigs - 1;
-  const long long rows = (long long)ntheta * nshift;
-  return rows >= (nearest ? 40LL : 14LL) * n && rows * nphi >= 4000;
+  const double rows = (double)ntheta * nshift;
+  if (rows * nphi < 4000) return false;
+  if (nearest) return rows >= 40.0 * n;
+  const bool paired = nphi % 2 == 0;
+  return rows * (paired ? 1.0 : 0.5) >= n * (7.0 + 0.4 * n / (paired ? nphi / 2 : nphi));
 }
 
 // The least workspace a request can be computed in: that of one unit.
 size_t profile_workspace_least(const ProfReq &r, float crop) {
   size_t ws = 1 << 20;
-  while (!Areas(ws).fits(unit_bytes(r, crop), 1, UnitBytes())) ws += ws / 16;
+  while (!Areas(ws).fits(unit_bytes(r, crop), chunk_group(r.n), UnitBytes())) ws += ws / 16;
   return ws;
 }
 
-// The workspace a set of requests asks for: enough units to fill a step, no
-// more than they have.
+// The workspace a set of requests asks for: all units at once, or enough to fill a
+// step.
 size_t profile_workspace_want(const ProfReq *reqs, const float *crop, int nreq) {
   size_t table = 0, least = 0;
   for (int q = 0; q < nreq; ++q) {
     const ProfReq &r = reqs[q];
-    table += unit_bytes(r, crop[q]).table * (r.paired ? r.nphi / 2 : r.nphi);
+    const int nbase = r.paired ? r.nphi / 2 : r.nphi;
+    int c0, c1;
+    chunk_range(r, crop[q], &c0, &c1);
+    const size_t u = unit_bytes(r, crop[q]).table;
+    // a lane's share of a single request is whole phis
+    table += u * std::min(c1 - c0, chunk_group(r.n)) * (nreq == 1 ? (nbase + kProfLanes - 1) / kProfLanes * kProfLanes : nbase);
     least = std::max(least, profile_workspace_least(r, crop[q]));
   }
-  return std::max(least, std::min(table, kProfTableBytes) / 176 * 256 + (1 << 20));
+  return std::max(least, std::min(table, kProfTableBytes) / 176 * 256 + (4 << 20));
 }
 
 int profile_lanes_init(wrt_ctx *ctx, ProfLanes *l) {
@@ -1063,7 +1123,7 @@ void profile_lanes_release(ProfLanes *l) {
 }
 
 int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const ProfReq *reqs,
-                    const float *crop, int nreq, void *ws, size_t ws_bytes) {
+                    const float *crop, int nreq, void *ws, size_t ws_bytes, bool forked) {
   if (nreq < 1) return WRT_OK;
   const bool near = reqs[0].nearest != 0;
   // ---- lanes: the launches of a step depend on one another and each ends with
@@ -1072,15 +1132,20 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
   size_t table = 0;
   for (int q = 0; q < nreq; ++q)
     table += unit_bytes(reqs[q], crop[q]).table * (reqs[q].paired ? reqs[q].nphi / 2 : reqs[q].nphi);
-  int nl = table >= kProfLaneBytes ? kProfLanes : 1;
+  const int most = forked ? kProfLanes - 1 : kProfLanes;
+  int nl = table >= kProfLaneBytes ? most : 1;
   for (int q = 0; q < nreq; ++q)  // every request has to fit a lane
-    while (nl > 1 && !Areas(ws_bytes / nl & ~(size_t)255).fits(unit_bytes(reqs[q], crop[q]), 1,
-                                                               UnitBytes()))
+    while (nl > 1 && !Areas(ws_bytes / nl & ~(size_t)255)
+                          .fits(unit_bytes(reqs[q], crop[q]), chunk_group(reqs[q].n), UnitBytes()))
       --nl;
-  if (nl > 1) {
+  if (nl > 1 && !forked) {
     int st = profile_lanes_init(ctx, lanes);
     if (st) return st;
   }
+  // lane l's stream: the caller's is lane 0 unless it has other work
+  auto lane_of = [&](int l) {
+    return forked ? lanes->stream[l] : l ? lanes->stream[l - 1] : stream;
+  };
   const size_t share = ws_bytes / nl & ~(size_t)255;
   const Areas area(share);
   // ---- jobs: groups of phis of one request, dealt to the lanes
@@ -1088,39 +1153,42 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
     int req, base0, nbase, c0, c1, c;
   };
   std::vector<std::vector<Job>> jobs(nl);
+  std::vector<int> home(nreq);  // the lane of all of a request's jobs, or -1
   size_t dealt = 0;
   for (int q = 0; q < nreq; ++q) {
     const ProfReq &r = reqs[q];
-    const double h = 0.5 * (r.nearest ? r.n : r.n - 1), toff = prof_t_off(r.n, r.nearest);
-    const double tmax = std::min(std::sqrt((double)crop[q]), 1.4142135623730952) * h + 1e-3;
     const UnitBytes b = unit_bytes(r, crop[q]);
     const int nbase = r.paired ? r.nphi / 2 : r.nphi;
     int fit = 1;
-    while (fit < nbase && fit < 0xffff && area.fits(b, fit + 1, UnitBytes())) ++fit;
+    const int group = chunk_group(r.n);
+    while (fit < nbase && fit < 0xffff && area.fits(b, (size_t)group * (fit + 1), UnitBytes())) ++fit;
     int groups = (nbase + fit - 1) / fit;
     if (nreq == 1 && nl > 1 && nbase >= nl) groups = (groups + nl - 1) / nl * nl;
     groups = std::min(groups, nbase);
+    home[q] = groups == 1 ? (int)(dealt % nl) : -1;
     for (int k = 0; k < groups; ++k) {
       Job j;
       j.req = q;
       j.base0 = (int)((long long)nbase * k / groups);
       j.nbase = (int)((long long)nbase * (k + 1) / groups) - j.base0;
-      j.c0 = std::max(0, (int)std::floor((toff - tmax) * r.n / kUnitBins));
-      j.c1 = (int)std::floor((toff + tmax) * r.n / kUnitBins) + 1;
+      chunk_range(r, crop[q], &j.c0, &j.c1);
       j.c = j.c0;
       jobs[dealt++ % nl].push_back(j);
     }
   }
   cudaError_t e = cudaSuccess;
-  if (nl > 1) {
-    e = cudaEventRecord(lanes->fork, stream);
-    for (int k = 1; k < nl && e == cudaSuccess; ++k)
-      e = cudaStreamWaitEvent(lanes->stream[k - 1], lanes->fork, 0);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "profile fork");
-  }
-  // ---- steps, lane by lane: of every job still open one range of t (a range
-  // adds to the sums of the one before, so they go to different steps), as many
-  // jobs as the lane's workspace holds
+  if (nl > 1 && !forked) e = cudaEventRecord(lanes->fork, stream);
+  for (int l = forked ? 0 : 1; l < nl && e == cudaSuccess; ++l)
+    e = cudaStreamWaitEvent(lane_of(l), lanes->fork, 0);
+  // nothing may still use the workspace when a failed call returns
+  auto failed = [&](const char *what) {
+    for (int l = 0; l < nl; ++l) cudaStreamSynchronize(lane_of(l));
+    return cuda_fail(ctx, e, what);
+  };
+  if (e != cudaSuccess) return failed("profile fork");
+  // ---- steps, lane by lane: of every job still open one group of ranges of t (a
+  // group adds to the sums of the one before, so they go to different steps), as
+  // many jobs as the lane's workspace holds
   std::vector<ProfSeg> out;
   for (bool any = true; any;) {
     any = false;
@@ -1134,10 +1202,13 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
         if (j.c >= j.c1) continue;
         const ProfReq &r = reqs[j.req];
         const UnitBytes u = unit_bytes(r, crop[j.req]);
-        if ((int)out.size() >= kManySegs || !area.fits(u, j.nbase, had)) break;
+        const int group = chunk_group(r.n), nc = std::min(j.c1, (j.c / group + 1) * group) - j.c;
+        if ((int)out.size() >= kManySegs || !area.fits(u, (size_t)j.nbase * nc, had)) break;
+        const size_t units = (size_t)j.nbase * nc;
         ProfSeg s = {};
         s.r = r;
         s.chunk = j.c;
+        s.nchunk = nc;
         s.base0 = j.base0;
         s.nbase = j.nbase;
         s.first = j.c == j.c0;
@@ -1151,49 +1222,56 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
         s.rec = rec + had.rec;
         s.keys = reinterpret_cast<unsigned long long *>(keys + had.keys);
         s.pos = reinterpret_cast<unsigned *>(place + had.pos + had.start);
-        s.ids = s.pos + (size_t)(s.cap + 16) * j.nbase;
-        s.start = reinterpret_cast<unsigned *>(place + had.pos + had.start + u.pos * j.nbase);
-        had.table += u.table * j.nbase;
-        had.rec += u.rec * j.nbase;
-        had.keys += u.keys * j.nbase;
-        had.pos += u.pos * j.nbase;
-        had.start += u.start * j.nbase;
-        had.list += u.list * j.nbase;
+        s.ids = s.pos + (size_t)(s.cap + 16) * units;
+        s.start = reinterpret_cast<unsigned *>(place + had.pos + had.start + u.pos * units);
+        had.table += u.table * units;
+        had.rec += u.rec * units;
+        had.keys += u.keys * units;
+        had.pos += u.pos * units;
+        had.start += u.start * units;
+        had.list += u.list * units;
         out.push_back(s);
-        ++j.c;
+        j.c += nc;
       }
       if (out.empty()) continue;
       any = true;
-      const cudaStream_t ls = l ? lanes->stream[l - 1] : stream;
+      const cudaStream_t ls = lane_of(l);
       if (near)
         e = out.size() == 1 ? launch_step<true, 1>(ctx, ls, out, list)
                             : launch_step<true, kManySegs>(ctx, ls, out, list);
       else
         e = out.size() == 1 ? launch_step<false, 1>(ctx, ls, out, list)
                             : launch_step<false, kManySegs>(ctx, ls, out, list);
-      if (e != cudaSuccess) return cuda_fail(ctx, e, "row-sum profile kernels");
+      if (e != cudaSuccess) return failed("row-sum profile kernels");
     }
   }
-  for (int k = 1; k < nl; ++k) {
-    e = cudaEventRecord(lanes->done[k - 1], lanes->stream[k - 1]);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, lanes->done[k - 1], 0);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "profile join");
-  }
-  for (int q = 0; q < nreq; ++q) {
+  // samples that no table holds: behind the request's last step where that is
+  // one lane's, else behind the join
+  auto extra = [&](int q, cudaStream_t where) {
     const ProfReq &r = reqs[q];
     // the nearest sampler's phis on an axis are not tabulated at all
-    if (r.nearest && !r.paired) continue;
+    if (r.nearest && !r.paired) return cudaSuccess;
     const double left = (double)crop[q] * r.n * r.n;
     const bool axis = !r.nearest && ((r.n & 1) || (double)r.n * r.n <= left);
-    if (!axis && !(r.paired && (double)r.L * r.L <= left)) continue;
+    if (!axis && !(r.paired && (double)r.L * r.L <= left)) return cudaSuccess;
     const long long planes = (long long)r.nphi * r.ntheta * r.nshift;
     profile_extra_kernel<<<(unsigned)((planes + kThreads / 32 - 1) / (kThreads / 32)), kThreads, 0,
-                           stream>>>(r);
+                           where>>>(r);
     ctx->launches++;
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "profile_extra_kernel");
+    return cudaGetLastError();
+  };
+  for (int q = 0; q < nreq && e == cudaSuccess; ++q)
+    if (home[q] >= 0) e = extra(q, lane_of(home[q]));
+  const cudaStream_t home_stream = lane_of(0);
+  for (int l = 1; l < nl && e == cudaSuccess; ++l) {
+    const int k = forked ? l : l - 1;
+    e = cudaEventRecord(lanes->done[k], lanes->stream[k]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(home_stream, lanes->done[k], 0);
   }
-  return WRT_OK;
+  for (int q = 0; q < nreq && e == cudaSuccess; ++q)
+    if (home[q] < 0) e = extra(q, home_stream);
+  if (forked && e == cudaSuccess) e = cudaEventRecord(lanes->done[0], home_stream);
+  return e == cudaSuccess ? WRT_OK : failed("row-sum profiles");
 }
 
 }  // namespace wrt

@@ -40,13 +40,18 @@ PROF_HD inline double prof_t_off(int n, bool nearest) {
 }
 
 // Most piece boundaries a unit can hold for data cropped at squared radius
-// `crop`: per cell of t the lines (chord / spacing, the chord at most 2 sqrt(crop)
-// half edges or the square's diagonal) times their crossings (sqrt 2 per cell),
-// i.e. at most 4 n; and every line's first and last crossing may round into the
-// unit.
+// `crop` (half edges): a length of line crosses at most sqrt 2 boundaries per cell,
+// lines are half a cell apart.  Per cell of t that is the chord (at most 2
+// sqrt(crop) half edges or the square's diagonal) times 2 sqrt 2, at most 4 n; over
+// all t the area (the square's or the disc's).  Every line's first and last
+// crossing may round into the unit; sub-range starts count too.
 PROF_HD inline int unit_cap(int n, double crop) {
   const double r = sqrt(crop < 2.0 ? crop : 2.0);
-  return (int)(2.8284272 * r * kUnitBins) + 8 * n + 64;
+  const double strip = 2.8284272 * r * kUnitBins;
+  const double disc = 0.7853982 * crop < 1.0 ? 0.7853982 * crop : 1.0;
+  const double area = 2.8284272 * disc * ((double)n + 2) * (n + 2);
+  const int sub = n < kUnitBins ? n : kUnitBins;
+  return (int)(strip < area ? strip : area) + 8 * n + 64 + (kUnitBins + sub - 1) / sub;
 }
 
 struct PieceRec {   // one piece boundary, read by whole warps of the build role

@@ -252,15 +252,15 @@ struct ProfReq {            // one plane transform
   int n, L, nphi, ntheta, nshift, storage, nearest;
   int paired;               // phi and phi + pi share their tables
 };
-struct ProfSeg {            // the units (consecutive phis, one range of t) of one request in a step
+struct ProfSeg {            // the units (nchunk ranges of t x nbase phis) of one request in a step
   ProfReq r;
   void *table, *rec;        // [unit][cap][n] coefficients; [unit][cap] piece records
   unsigned *pos, *ids;      // [unit][cap + 16] piece starts; what starts there
   unsigned *start;          // [unit][kUnitBins + 8] first piece of a bin
   unsigned long long *keys; // [unit][cap]
-  int chunk, base0, nbase, first;
+  int chunk, nchunk, base0, nbase, first;
   int cap, nsub, sub_bins;
-  int blk_rows;             // blocks of the rows role per unit
+  int blk_rows;             // blocks of the rows role per phi
 };
 template <int S>
 struct ProfStep {
@@ -269,11 +269,9 @@ struct ProfStep {
   int n;
 };
 // Whether phi and phi + pi share tables: their lattices differ by one end sample
-// (-L for L), which lies outside any crop ball for L >= 1.75 n, and outside that
-// of data in the unit ball for L >= n unless the grid is coarse.
-inline bool profile_paired(int n, int nphi, int L) {
-  return nphi % 2 == 0 && (L >= 1.75 * n || (L >= n && n >= 40));
-}
+// (-L for L), which the extra kernel exchanges where it lies in the crop ball:
+// few rows or none for L >= n, most rows of shorter lattices.
+inline bool profile_paired(int n, int nphi, int L) { return nphi % 2 == 0 && L >= n; }
 // Whether the sizes of a request suit the profiles, and whether a request goes
 // there under the context's tile configuration (the same rule for a request
 // alone, in a batch and in the server).
@@ -286,9 +284,11 @@ bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift, 
 // it limits which empty ranges of t are visited and the room for pieces).  ws: at least profile_workspace_least for every
 // request.
 // lanes: streams for side-by-side steps, created on first use; the work is
-// forked from `stream` and joined to it again.
+// forked from `stream` and joined to it again.  forked: on side streams only, which
+// wait for lanes->fork (recorded by the caller); the caller's stream has to wait
+// for lanes->done[0] afterwards.
 int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const ProfReq *reqs,
-                    const float *crop, int nreq, void *ws, size_t ws_bytes);
+                    const float *crop, int nreq, void *ws, size_t ws_bytes, bool forked = false);
 int profile_lanes_init(wrt_ctx *ctx, ProfLanes *l);
 void profile_lanes_release(ProfLanes *l);
 
