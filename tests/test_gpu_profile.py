@@ -100,6 +100,17 @@ def test_tight_budget_takes_the_staged_kernel():
     assert rel_l2(got, ref) < TOL_L2
 
 
+@pytest.mark.parametrize("n,grid", [(64, (8, 16, 64)), (31, (12, 9, 70)), (45, (4, 33, 40))])
+def test_nearest_in_little_memory(n, grid):
+    # the tables of phis on an axis in several groups of cells
+    vol = _volume("noise", n)
+    with wrt.Context(0, budget_bytes=24 << 20) as c:
+        got = c.radon_grid(vol, *grid, sampler=wrt.NEAREST, half_extent=n)
+    ref = O.radon_forward(vol, *grid, sampler=O.NEAREST, half_extent=n)
+    assert rel_l2(got, ref) < TOL_L2
+    assert rel_max(got, ref) < TOL_MAX
+
+
 # ---- backprojection from merged splines (csrc/k_backproj.cu): just beyond the
 # sizes of the allocation-free path; odd longitudes (nothing merged), longitudes
 # not a multiple of 32, odd latitudes, one voxel tile and several, few knots

@@ -651,11 +651,8 @@ namespace {
 
 // Staged-kernel launch of one request; see k_staged.cu.  Trilinear: the
 // volume's layer pairs; nearest: its z-major cell layers (FP32 storage).
-// phis / nphis: the planes of these phis only (the others are zeroed), all
-// when nphis is 0.
 int radon_forward_staged(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, int L,
-                         double *dev_out, bool nearest, const int *phis = nullptr,
-                         int nphis = 0) {
+                         double *dev_out, bool nearest) {
   int st = nearest ? volume_ensure_layers(vol) : volume_ensure_pairs(vol);
   if (st) return st;
   const int n = vol->n;
@@ -687,8 +684,7 @@ int radon_forward_staged(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, in
   StagedItem *d_items = nullptr;
   const int *d_nitems = nullptr;
   int nitems = 0;
-  st = staged_items_cached(ctx, n, th, r.crop_r2, r.ndir, &d_items, &d_nitems, &nitems, nearest,
-                           phis, nphis, grid->ntheta);
+  st = staged_items_cached(ctx, n, th, r.crop_r2, r.ndir, &d_items, &d_nitems, &nitems, nearest);
   if (st) return st;
   st = staged_scratch(ctx, sizeof(StagedReq));
   if (st) return st;
@@ -704,9 +700,6 @@ int radon_forward_staged(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, in
     if (st) return st;
   }
   const double delta = 1.0 / n;
-  if (nphis)
-    return plane_finalize_phis(ctx, dev_out, phis, nphis, grid->nphi, grid->ntheta, grid->nshift,
-                               delta * delta / r.scale);
   return plane_finalize(ctx, dev_out, (long long)nout, delta * delta / r.scale);
 }
 
@@ -759,16 +752,11 @@ int radon_forward_profile(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, i
   if (profile_ws(ctx, &r, &crop, 1, &ws, &bytes)) return WRT_OK;  // no room: the staged kernel
   *done = true;
   if (nearest) {
-    // phis on an axis: half of every row's samples lie on a cell boundary for
-    // every t, so no table serves them
     int phis[4], m = 0;
     for (int p = 0; p < grid->nphi; ++p)
       if ((fabs(cos(grid->phi[p])) < 1e-9 || fabs(sin(grid->phi[p])) < 1e-9) && m < 4)
         phis[m++] = p;
-    if (m) {
-      int st = radon_forward_staged(ctx, vol, grid, L, dev_out, true, phis, m);
-      if (st) return st;
-    }
+    return profile_forward_nearest(ctx, ctx->stream, &ctx->prof_lanes, r, crop, phis, m, ws, bytes);
   }
   return profile_forward(ctx, ctx->stream, &ctx->prof_lanes, &r, &crop, 1, ws, bytes);
 }
@@ -799,7 +787,7 @@ int wrt_radon_forward_device(wrt_ctx *ctx, const wrt_volume *cvol, const wrt_gri
   if (o.kernel == WRT_KERNEL_STAGED && !staged_ok)
     return fail(ctx, WRT_ERR_INVALID_ARGUMENT, "staged kernel: volume edge below 4");
   if (o.kernel != WRT_KERNEL_PLAIN && staged_ok) {
-    if (profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift, nearest)) {
+    if (profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift)) {
       bool done = false;
       st = radon_forward_profile(ctx, vol, grid, L, dev_out, nearest, &done);
       if (st || done) return st;
@@ -843,7 +831,7 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
         reqs[r].half_extent > 8 * vol->n)
       continue;  // refused below
     const int L = reqs[r].half_extent ? reqs[r].half_extent : 2 * vol->n;
-    if (!profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift, false)) continue;
+    if (!profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift)) continue;
     routed[r] = 1;
     prof.push_back(profile_request(ctx, vol, grid, L, false, reqs[r].dev_out));
     prof_crop.push_back(trilinear_crop_r2(vol->r2, vol->n));
@@ -887,13 +875,13 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
     a.prep = 0;
     batch_add_forward(b, q, a, trilinear_crop_r2(vol->r2, n));
   }
-  auto profiles = [&](bool forked) {
+  auto profiles = [&](ProfFork fork) {
     return prof.empty() ? WRT_OK
                         : profile_forward(ctx, ctx->stream, &ctx->prof_lanes, prof.data(),
                                           prof_crop.data(), (int)prof.size(), prof_ws, prof_bytes,
-                                          forked);
+                                          fork);
   };
-  if (b.fwd.empty()) return profiles(false);
+  if (b.fwd.empty()) return profiles(PROF_ALONE);
   if (!prof.empty()) {
     // beside the staged kernel, and before it: its blocks hold their SM until
     // the item list is empty, so they take what the profiles leave free
@@ -901,7 +889,7 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
     if (st) return st;
     cudaError_t e = cudaEventRecord(ctx->prof_lanes.fork, ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "profile fork");
-    st = profiles(true);
+    st = profiles(PROF_BESIDE);
     if (st) return st;
   }
   if (!ctx->batch_slot) {

@@ -537,6 +537,27 @@ __device__ __forceinline__ RowAt row_at(double di, double u0, double u1, double 
   return a;
 }
 
+// The nearest sampler's cell of one coordinate: -1 below the cube, n above.
+__device__ __forceinline__ int axis_cell(double x, int n, double width) {
+  if (fabs(x) > 1.0) return x < 0.0 ? -1 : n;
+  return min((int)__ddiv_rn(__dadd_rn(x, 1.0), width), n - 1);
+}
+
+// The nearest sampler's row on a cell face: its samples' z differ by the rounding of
+// v2's at most, so where the extremes share a cell by the reference's arithmetic
+// (which is monotone), all do.  At theta = pi/2 every other row of a plane is one.
+__device__ __noinline__ bool settle_layer(const ProfReq &r, int d, double sh, double di, RowAt *a) {
+  const double *D = r.dir + 9 * (size_t)d;
+  const double delta = 1.0 / r.n, width = __ddiv_rn(2.0, (double)r.n);
+  const double z = __dadd_rn(__dmul_rn(sh, __ldg(D + 2)), __dmul_rn(__dmul_rn(delta, __ldg(D + 5)), di));
+  const double c = fabs(__dmul_rn(__dmul_rn(delta, __ldg(D + 8)), (double)r.L));
+  const int lo = axis_cell(__dadd_rn(z, -c), r.n, width);
+  if (lo != axis_cell(__dadd_rn(z, c), r.n, width)) return false;
+  a->iz = lo;
+  a->layer = false;
+  return true;
+}
+
 // Rows lo .. lo + len - 1 of shift sh that can lie in the unit, the cube and the
 // crop ball.
 __device__ __forceinline__ int row_range(const ProfReq &r, const Geo &g, const RowGeo &w,
@@ -574,8 +595,10 @@ __device__ __forceinline__ double slow_rows(const ProfSeg &s, const Geo &g, cons
   const unsigned *ids = s.ids + (size_t)unit * (s.cap + 16);
   const unsigned *start = s.start + (size_t)unit * (kUnitBins + 8);
   const int total = start[kUnitBins], lane = threadIdx.x & 31, n = r.n;
-  const RowAt a = row_at((double)i, u0, q.u1, w0, q.w1);
+  RowAt a = row_at((double)i, u0, q.u1, w0, q.w1);
   act = act && a.in;
+  // a settled row is read here, the others' table values the fast pass has added
+  const bool settled = r.nearest && act && a.layer && settle_layer(r, d, __ldg(r.shift + is), (double)i, &a);
   bool whole = act && a.layer && a.iz >= -1 && a.iz <= g.W;
   double add = 0.0, val = 0.0;
   if (act && !a.layer && (unsigned)a.iz < (unsigned)g.W) {
@@ -583,9 +606,7 @@ __device__ __forceinline__ double slow_rows(const ProfSeg &s, const Geo &g, cons
     int q0 = e, q1 = e;
     while (q0 > 0 && a.fx - pos[q0 - 1] <= kBoundary && e - q0 <= kMaxWindow) --q0;
     while (q1 < total && pos[q1] - a.fx <= kBoundary && q1 - e <= kMaxWindow) ++q1;
-    if (q1 - q0 > kMaxWindow) {
-      whole = true;
-      // the table's value, which the fast pass has added
+    if (q1 - q0 > kMaxWindow || settled) {
       const size_t o = ((size_t)unit * s.cap + (e - 1)) * n + a.iz;
       if (r.nearest) {
         val = (double)__ldg(static_cast<const float *>(s.table) + o);
@@ -597,10 +618,17 @@ __device__ __forceinline__ double slow_rows(const ProfSeg &s, const Geo &g, cons
         const float vb = fmaf(td, fmaf(td, y.z, y.y), y.x);
         val = (double)fmaf(a.tz, vb - va, va);
       }
+    }
+    if (q1 - q0 > kMaxWindow) {
+      whole = true;
     } else if (q1 > q0) {
       const double t = (fma((double)i, q.u1, u0) - q.uo) / n;
       const double w = fma((double)i, q.w1, w0);
       add = boundary_terms(r, g, ids, q0, q1, a.fx, t, a.iz, w - (double)a.iz, d, is, i, mirrored);
+    }
+    if (settled) {
+      add += val;
+      val = 0.0;
     }
   }
   unsigned m = __ballot_sync(kAll, whole);
@@ -951,6 +979,257 @@ __global__ void __launch_bounds__(kThreads, 3)
   }
 }
 
+// ------------------------------- the nearest sampler's phis on a horizontal axis
+// There the lattice runs along a grid axis with every other sample on a cell
+// boundary, whatever t is, so that the reference's rounding decides half of the
+// cells.  With r the axis that the lattice runs along, the coordinate of sample j
+// is fl(e + c_j): c_j = fl(fl(delta v2_r) j) is the same for all planes with one
+// v2_r (a phi has two or three: the latitudes round it differently), and
+// e = fl(s u_r + ..) is the row's, a few 1e-16.  The cell is monotone in e, so each
+// boundary sample has one threshold; thresholds are few (the ties of a few binades),
+// and between two of them the row sum depends on the row's other two cells alone.
+// So a table [thresholds passed][cell][layer] of each v2_r serves all rows: one
+// read each.  128^3, 4 of 128 phis, 64 latitudes, 256 shifts: 0.09 ms for the
+// thresholds (four blocks, beside other kernels), 0.08 for the tables, 0.33 for the
+// rows, which wait for FP64 divisions and gathers; by the staged kernel, every other
+// sample in FP64, 11 ms.
+constexpr int kAxisFamilies = 8;  // values of v2_r; rows of others are summed sample by sample
+constexpr int kAxisSlots = 96;    // layers of a phi's table
+constexpr int kAxisThreads = 128;
+
+struct AxisHead {
+  double emax;      // no row's e is beyond
+  int run, nfam;    // axis of the lattice (0 or 1)
+  int slot0[kAxisFamilies], nrank[kAxisFamilies], nflip[kAxisFamilies];
+};
+struct AxisJob {
+  ProfReq r;
+  int phi[4];
+  int a0, na, first;  // cells of the fixed axis in the table; nothing added before
+  char *head;         // [phi] AxisHead and lists
+  size_t head_bytes;
+  float *table;       // [phi][slot][na][n]
+};
+struct AxisLists {
+  AxisHead *h;
+  double *thr, *step;  // [family][n + 4]: thresholds of samples in order; distinct ones
+  int *cell, *rank;    // the cell below; which distinct one
+  int *weight;         // [family][n]: samples in a cell below all thresholds
+  unsigned char *fam;  // [theta]
+};
+__host__ __device__ inline size_t axis_head_bytes(int n, int ntheta) {
+  return (sizeof(AxisHead) + (size_t)kAxisFamilies * ((n + 4) * 24 + n * 4) + ntheta + 255) &
+         ~(size_t)255;
+}
+__device__ __forceinline__ AxisLists axis_lists(const AxisJob &a, int p) {
+  const int n = a.r.n, m = kAxisFamilies * (n + 4);
+  AxisLists l;
+  l.h = reinterpret_cast<AxisHead *>(a.head + a.head_bytes * p);
+  l.thr = reinterpret_cast<double *>(l.h + 1);
+  l.step = l.thr + m;
+  l.cell = reinterpret_cast<int *>(l.step + m);
+  l.rank = l.cell + m;
+  l.weight = l.rank + m;
+  l.fam = reinterpret_cast<unsigned char *>(l.weight + kAxisFamilies * n);
+  return l;
+}
+
+// Doubles in order as integers and back.
+__device__ __forceinline__ long long order_of(double x) {
+  const long long b = __double_as_longlong(x);
+  return b >= 0 ? b : -(b & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double of_order(long long k) {
+  return k >= 0 ? __longlong_as_double(k) : -__longlong_as_double(-k);
+}
+
+// One block per phi: families and their thresholds.
+__global__ void __launch_bounds__(kThreads) axis_prepare_kernel(const AxisJob a) {
+  const ProfReq &r = a.r;
+  const AxisLists l = axis_lists(a, blockIdx.x);
+  const double *D = r.dir + 9 * (size_t)a.phi[blockIdx.x] * r.ntheta;
+  const int run = fabs(__ldg(D + 6)) < kAxis ? 1 : 0, tid = threadIdx.x, n = r.n;
+  const double delta = 1.0 / n, width = __ddiv_rn(2.0, (double)n);
+  __shared__ unsigned long long s_max;
+  __shared__ int s_pick, s_count;
+  if (tid == 0) s_max = 0;
+  __syncthreads();
+  for (int it = tid; it < r.ntheta; it += kThreads) {
+    // |s|, |i delta| <= sqrt(3) inside the cube
+    const double e = 1.75 * (fabs(__ldg(D + 9 * it + run)) + fabs(__ldg(D + 9 * it + 3 + run)));
+    atomicMax(&s_max, (unsigned long long)__double_as_longlong(e));
+    l.fam[it] = 255;
+  }
+  __syncthreads();
+  const double emax = __longlong_as_double((long long)s_max);
+  int slots = 0, f = 0;
+  for (; f < kAxisFamilies; ++f) {
+    if (tid == 0) {
+      s_pick = r.ntheta;
+      s_count = 0;
+    }
+    __syncthreads();
+    for (int it = tid; it < r.ntheta; it += kThreads)
+      if (l.fam[it] == 255) atomicMin(&s_pick, it);
+    for (int m = tid; m < n; m += kThreads) l.weight[f * n + m] = 0;
+    __syncthreads();
+    if (s_pick == r.ntheta) break;
+    const double v = __ldg(D + 9 * s_pick + 6 + run), step = __dmul_rn(delta, v);
+    for (int it = tid; it < r.ntheta; it += kThreads)
+      if (l.fam[it] == 255 && __ldg(D + 9 * it + 6 + run) == v) l.fam[it] = (unsigned char)f;
+    double *thr = l.thr + f * (n + 4), *raw = l.step + f * (n + 4);
+    int *cell = l.cell + f * (n + 4), *rank = l.rank + f * (n + 4);
+    const int jlo = max(-r.L, -n - 2), jhi = min(r.L - 1, n + 2);
+    for (int j = jlo + tid; j <= jhi; j += kThreads) {
+      const double c = __dmul_rn(step, (double)j);
+      const int lo = axis_cell(__dadd_rn(-emax, c), n, width);
+      if (lo >= 0 && lo < n) atomicAdd(&l.weight[f * n + lo], 1);
+      if (axis_cell(__dadd_rn(emax, c), n, width) == lo) continue;
+      long long x = order_of(-emax), y = order_of(emax);  // cell lo at x, not at y
+      while (y - x > 1) {
+        const long long m = x + (y - x) / 2;
+        if (axis_cell(__dadd_rn(of_order(m), c), n, width) == lo) x = m;
+        else y = m;
+      }
+      const int k = atomicAdd(&s_count, 1);
+      if (k < n + 4) {
+        raw[k] = of_order(y);
+        rank[k] = j;
+      }
+    }
+    __syncthreads();
+    const int count = min(s_count, n + 4);
+    for (int k = tid; k < count; k += kThreads) {
+      int pos = 0;
+      for (int q = 0; q < count; ++q)
+        pos += raw[q] < raw[k] || (raw[q] == raw[k] && rank[q] < rank[k]);
+      thr[pos] = raw[k];
+      cell[pos] = axis_cell(__dadd_rn(-emax, __dmul_rn(step, (double)rank[k])), n, width);
+    }
+    __syncthreads();
+    if (tid == 0) {
+      int ranks = 0;
+      for (int k = 0; k < count; ++k) {
+        if (!k || thr[k] != thr[k - 1]) raw[ranks++] = thr[k];
+        rank[k] = ranks;
+      }
+      const bool fits = s_count <= n + 4 && slots + ranks + 1 <= kAxisSlots;
+      l.h->slot0[f] = fits ? slots : -1;
+      l.h->nrank[f] = ranks + 1;
+      l.h->nflip[f] = count;
+      s_count = fits ? ranks + 1 : 0;
+    }
+    __syncthreads();
+    slots += s_count;
+    __syncthreads();
+  }
+  if (tid == 0) {
+    l.h->emax = emax;
+    l.h->run = run;
+    l.h->nfam = f;
+  }
+}
+
+// One thread per (cell of the fixed axis, layer): the sum below all thresholds
+// from the cells' weights, then threshold by threshold.
+__global__ void __launch_bounds__(kAxisThreads) axis_table_kernel(const AxisJob a) {
+  const AxisLists l = axis_lists(a, blockIdx.y);
+  const int n = a.r.n, groups = (n + kAxisThreads - 1) / kAxisThreads;
+  const int ia = blockIdx.x / groups, k = blockIdx.x % groups * kAxisThreads + threadIdx.x;
+  if (k >= n) return;
+  const size_t step = l.h->run ? n : (size_t)n * n;
+  const float *v = static_cast<const float *>(a.r.vol) +
+                   (size_t)(a.a0 + ia) * (l.h->run ? (size_t)n * n : n) + k;
+  for (int f = 0; f < l.h->nfam; ++f) {
+    if (l.h->slot0[f] < 0) continue;
+    float *t = a.table + (((size_t)blockIdx.y * kAxisSlots + l.h->slot0[f]) * a.na + ia) * n + k;
+    const int *w = l.weight + f * n, *cell = l.cell + f * (n + 4), *rank = l.rank + f * (n + 4);
+    double sum = 0.0;
+#pragma unroll 8
+    for (int m = 0; m < n; ++m) sum += (double)w[m] * (double)__ldg(v + step * m);
+    int q = 0;
+    for (int h = 0;; ++h) {
+      t[(size_t)h * a.na * n] = (float)sum;
+      if (h + 1 == l.h->nrank[f]) break;
+      for (; q < l.h->nflip[f] && rank[q] == h + 1; ++q) {
+        const int c = cell[q];
+        const double up = c + 1 < n ? (double)__ldg(v + step * (c + 1)) : 0.0;
+        sum += up - (c >= 0 ? (double)__ldg(v + step * c) : 0.0);
+      }
+    }
+  }
+}
+
+// One block per plane, threads on its rows.
+__global__ void __launch_bounds__(kAxisThreads) axis_rows_kernel(const AxisJob a) {
+  const ProfReq &r = a.r;
+  const AxisLists l = axis_lists(a, blockIdx.y);
+  const int n = r.n, it = blockIdx.x % r.ntheta, is = blockIdx.x / r.ntheta;
+  const int d = a.phi[blockIdx.y] * r.ntheta + it, run = l.h->run, fix = 1 - run;
+  const double *D = r.dir + 9 * (size_t)d;
+  const double s = __ldg(r.shift + is), delta = 1.0 / n, width = __ddiv_rn(2.0, (double)n);
+  const double emax = l.h->emax, crop = (double)crop_of(r);
+  const double rem = crop - s * s;
+  const int im = rem >= 0.0 ? (int)(sqrt(rem) * n) : -1;
+  const int lo = max(-r.L, -im), hi = rem >= 0.0 ? min(r.L - 1, im) : lo - 1;
+  // what the samples' other two coordinates differ by along the row, at most
+  const double cx = fabs(__dmul_rn(__dmul_rn(delta, __ldg(D + 6 + fix)), (double)r.L));
+  const double cz = fabs(__dmul_rn(__dmul_rn(delta, __ldg(D + 8)), (double)r.L));
+  const double sx = __dmul_rn(s, __ldg(D + fix)), dx = __dmul_rn(delta, __ldg(D + 3 + fix));
+  const double se = __dmul_rn(s, __ldg(D + run)), de = __dmul_rn(delta, __ldg(D + 3 + run));
+  const double sz = __dmul_rn(s, __ldg(D + 2)), dz = __dmul_rn(delta, __ldg(D + 5));
+  const int f = l.fam[it], slot0 = f < kAxisFamilies ? l.h->slot0[f] : -1;
+  const int nstep = slot0 >= 0 ? l.h->nrank[f] - 1 : 0;
+  const double *step = l.step + (slot0 >= 0 ? f * (n + 4) : 0);
+  const float *t = a.table + ((size_t)blockIdx.y * kAxisSlots + max(slot0, 0)) * a.na * n;
+  double sum = 0.0;
+  unsigned long long counted = 0;
+  for (int i0 = lo + (threadIdx.x & ~31); i0 <= hi; i0 += kAxisThreads) {
+    const int i = i0 + (threadIdx.x & 31);
+    const double di = (double)i;
+    const double x = __dadd_rn(sx, __dmul_rn(dx, di)), z = __dadd_rn(sz, __dmul_rn(dz, di));
+    const double e = __dadd_rn(se, __dmul_rn(de, di));
+    const int ix = axis_cell(__dadd_rn(x, -cx), n, width), iz = axis_cell(__dadd_rn(z, -cz), n, width);
+    const int own = min(max(ix, 0), n - 1) - a.a0;
+    const bool mine = i <= hi && own >= 0 && own < a.na;
+    const bool one = slot0 >= 0 && fabs(e) <= emax && ix == axis_cell(__dadd_rn(x, cx), n, width) &&
+                     iz == axis_cell(__dadd_rn(z, cz), n, width);
+    if (mine && one && ix >= 0 && ix < n && iz >= 0 && iz < n) {
+      int p = 0, q = nstep;  // thresholds at or below e
+      while (p < q) {
+        const int m = (p + q) >> 1;
+        if (step[m] <= e) p = m + 1;
+        else q = m;
+      }
+      sum += (double)__ldg(t + ((size_t)p * a.na + own) * n + iz);
+    }
+    unsigned m = __ballot_sync(kAll, mine && !one);
+    while (m) {
+      const int src = __ffs(m) - 1;
+      m &= m - 1;
+      const double v = exact_row(r, d, is, i0 + src, crop, false, false);
+      if ((threadIdx.x & 31) == src) sum += v;
+    }
+    if (r.counter && a.first && i <= hi) {
+      const int jm = (int)(sqrt(fmax(0.0, rem - di * di * delta * delta)) * n);
+      counted += min(r.L - 1, jm) - max(-r.L, -jm) + 1;
+    }
+  }
+  if (counted) atomicAdd(r.counter, counted);
+  __shared__ double s_sum[kAxisThreads / 32];
+  sum = wrtd::warp_sum(sum);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double v = 0.0;
+    for (int w = 0; w < kAxisThreads / 32; ++w) v += s_sum[w];
+    v /= (double)n * n;
+    double *o = r.out + ((size_t)is * r.nphi + a.phi[blockIdx.y]) * r.ntheta + it;
+    if (a.first) *o = v;
+    else if (v != 0.0) *o += v;
+  }
+}
+
 // ------------------------------------------------------------------ host side
 size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -1065,22 +1344,27 @@ bool profile_covers(int n, int nphi, int ntheta, int nshift) {
 // the staged kernel on 110 random sizes past the line (n 10 .. 176, 3 .. 64 latitudes,
 // 8 .. 256 shifts, 4000 planes up): 0.93 of its speed at worst, 1.05-2.5 times within a
 // fifth of the line, 2-4 times at twice; just below it 0.5-1.3 times for n > 100, up
-// to 2.5 for n < 60.  The nearest sampler's (whose phis on an axis stay with the staged
-// kernel) are even at 30-40.  Below 4000 planes both are launches: 0.7-1.6 times.
-bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift, bool nearest) {
+// to 2.5 for n < 60.  Nearest on 86 sizes past the line: 1.03 at worst, 1.3-9 as a
+// rule.  Below 4000 planes both are launches: 0.7-1.6 times.
+bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift) {
   if (!profile_covers(n, nphi, ntheta, nshift)) return false;
   if (ctx->staged_config >= 0) return ctx->staged_config == kNumStagedConfigs - 1;
   const double rows = (double)ntheta * nshift;
   if (rows * nphi < 4000) return false;
-  if (nearest) return rows >= 40.0 * n;
   const bool paired = nphi % 2 == 0;
   return rows * (paired ? 1.0 : 0.5) >= n * (7.0 + 0.4 * n / (paired ? nphi / 2 : nphi));
+}
+
+// The least workspace for nphis phis on an axis, and what holds their whole table.
+static size_t axis_workspace(const ProfReq &r, int nphis, int cells) {
+  return nphis * (axis_head_bytes(r.n, r.ntheta) + (size_t)kAxisSlots * cells * r.n * 4) + 256;
 }
 
 // The least workspace a request can be computed in: that of one unit.
 size_t profile_workspace_least(const ProfReq &r, float crop) {
   size_t ws = 1 << 20;
   while (!Areas(ws).fits(unit_bytes(r, crop), chunk_group(r.n), UnitBytes())) ws += ws / 16;
+  if (r.nearest) ws = al(ws) + std::max(al(axis_workspace(r, 4, 1)), al(ws / 7));
   return ws;
 }
 
@@ -1098,7 +1382,33 @@ size_t profile_workspace_want(const ProfReq *reqs, const float *crop, int nreq) 
     table += u * std::min(c1 - c0, chunk_group(r.n)) * (nreq == 1 ? (nbase + kProfLanes - 1) / kProfLanes * kProfLanes : nbase);
     least = std::max(least, profile_workspace_least(r, crop[q]));
   }
-  return std::max(least, std::min(table, kProfTableBytes) / 176 * 256 + (4 << 20));
+  const size_t ws = std::min(table, kProfTableBytes) / 176 * 256 + (4 << 20);
+  // (the nearest sampler's phis on an axis come first, in up to an eighth)
+  return std::max(least, reqs[0].nearest ? ws + ws / 7 : ws);
+}
+
+static int axis_forward(wrt_ctx *ctx, cudaStream_t stream, const ProfReq &r, const int *phis, int nphis,
+                        void *ws, size_t ws_bytes) {
+  int cells = r.n;
+  while (cells > 1 && axis_workspace(r, nphis, cells) > ws_bytes) --cells;
+  AxisJob a = {};
+  a.r = r;
+  for (int p = 0; p < nphis; ++p) a.phi[p] = phis[p];
+  a.head = static_cast<char *>(ws);
+  a.head_bytes = axis_head_bytes(r.n, r.ntheta);
+  a.table = reinterpret_cast<float *>(a.head + a.head_bytes * nphis);
+  axis_prepare_kernel<<<nphis, kThreads, 0, stream>>>(a);
+  ctx->launches++;
+  const int groups = (r.n + kAxisThreads - 1) / kAxisThreads;
+  for (a.a0 = 0; a.a0 < r.n; a.a0 += a.na) {
+    a.na = std::min(cells, r.n - a.a0);
+    a.first = a.a0 == 0;
+    axis_table_kernel<<<dim3(a.na * groups, nphis), kAxisThreads, 0, stream>>>(a);
+    axis_rows_kernel<<<dim3(r.ntheta * r.nshift, nphis), kAxisThreads, 0, stream>>>(a);
+    ctx->launches += 2;
+  }
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? WRT_OK : cuda_fail(ctx, e, "row sums on an axis");
 }
 
 int profile_lanes_init(wrt_ctx *ctx, ProfLanes *l) {
@@ -1123,7 +1433,7 @@ void profile_lanes_release(ProfLanes *l) {
 }
 
 int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const ProfReq *reqs,
-                    const float *crop, int nreq, void *ws, size_t ws_bytes, bool forked) {
+                    const float *crop, int nreq, void *ws, size_t ws_bytes, ProfFork fork) {
   if (nreq < 1) return WRT_OK;
   const bool near = reqs[0].nearest != 0;
   // ---- lanes: the launches of a step depend on one another and each ends with
@@ -1132,13 +1442,14 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
   size_t table = 0;
   for (int q = 0; q < nreq; ++q)
     table += unit_bytes(reqs[q], crop[q]).table * (reqs[q].paired ? reqs[q].nphi / 2 : reqs[q].nphi);
+  const bool forked = fork == PROF_BESIDE;
   const int most = forked ? kProfLanes - 1 : kProfLanes;
   int nl = table >= kProfLaneBytes ? most : 1;
   for (int q = 0; q < nreq; ++q)  // every request has to fit a lane
     while (nl > 1 && !Areas(ws_bytes / nl & ~(size_t)255)
                           .fits(unit_bytes(reqs[q], crop[q]), chunk_group(reqs[q].n), UnitBytes()))
       --nl;
-  if (nl > 1 && !forked) {
+  if (nl > 1 && fork == PROF_ALONE) {
     int st = profile_lanes_init(ctx, lanes);
     if (st) return st;
   }
@@ -1177,7 +1488,7 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
     }
   }
   cudaError_t e = cudaSuccess;
-  if (nl > 1 && !forked) e = cudaEventRecord(lanes->fork, stream);
+  if (nl > 1 && fork == PROF_ALONE) e = cudaEventRecord(lanes->fork, stream);
   for (int l = forked ? 0 : 1; l < nl && e == cudaSuccess; ++l)
     e = cudaStreamWaitEvent(lane_of(l), lanes->fork, 0);
   // nothing may still use the workspace when a failed call returns
@@ -1272,6 +1583,31 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
     if (home[q] < 0) e = extra(q, home_stream);
   if (forked && e == cudaSuccess) e = cudaEventRecord(lanes->done[0], home_stream);
   return e == cudaSuccess ? WRT_OK : failed("row-sum profiles");
+}
+
+// The phis on an axis beside the others: their first kernel is a few blocks only.  A
+// small request's others are on one side stream, a large one's on all lanes.
+int profile_forward_nearest(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const ProfReq &r,
+                            float crop, const int *phis, int nphis, void *ws, size_t ws_bytes) {
+  if (!nphis) return profile_forward(ctx, stream, lanes, &r, &crop, 1, ws, ws_bytes);
+  int st = profile_lanes_init(ctx, lanes);
+  if (st) return st;
+  cudaError_t e = cudaEventRecord(lanes->fork, stream);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "profile fork");
+  const size_t part = al(std::min(axis_workspace(r, nphis, r.n),
+                                  std::max(axis_workspace(r, nphis, 1), ws_bytes / 8)));
+  char *rest = static_cast<char *>(ws) + part;
+  const bool small = unit_bytes(r, crop).table * (r.paired ? r.nphi / 2 : r.nphi) < kProfLaneBytes;
+  if (small) {
+    st = profile_forward(ctx, stream, lanes, &r, &crop, 1, rest, ws_bytes - part, PROF_BESIDE);
+    if (st) return st;
+  }
+  st = axis_forward(ctx, stream, r, phis, nphis, ws, part);
+  if (!small)
+    return st ? st : profile_forward(ctx, stream, lanes, &r, &crop, 1, rest, ws_bytes - part,
+                                     PROF_FORKED);
+  e = cudaStreamWaitEvent(stream, lanes->done[0], 0);
+  return st || e == cudaSuccess ? st : cuda_fail(ctx, e, "profile join");
 }
 
 }  // namespace wrt

@@ -726,18 +726,6 @@ __global__ void plane_finalize_kernel(double *out, long long count, double facto
   }
 }
 
-__global__ void plane_finalize_phis_kernel(double *out, int4 phis, int nphis, int nphi, int ntheta,
-                                           int nshift, double factor) {
-  const int per = nphis * ntheta;
-  for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < (long long)nshift * per;
-       k += (long long)gridDim.x * blockDim.x) {
-    const int r = (int)(k % per), p = r / ntheta;
-    const int ip = p == 0 ? phis.x : p == 1 ? phis.y : p == 2 ? phis.z : phis.w;
-    const long long o = (k / per * nphi + ip) * ntheta + r % ntheta;
-    out[o] = (double)reinterpret_cast<const long long *>(out)[o] * factor;
-  }
-}
-
 }  // namespace
 
 namespace wrt {
@@ -828,16 +816,6 @@ int plane_finalize(wrt_ctx *ctx, double *out, long long count, double factor) {
   return check_launch(ctx, "plane_finalize_kernel");
 }
 
-int plane_finalize_phis(wrt_ctx *ctx, double *out, const int *phis, int nphis, int nphi,
-                        int ntheta, int nshift, double factor) {
-  const int4 p = make_int4(phis[0], phis[nphis > 1 ? 1 : 0], phis[nphis > 2 ? 2 : 0],
-                           phis[nphis > 3 ? 3 : 0]);
-  plane_finalize_phis_kernel<<<ctx->sm_count * 2, 256, 0, ctx->stream>>>(out, p, nphis, nphi,
-                                                                         ntheta, nshift, factor);
-  ctx->launches++;
-  return check_launch(ctx, "plane_finalize_phis_kernel");
-}
-
 // Work items of one request, largest estimated cost first.  Cost of a
 // (layer, tile): voxels of the tile's slab inside the crop radius.
 void staged_items_costed(int req, int n, int tile_h, float crop_r2, int ndir, int dir_chunk,
@@ -886,22 +864,19 @@ struct ItemList {
   size_t bytes = 0;
 };
 struct StagedCache {
-  // n, tile rows, crop, directions, sampler, number of phis on an axis (0: all
-  // phis) and ntheta (with the directions they fix which phis those are)
-  std::map<std::tuple<int, int, unsigned, int, bool, int, int>, ItemList> lists;
+  std::map<std::tuple<int, int, unsigned, int, bool>, ItemList> lists;
 };
 }  // namespace
 
 // Device copy of the item list of one geometry: a 16-byte header holding the
 // item count (the kernel reads it from there), then the items.
 int staged_items_cached(wrt_ctx *ctx, int n, int tile_h, float crop_r2, int ndir,
-                        StagedItem **d_items, const int **d_nitems, int *nitems, bool nearest,
-                        const int *phis, int nphis, int ntheta) {
+                        StagedItem **d_items, const int **d_nitems, int *nitems, bool nearest) {
   if (!ctx->staged_cache) ctx->staged_cache = new StagedCache();
   StagedCache *c = static_cast<StagedCache *>(ctx->staged_cache);
   unsigned bits;
   memcpy(&bits, &crop_r2, sizeof(bits));
-  const auto key = std::make_tuple(n, tile_h, bits, ndir, nearest, nphis, ntheta);
+  const auto key = std::make_tuple(n, tile_h, bits, ndir, nearest);
   auto it = c->lists.find(key);
   if (it == c->lists.end()) {
     if (c->lists.size() > 64) {  // bounded: drop everything, rebuild on demand
@@ -910,21 +885,7 @@ int staged_items_cached(wrt_ctx *ctx, int n, int tile_h, float crop_r2, int ndir
       c->lists.clear();
     }
     std::vector<StagedItem> items;
-    if (nphis) {
-      // a few phis only: chunks of 64 directions, so that they fill the SMs
-      std::vector<std::pair<double, StagedItem>> v;
-      for (int p = 0; p < nphis; ++p) {
-        const size_t v0 = v.size();
-        staged_items_costed(0, n, tile_h, crop_r2, ntheta, 64, 1.0, v, nearest);
-        for (size_t k = v0; k < v.size(); ++k) v[k].second.dir0 += phis[p] * ntheta;
-      }
-      std::stable_sort(v.begin(), v.end(),
-                       [](const std::pair<double, StagedItem> &a,
-                          const std::pair<double, StagedItem> &b) { return a.first > b.first; });
-      for (auto &c : v) items.push_back(c.second);
-    } else {
-      staged_items(0, n, tile_h, crop_r2, ndir, kStagedDirChunk, items, nearest);
-    }
+    staged_items(0, n, tile_h, crop_r2, ndir, kStagedDirChunk, items, nearest);
     ItemList l;
     l.count = (int)items.size();
     l.bytes = 16 + sizeof(StagedItem) * items.size();

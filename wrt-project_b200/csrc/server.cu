@@ -430,7 +430,7 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
     p.nshift = r.nshift;
     p.storage = WRT_STORAGE_F32;
     p.paired = wrt::profile_paired(n, r.nphi, L);
-    if (wrt::profile_route(s->ctx, n, r.nphi, r.ntheta, r.nshift, false) &&
+    if (wrt::profile_route(s->ctx, n, r.nphi, r.ntheta, r.nshift) &&
         slot.prof_bytes >= wrt::profile_workspace_least(p, 3.0f + 1e-5f)) {
       a.pairs = nullptr;
       a.nout = 0;

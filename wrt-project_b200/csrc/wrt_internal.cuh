@@ -218,9 +218,6 @@ int plane_staged_launch_nearest(wrt_ctx *ctx, cudaStream_t stream, const StagedR
                                 const StagedItem *d_items, const int *d_nitems, int max_smem,
                                 int *d_next);
 int plane_finalize(wrt_ctx *ctx, double *out, long long count, double factor);
-// The same for the planes of up to four phis of [nshift][nphi][ntheta].
-int plane_finalize_phis(wrt_ctx *ctx, double *out, const int *phis, int nphis, int nphi,
-                        int ntheta, int nshift, double factor);
 // Work items of one request (layer x y-tile x direction chunk) with their
 // estimated cost (staged voxels inside the crop radius x directions x weight).
 void staged_items_costed(int req, int n, int tile_h, float crop_r2, int ndir, int dir_chunk,
@@ -228,12 +225,9 @@ void staged_items_costed(int req, int n, int tile_h, float crop_r2, int ndir, in
                          bool nearest = false);
 void staged_items(int req, int n, int tile_h, float crop_r2, int ndir, int dir_chunk,
                   std::vector<StagedItem> &out, bool nearest = false);
-// phis / nphis: only the directions of these phis (ntheta = ndir / nphi each),
-// all of them when nphis is 0.
 int staged_items_cached(wrt_ctx *ctx, int n, int tile_h, float crop_r2, int ndir,
                         StagedItem **d_items, const int **d_nitems, int *nitems,
-                        bool nearest = false, const int *phis = nullptr, int nphis = 0,
-                        int ntheta = 0);
+                        bool nearest = false);
 int staged_scratch(wrt_ctx *ctx, size_t req_bytes);
 void staged_release(wrt_ctx *ctx);
 
@@ -278,17 +272,24 @@ inline bool profile_paired(int n, int nphi, int L) { return nphi % 2 == 0 && L >
 bool profile_covers(int n, int nphi, int ntheta, int nshift);
 size_t profile_workspace_least(const ProfReq &r, float crop);
 size_t profile_workspace_want(const ProfReq *reqs, const float *crop, int nreq);
-bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift, bool nearest);
+bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift);
 // The plane integrals of nreq requests (one sampler) on a stream.  crop[q]: a bound on the
 // squared crop radius (3 where the host does not know the volume's support yet;
 // it limits which empty ranges of t are visited and the room for pieces).  ws: at least profile_workspace_least for every
 // request.
 // lanes: streams for side-by-side steps, created on first use; the work is
-// forked from `stream` and joined to it again.  forked: on side streams only, which
-// wait for lanes->fork (recorded by the caller); the caller's stream has to wait
-// for lanes->done[0] afterwards.
+// forked from `stream` and joined to it again.
+enum ProfFork {
+  PROF_ALONE,
+  PROF_FORKED,  // lanes->fork was recorded by the caller
+  PROF_BESIDE,  // .. and only side streams are used: the caller's has to wait for lanes->done[0]
+};
 int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const ProfReq *reqs,
-                    const float *crop, int nreq, void *ws, size_t ws_bytes, bool forked = false);
+                    const float *crop, int nreq, void *ws, size_t ws_bytes,
+                    ProfFork fork = PROF_ALONE);
+// The nearest sampler's plane integrals; phis: those on an axis, up to four.
+int profile_forward_nearest(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const ProfReq &r,
+                            float crop, const int *phis, int nphis, void *ws, size_t ws_bytes);
 int profile_lanes_init(wrt_ctx *ctx, ProfLanes *l);
 void profile_lanes_release(ProfLanes *l);
 
