@@ -126,3 +126,23 @@ def test_backprojection_matches_oracle(ctx, n, nphi, ntheta, nshift):
     pick = np.random.default_rng(1).integers(0, n, (400, 3))
     ref = O.adjoint_points(radon, x[pick[:, 1]], x[pick[:, 2]], x[pick[:, 0]])
     assert rel_l2(got[pick[:, 0], pick[:, 1], pick[:, 2]], ref) < TOL_L2
+
+
+def test_tables_make_room():
+    # the tables' buffer may fill the budget; what is allocated next still fits
+    with wrt.Context(0, budget_bytes=96 << 20) as c:
+        v = wrt.Volume(c, 64)
+        v.upload(_volume("noise", 64))
+        g = wrt.Grid(c, 32, 16, 64)
+        out = wrt.DeviceBuffer(c, g.nplanes * 8)
+        wrt.radon_forward_device(c, v, g, out.ptr, half_extent=64)
+        c.synchronize()
+        first = out.download(np.empty(g.nplanes))
+        big = wrt.DeviceBuffer(c, 80 << 20)
+        wrt.radon_forward_device(c, v, g, out.ptr, half_extent=64)
+        c.synchronize()
+        again = out.download(np.empty(g.nplanes))
+        del big
+    assert rel_l2(first, again) < TOL_L2
+    ref = O.radon_forward(_volume("noise", 64), 32, 16, 64, sampler=O.TRILINEAR, half_extent=64)
+    assert rel_l2(first, ref.ravel()) < TOL_L2

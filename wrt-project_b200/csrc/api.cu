@@ -68,13 +68,30 @@ int cuda_fail(wrt_ctx *ctx, cudaError_t e, const char *what) {
   return fail(ctx, WRT_ERR_CUDA, "%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));
 }
 
+// The tables' working buffer is only there for speed: it makes room for anything else
+// (unless the running call works in it).
+static bool release_tables(wrt_ctx *ctx) {
+  if (ctx->tables_held || !ctx->ws[WS_PROFILE]) return false;
+  cudaStreamSynchronize(ctx->stream);
+  ctx->tables_refused = ctx->ws_bytes[WS_PROFILE];
+  ctx_free(ctx, ctx->ws[WS_PROFILE], ctx->ws_bytes[WS_PROFILE]);
+  ctx->ws[WS_PROFILE] = nullptr;
+  ctx->ws_bytes[WS_PROFILE] = 0;
+  return true;
+}
+
 int ctx_alloc(wrt_ctx *ctx, void **p, size_t bytes) {
   *p = nullptr;
   if (bytes == 0) return WRT_OK;
+  if (ctx->budget && ctx->in_use + bytes > ctx->budget) release_tables(ctx);
   if (ctx->budget && ctx->in_use + bytes > ctx->budget)
     return fail(ctx, WRT_ERR_BUDGET, "device budget: %zu bytes in use + %zu requested > %zu",
                 ctx->in_use, bytes, ctx->budget);
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    if (release_tables(ctx)) e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
@@ -723,17 +740,29 @@ ProfReq profile_request(const wrt_ctx *ctx, const wrt_volume *vol, const wrt_gri
   return r;
 }
 
+// While a call works in the tables' buffer it stays.
+struct TablesHeld {
+  wrt_ctx *ctx;
+  explicit TablesHeld(wrt_ctx *c) : ctx(c) { ctx->tables_held = true; }
+  ~TablesHeld() { ctx->tables_held = false; }
+};
+
 // The profiles' working memory of these requests in the context's workspace:
-// what they ask for, or the least that serves them; an error (cleared) when
-// the context's budget or the device holds neither.
+// what they ask for, or as much of it as the context's budget and the device hold,
+// halving down to the least that serves them; an error (cleared) below that.
 int profile_ws(wrt_ctx *ctx, const ProfReq *reqs, const float *crop, int nreq, void **ws,
                size_t *bytes) {
-  const size_t want = profile_workspace_want(reqs, crop, nreq);
-  size_t least = 0;
+  size_t want = profile_workspace_want(reqs, crop, nreq), least = 0;
   for (int q = 0; q < nreq; ++q)
     least = std::max(least, profile_workspace_least(reqs[q], crop[q]));
+  auto half = [&] { return std::max(want / 2 & ~(size_t)255, least); };
+  while (want > least && want >= ctx->tables_refused) want = half();
   int st = ws_get(ctx, WS_PROFILE, want, ws);
-  if (st) st = ws_get(ctx, WS_PROFILE, least, ws);
+  while (st && want > least) {
+    ctx->tables_refused = want;
+    want = half();
+    st = ws_get(ctx, WS_PROFILE, want, ws);
+  }
   if (st) {
     ctx->err[0] = 0;
     return st;
@@ -750,6 +779,7 @@ int radon_forward_profile(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, i
   size_t bytes = 0;
   *done = false;
   if (profile_ws(ctx, &r, &crop, 1, &ws, &bytes)) return WRT_OK;  // no room: the staged kernel
+  const TablesHeld held(ctx);
   *done = true;
   if (nearest) {
     int phis[4], m = 0;
@@ -836,15 +866,7 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
     prof.push_back(profile_request(ctx, vol, grid, L, false, reqs[r].dev_out));
     prof_crop.push_back(trilinear_crop_r2(vol->r2, vol->n));
   }
-  void *prof_ws = nullptr;
-  size_t prof_bytes = 0;
-  if (!prof.empty() && profile_ws(ctx, prof.data(), prof_crop.data(), (int)prof.size(), &prof_ws,
-                                  &prof_bytes)) {
-    prof.clear();
-    std::fill(routed.begin(), routed.end(), 0);
-  }
-  for (int r = 0; r < nreq; ++r) {
-    if (routed[r]) continue;
+  auto add_staged = [&](int r) -> int {
     wrt_volume *vol = const_cast<wrt_volume *>(reqs[r].volume);
     const wrt_grid *grid = reqs[r].grid;
     if (!vol || !grid || !reqs[r].dev_out || vol->ctx != ctx || grid->ctx != ctx)
@@ -855,8 +877,8 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
       return fail(ctx, WRT_ERR_INVALID_ARGUMENT, "batch request %d: volume edge %d unsupported", r, n);
     if (reqs[r].half_extent < 0 || reqs[r].half_extent > 8 * n)
       return fail(ctx, WRT_ERR_INVALID_ARGUMENT, "batch request %d: bad half extent", r);
-    st = volume_ensure_pairs(vol);
-    if (st) return st;
+    const int es = volume_ensure_pairs(vol);
+    if (es) return es;
     const int L = reqs[r].half_extent ? reqs[r].half_extent : 2 * n;
     StagedReq q;
     const bool bf16 = vol->storage == WRT_STORAGE_BF16;
@@ -874,7 +896,22 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
     a.L = L;
     a.prep = 0;
     batch_add_forward(b, q, a, trilinear_crop_r2(vol->r2, n));
+    return WRT_OK;
+  };
+  for (int r = 0; r < nreq && !st; ++r)
+    if (!routed[r]) st = add_staged(r);
+  if (st) return st;
+  // the tables after all that has to be there
+  void *prof_ws = nullptr;
+  size_t prof_bytes = 0;
+  if (!prof.empty() && profile_ws(ctx, prof.data(), prof_crop.data(), (int)prof.size(), &prof_ws,
+                                  &prof_bytes)) {
+    prof.clear();
+    for (int r = 0; r < nreq && !st; ++r)
+      if (routed[r]) st = add_staged(r);
+    if (st) return st;
   }
+  const TablesHeld held(ctx);
   auto profiles = [&](ProfFork fork) {
     return prof.empty() ? WRT_OK
                         : profile_forward(ctx, ctx->stream, &ctx->prof_lanes, prof.data(),
@@ -882,16 +919,6 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
                                           fork);
   };
   if (b.fwd.empty()) return profiles(PROF_ALONE);
-  if (!prof.empty()) {
-    // beside the staged kernel, and before it: its blocks hold their SM until
-    // the item list is empty, so they take what the profiles leave free
-    st = profile_lanes_init(ctx, &ctx->prof_lanes);
-    if (st) return st;
-    cudaError_t e = cudaEventRecord(ctx->prof_lanes.fork, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "profile fork");
-    st = profiles(PROF_BESIDE);
-    if (st) return st;
-  }
   if (!ctx->batch_slot) {
     BatchSlot *s = new (std::nothrow) BatchSlot();
     if (!s) return WRT_ERR_OUT_OF_MEMORY;
@@ -902,6 +929,16 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
       return st;
     }
     ctx->batch_slot = s;
+  }
+  if (!prof.empty()) {
+    // beside the staged kernel, and before it: its blocks hold their SM until
+    // the item list is empty, so they take what the profiles leave free
+    st = profile_lanes_init(ctx, &ctx->prof_lanes);
+    if (st) return st;
+    cudaError_t e = cudaEventRecord(ctx->prof_lanes.fork, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "profile fork");
+    st = profiles(PROF_BESIDE);
+    if (st) return st;
   }
   st = batch_slot_launch(static_cast<BatchSlot *>(ctx->batch_slot), b);
   if (!prof.empty()) {
@@ -1163,10 +1200,13 @@ int wrt_radon3d_adjoint_device(wrt_ctx *ctx, const double *dev_radon, const wrt_
   if (backproj_covers(grid->nphi, grid->ntheta, grid->nshift, ngrid)) {
     const size_t want = backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, false);
     void *ws = nullptr, *cp = nullptr;
-    st = ws_get(ctx, WS_PROFILE, want, &ws);
-    if (st)
+    st = want < ctx->tables_refused ? ws_get(ctx, WS_PROFILE, want, &ws) : WRT_ERR_BUDGET;
+    if (st) {
+      ctx->tables_refused = std::min(ctx->tables_refused, want);
       st = ws_get(ctx, WS_PROFILE,
                   backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, true), &ws);
+    }
+    const TablesHeld held(ctx);
     if (!st) st = ws_get(ctx, WS_COEF, sizeof(double) * 2 * grid->nshift, &cp);
     if (!st) {
       std::vector<double> coef(2 * (size_t)grid->nshift);

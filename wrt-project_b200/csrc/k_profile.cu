@@ -41,7 +41,7 @@
 // launch waits for its gathers (random 32-byte reads, mostly from L2) and FP64
 // geometry, the build for its node loads.  128^3, 64 x 128 directions x 256
 // shifts, lattice [-n, n)^2: 53.7 ms by the staged kernel (lattice samples
-// through shared memory), 5.2 ms here; 256^3 BF16, 96 x 192 x 384: 750 and 64
+// through shared memory), 4.6 ms here; 256^3 BF16, 96 x 192 x 384: 750 and 44
 // ms; error against FP64 6.5e-8 (staged 8.9e-8).  Small requests wait for the four
 // launches one after another (24^3, 8 x 16 x 32: 109 and 80 us).
 #include <math.h>
@@ -60,6 +60,7 @@ using wrt::ProfSeg;
 
 constexpr unsigned kAll = 0xffffffffu;
 constexpr int kThreads = 256;
+constexpr int kSortThreads = 1024;
 constexpr int kMaxChunks = 6;  // ranges of t of one phi in a step
 constexpr double kMagicPos = 6442450944.0;            // 1.5 * 2^32: 20 fraction bits
 constexpr double kMagicInt = 6755399441055744.0;      // 1.5 * 2^52
@@ -81,7 +82,8 @@ __device__ __forceinline__ Geo geo_of_unit(const ProfSeg &s, int unit) {
 }
 
 // ------------------------------------------------------------------ sort role
-// One block finds the unit's piece boundaries, counts them per bin, and writes
+// One block (of 1024 threads: few blocks, on which the whole step waits) finds the
+// unit's piece boundaries, counts them per bin, and writes
 // them in order of (position, identity): a bin's few entries are ranked by
 // counting, so the order does not depend on the atomics.
 __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
@@ -91,17 +93,17 @@ __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
   unsigned *start = s.start + (size_t)unit * (kUnitBins + 8);
   int *cnt = reinterpret_cast<int *>(smem);           // [kUnitBins]
   int *cur = cnt + kUnitBins;                         // [kUnitBins]
-  __shared__ int s_warp[kThreads / 32];
+  __shared__ int s_warp[kSortThreads / 32];
   const int tid = threadIdx.x;
   const bool skip = s.r.nearest && on_axis(g);
-  for (int b = tid; b < kUnitBins; b += kThreads) cnt[b] = 0;
+  for (int b = tid; b < kUnitBins; b += kSortThreads) cnt[b] = 0;
   __syncthreads();
   if (!skip)
-    each_boundary(g, s.nsub, s.sub_bins, (int)threadIdx.x, kThreads,
+    each_boundary(g, s.nsub, s.sub_bins, (int)threadIdx.x, kSortThreads,
                   [&](unsigned p, int, int, int) { atomicAdd(&cnt[p >> 20], 1); });
   __syncthreads();
-  // exclusive scan of the bins: kUnitBins / kThreads per thread
-  constexpr int kPer = kUnitBins / kThreads;
+  // exclusive scan of the bins: kUnitBins / kSortThreads per thread
+  constexpr int kPer = kUnitBins / kSortThreads;
   int sum = 0;
 #pragma unroll
   for (int q = 0; q < kPer; ++q) sum += cnt[tid * kPer + q];
@@ -123,13 +125,13 @@ __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
     before += c;
   }
   int total = 0;
-  for (int w = 0; w < kThreads / 32; ++w) total += s_warp[w];
+  for (int w = 0; w < kSortThreads / 32; ++w) total += s_warp[w];
   __syncthreads();
   total = min(total, s.cap);  // the capacity bounds every geometry; never exceeded
   if (tid == 0) start[kUnitBins] = total;
   unsigned long long *keys = s.keys + (size_t)unit * s.cap;
   if (!skip)
-    each_boundary(g, s.nsub, s.sub_bins, (int)threadIdx.x, kThreads, [&](unsigned p, int kind, int li, int m) {
+    each_boundary(g, s.nsub, s.sub_bins, (int)threadIdx.x, kSortThreads, [&](unsigned p, int kind, int li, int m) {
       const int slot = atomicAdd(&cur[p >> 20], 1);
       // the sub-range's start precedes everything at its position
       const unsigned id = kind == K_NULL ? 0u
@@ -139,7 +141,7 @@ __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
     });
   __syncthreads();
   PieceRec *rec = static_cast<PieceRec *>(s.rec) + (size_t)unit * s.cap;
-  for (int e = tid; e < total; e += kThreads) {
+  for (int e = tid; e < total; e += kSortThreads) {
     const unsigned long long key = keys[e];
     const unsigned p = (unsigned)(key >> 32), id = (unsigned)key;
     const int b = p >> 20;
@@ -797,17 +799,15 @@ __device__ __noinline__ int row_samples(const ProfReq &r, int is, int i, double 
   return min(r.L - 1, jm) - max(-r.L, -jm) + 1;
 }
 
-// One warp per 32 planes (one theta, consecutive shifts).  A plane has
-// 32 / |cos theta| rows in a unit of 16 cells: up to kLongRows of them, each
-// lane walks the rows of its own plane (the lanes' counts are nearly equal, no
-// sums across lanes), else (theta near pi/2, where only some planes meet the
-// unit, with all their rows, and consecutive rows read neighbouring layers of
-// one piece) the warp takes the planes one after another with its lanes on the
-// rows.  Either way four rows per lane are in flight.  The unit's piece
+// One warp per 32 planes (one theta, consecutive shifts).  As a rule each lane walks
+// the rows of its own plane (a plane has 4096 / (n |cos theta|) rows in a unit; the
+// lanes' counts are nearly equal, no sums across lanes); where that takes more rounds
+// (theta near pi/2, where only some planes meet the unit, with all their rows, and
+// consecutive rows read neighbouring layers of one piece) the warp takes the planes
+// one after another with its lanes on the rows (128^3: 5.7 -> 5.5 ms against a fixed
+// 96 rows).  Either way four rows per lane are in flight.  The unit's piece
 // positions are in shared memory.  Rows that need more than the table are
 // marked for profile_slow_kernel.
-constexpr int kLongRows = 96;
-
 template <bool NEAR>
 __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long *list,
                           char *smem) {
@@ -859,7 +859,9 @@ __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long
     if (!most) continue;
     some |= len > 0;
     bool flag = false;
-    if (most <= kLongRows) {
+    // rounds of four rows per lane, one way and the other
+    const int wide = (int)__reduce_add_sync(kAll, (unsigned)((len + 127) >> 7));
+    if ((most + 3) >> 2 <= wide) {
       double di = (double)lo;
       for (int x = 0; x < most; x += 4, di += 4.0)
         flag |= rows4<NEAR>(table, pos, start, n, W, di, 1.0, u0, w.u1, w0, w.w1, len - x, &mine);
@@ -935,7 +937,7 @@ __global__ void __launch_bounds__(kThreads) profile_extra_kernel(const ProfReq r
 }
 
 template <int S>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kSortThreads)
     profile_sort_kernel(const __grid_constant__ wrt::ProfStep<S> st) {
   extern __shared__ __align__(16) char smem[];
   if (blockIdx.x == 0 && threadIdx.x == 0) st.list[0] = 0;
@@ -1274,12 +1276,17 @@ struct Areas {
 constexpr int kManySegs = 24;
 static_assert(kManySegs <= 32, "marks");
 
-// Ranges of t that are computed together: a small volume's all in one step (64^3
-// with 14 x 28 directions 600 -> 240 us), where a large one's fill the device one by
-// one (128^3 in groups of two 5.7 -> 6.4 ms).  By the size alone, because the order in
-// which a plane's sum is added up follows it.
-int chunk_group(int n) {
-  return n <= 64 ? 4 : 1;
+// Ranges of t that are computed together: as many as fit half the tables' memory with
+// all phis, so that few phis fill the device too (64^3 with 14 x 28 directions 600 ->
+// 240 us; 68^3 with 11 x 22 385 -> 230, 78^3 with 23 x 46 850 -> 490), and a phi's
+// together in 128 MB.  By the sizes alone, because the order in which a plane's sum
+// is added up follows it.
+int chunk_group(const ProfReq &r) {
+  const double unit = (double)unit_cap(r.n, 3.0) * r.n * (r.nearest ? 4 : 16);
+  const int nbase = r.paired ? r.nphi / 2 : r.nphi;
+  const double fit = std::min((double)(wrt::kProfTableBytes / 2) / (unit * nbase) + 0.5,
+                              (double)((size_t)128 << 20) / unit);
+  return std::min(std::max((int)fit, 1), 4);
 }
 
 // The ranges of t in which data within the crop bound has rows.
@@ -1319,7 +1326,7 @@ cudaError_t launch_step(wrt_ctx *ctx, cudaStream_t stream, const std::vector<Pro
     e = cudaFuncSetAttribute(profile_rows_kernel<NEAR, S>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_rows);
   if (e != cudaSuccess) return e;
-  profile_sort_kernel<S><<<(unsigned)sort, kThreads, kUnitBins * 8, stream>>>(st);
+  profile_sort_kernel<S><<<(unsigned)sort, kSortThreads, kUnitBins * 8, stream>>>(st);
   profile_build_kernel<NEAR, S><<<(unsigned)build, th_build, sm_build, stream>>>(st);
   profile_rows_kernel<NEAR, S><<<(unsigned)rows, kThreads, sm_rows, stream>>>(st);
   profile_slow_kernel<S><<<ctx->sm_count * 2, kSlowThreads, 0, stream>>>(st);
@@ -1363,7 +1370,7 @@ static size_t axis_workspace(const ProfReq &r, int nphis, int cells) {
 // The least workspace a request can be computed in: that of one unit.
 size_t profile_workspace_least(const ProfReq &r, float crop) {
   size_t ws = 1 << 20;
-  while (!Areas(ws).fits(unit_bytes(r, crop), chunk_group(r.n), UnitBytes())) ws += ws / 16;
+  while (!Areas(ws).fits(unit_bytes(r, crop), chunk_group(r), UnitBytes())) ws += ws / 16;
   if (r.nearest) ws = al(ws) + std::max(al(axis_workspace(r, 4, 1)), al(ws / 7));
   return ws;
 }
@@ -1379,7 +1386,7 @@ size_t profile_workspace_want(const ProfReq *reqs, const float *crop, int nreq) 
     chunk_range(r, crop[q], &c0, &c1);
     const size_t u = unit_bytes(r, crop[q]).table;
     // a lane's share of a single request is whole phis
-    table += u * std::min(c1 - c0, chunk_group(r.n)) * (nreq == 1 ? (nbase + kProfLanes - 1) / kProfLanes * kProfLanes : nbase);
+    table += u * std::min(c1 - c0, chunk_group(r)) * (nreq == 1 ? (nbase + kProfLanes - 1) / kProfLanes * kProfLanes : nbase);
     least = std::max(least, profile_workspace_least(r, crop[q]));
   }
   const size_t ws = std::min(table, kProfTableBytes) / 176 * 256 + (4 << 20);
@@ -1447,7 +1454,7 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
   int nl = table >= kProfLaneBytes ? most : 1;
   for (int q = 0; q < nreq; ++q)  // every request has to fit a lane
     while (nl > 1 && !Areas(ws_bytes / nl & ~(size_t)255)
-                          .fits(unit_bytes(reqs[q], crop[q]), chunk_group(reqs[q].n), UnitBytes()))
+                          .fits(unit_bytes(reqs[q], crop[q]), chunk_group(reqs[q]), UnitBytes()))
       --nl;
   if (nl > 1 && fork == PROF_ALONE) {
     int st = profile_lanes_init(ctx, lanes);
@@ -1471,7 +1478,7 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
     const UnitBytes b = unit_bytes(r, crop[q]);
     const int nbase = r.paired ? r.nphi / 2 : r.nphi;
     int fit = 1;
-    const int group = chunk_group(r.n);
+    const int group = chunk_group(r);
     while (fit < nbase && fit < 0xffff && area.fits(b, (size_t)group * (fit + 1), UnitBytes())) ++fit;
     int groups = (nbase + fit - 1) / fit;
     if (nreq == 1 && nl > 1 && nbase >= nl) groups = (groups + nl - 1) / nl * nl;
@@ -1513,7 +1520,7 @@ int profile_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, const P
         if (j.c >= j.c1) continue;
         const ProfReq &r = reqs[j.req];
         const UnitBytes u = unit_bytes(r, crop[j.req]);
-        const int group = chunk_group(r.n), nc = std::min(j.c1, (j.c / group + 1) * group) - j.c;
+        const int group = chunk_group(r), nc = std::min(j.c1, (j.c / group + 1) * group) - j.c;
         if ((int)out.size() >= kManySegs || !area.fits(u, (size_t)j.nbase * nc, had)) break;
         const size_t units = (size_t)j.nbase * nc;
         ProfSeg s = {};

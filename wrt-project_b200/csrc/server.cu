@@ -87,7 +87,7 @@ struct Request {
   bool has_frame = false;
 };
 
-constexpr size_t kServerProfBytes = (size_t)768 << 20;
+constexpr size_t kServerProfBytes = (size_t)1536 << 20;
 constexpr size_t kServerProfLeast = (size_t)16 << 20;
 
 struct Slot {

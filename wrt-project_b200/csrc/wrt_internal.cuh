@@ -70,6 +70,8 @@ struct wrt_ctx {
   void *ws[10] = {};
   size_t ws_bytes[10] = {};
   wrt::ProfLanes prof_lanes;  // side streams of the plane transform's profiles
+  bool tables_held = false;   // a running call works in ws[WS_PROFILE]
+  size_t tables_refused = ~(size_t)0;  // a size that WS_PROFILE could not have or had to give up
   void *fft_plans = nullptr;  // spectral Laplacian plans (k_laplace.cu)
   // the volume and sphere grid of the last drop-in (host-array) call, kept
   // for the next call of the same sizes
@@ -232,9 +234,12 @@ int staged_scratch(wrt_ctx *ctx, size_t req_bytes);
 void staged_release(wrt_ctx *ctx);
 
 // Row-sum profiles (k_profile.cu): plane integrals from tables of row sums.
-// Tables of the steps in flight, all lanes together; requests with at least
-// kProfLaneBytes of tables are dealt to kProfLanes streams.
-constexpr size_t kProfTableBytes = (size_t)512 << 20;
+// Tables of the steps in flight, all lanes together: each step's launches end with
+// late blocks and wait for one another, so larger ones are faster (128^3, 64 x 128 x 256:
+// 5.4 ms with 0.5 GB, 4.6 with 1 or 2; 256^3, 96 x 192 x 384: 63, 48, 44), in what
+// the context's budget and the device leave.  Requests with at least kProfLaneBytes of
+// tables are dealt to kProfLanes streams (6 or 8: no faster).
+constexpr size_t kProfTableBytes = (size_t)2048 << 20;
 constexpr size_t kProfLaneBytes = (size_t)64 << 20;
 struct ProfReq {            // one plane transform
   const void *vol;          // v[ix][iy][iz], float or bf16
