@@ -23,7 +23,7 @@
 //           range's start from the lines directly, then one knot after another,
 //           each piece's coefficients at its own start rounded once to FP32
 //   gather: threads on voxels of one z, the list's positions in shared memory,
-//           one 16-byte record per (voxel, longitude); FP32 over 8 longitudes,
+//           one 16-byte record per (voxel, longitude); FP32 over 2 longitudes,
 //           FP64 beyond, every voxel in a fixed order by one thread
 //
 // A voxel within 2 positions (1.3e-9 in t) of the end of a line, where S jumps to
@@ -34,9 +34,8 @@
 // What bounds it: the gather's L1 tag lookups (32 lanes, 32 lines, 32 cycles per
 // request: 0.5 ms of the 128^3 case if every SM were busy), the build's latency.
 // 128^3 from 64 x 128 directions x 256 shifts: 15.9 ms by the direct kernel (16
-// bytes and ~7 instructions per voxel and direction), 1.8 here; 256^3 from 96 x
-// 192 x 384: 237 and 19.5 ms; error against FP64 6e-8 both (the float32 of the
-// comparison).
+// bytes and ~7 instructions per voxel and direction), 1.87 here; 256^3 from 96 x
+// 192 x 384: 237 and 20 ms; error against FP64 5.4e-8 both.
 #include <math.h>
 
 #include <algorithm>
@@ -98,37 +97,62 @@ __global__ void __launch_bounds__(kThreads) back_merge_kernel(const BackReq r) {
 
 // m_{i-1} + 4 m_i + m_{i+1} = y_{i+1} - 2 y_i + y_{i-1} with m_0 = m_{ns-1} = 0
 // (elimination factors cp from the host), one thread per line, lanes on
-// longitudes; on the way back the changes of the third derivative.
+// longitudes; on the way back the changes of the third derivative.  Bound by latency
+// (a few warps per SM, two chains of ns steps), so the loads of 16 steps are issued
+// together: the compiler cannot move one past the stores (40^3 from 50 x 100 x 220:
+// 455 -> 427 us in all, 334 with the lists sorted beside it).
 __global__ void __launch_bounds__(64) back_solve_kernel(const BackReq r) {
   const int L = blockIdx.x * blockDim.x + threadIdx.x;
   if (L >= r.ntheta * r.nbase) return;
   const int th = L / r.nbase, b = L % r.nbase, ns = r.ns;
   const size_t st = r.nbase, o = (size_t)th * ns * st + b;
-  const double *y = r.Y + o;
-  double *m = r.M + o, *D = r.D + o;
+  const double *__restrict__ y = r.Y + o, *__restrict__ cp = r.cp;
+  double *__restrict__ m = r.M + o, *__restrict__ D = r.D + o;
   const double kap = r.cs[2 * th + 1] * 0.5 * (ns - 1), k3 = kap * kap * kap;
+  constexpr int U = 16;  // elements whose loads are in flight together
   double prev = 0.0, ya = y[0], yb = y[st];
   m[0] = 0.0;
-#pragma unroll 8
-  for (int i = 1; i + 1 < ns; ++i) {
-    const double yc = y[(i + 1) * st];
-    prev = ((yc - 2.0 * yb + ya) - (i > 1 ? prev : 0.0)) * r.cp[i];
-    m[i * st] = prev;
-    ya = yb;
-    yb = yc;
+  for (int i0 = 1; i0 + 1 < ns; i0 += U) {
+    double v[U], w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = min(i0 + u, ns - 2);
+      v[u] = y[(i + 1) * st];
+      w[u] = cp[i];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 + u;
+      if (i + 1 >= ns) break;
+      prev = ((v[u] - 2.0 * yb + ya) - (i > 1 ? prev : 0.0)) * w[u];
+      m[i * st] = prev;
+      ya = yb;
+      yb = v[u];
+    }
   }
   // from the end: mc = m_{i+1}, md = m_{i+2}
   double mc = 0.0, md = 0.0;
   m[(ns - 1) * st] = 0.0;
-#pragma unroll 8
-  for (int i = ns - 2; i >= 0; --i) {
-    const double mi = i ? m[i * st] - r.cp[i] * mc : 0.0;
-    m[i * st] = mi;
-    // the knot i + 1: its intervals' cubic coefficients are m_{i+2} - m_{i+1}
-    // above and m_{i+1} - m_i below
-    D[(i + 1) * st] = (i + 1 == ns - 1 ? -(mc - mi) : (md - mc) - (mc - mi)) * k3;
-    md = mc;
-    mc = mi;
+  for (int i0 = ns - 2; i0 >= 0; i0 -= U) {
+    double v[U], w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = max(i0 - u, 1);
+      v[u] = m[i * st];
+      w[u] = cp[i];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int i = i0 - u;
+      if (i < 0) break;
+      const double mi = i ? v[u] - w[u] * mc : 0.0;
+      m[i * st] = mi;
+      // the knot i + 1: its intervals' cubic coefficients are m_{i+2} - m_{i+1}
+      // above and m_{i+1} - m_i below
+      D[(i + 1) * st] = (i + 1 == ns - 1 ? -(mc - mi) : (md - mc) - (mc - mi)) * k3;
+      md = mc;
+      mc = mi;
+    }
   }
   D[0] = (md - mc) * k3;
 }
@@ -376,70 +400,73 @@ __global__ void __launch_bounds__(kGatherThreads, 2) back_gather_kernel(const Ba
       y[u] = z_of(n, v % n);
       tot[u] = 0.0;
     }
-    for (int b0 = 0; b0 < B; b0 += 8) {
-      float acc[kVox];
+    float acc[kVox];
 #pragma unroll
-      for (int u = 0; u < kVox; ++u) acc[u] = 0.0f;
-      const int b1 = min(B, b0 + 8);
-      for (int b = b0; b < b1; ++b) {
-        const double2 cs = dir[b];
-        unsigned fx[kVox], nx[kVox], dt[kVox];
-        int e[kVox];
-        bool more = false, edge = false;
+    for (int u = 0; u < kVox; ++u) acc[u] = 0.0f;
+    for (int b = 0; b < B; ++b) {
+      const double2 cs = dir[b];
+      unsigned fx[kVox], nx[kVox], dt[kVox];
+      int e[kVox];
+      bool more = false, edge = false;
 #pragma unroll
-        for (int u = 0; u < kVox; ++u) {
-          const double p = fma(x[u], cs.x, fma(y[u], cs.y, kTMax * kPerT));
-          fx[u] = (unsigned)__double2loint(__dadd_rd(p, 4503599627370496.0));  // floor, + 2^52
-          e[u] = start[fx[u] >> shift];
-        }
-#pragma unroll
-        for (int h = 8; h > 0; h >>= 1)
-#pragma unroll
-          for (int u = 0; u < kVox; ++u)
-            if (pos[e[u] + h - 1] <= fx[u]) e[u] += h;
-#pragma unroll
-        for (int u = 0; u < kVox; ++u) {
-          nx[u] = pos[e[u]];
-          more |= nx[u] <= fx[u] && e[u] < total;
-        }
-        if (more) {
-#pragma unroll 1
-          for (int u = 0; u < kVox; ++u) {
-            int q = u == 0 ? e[0] : u == 1 ? e[1] : u == 2 ? e[2] : e[3];
-            const unsigned f = u == 0 ? fx[0] : u == 1 ? fx[1] : u == 2 ? fx[2] : fx[3];
-            while (q < total && pos[q] <= f) ++q;
-            if (u == 0) e[0] = q;
-            else if (u == 1) e[1] = q;
-            else if (u == 2) e[2] = q;
-            else e[3] = q;
-          }
-#pragma unroll
-          for (int u = 0; u < kVox; ++u) nx[u] = pos[e[u]];
-        }
-#pragma unroll
-        for (int u = 0; u < kVox; ++u) {
-          dt[u] = fx[u] - pos[e[u] - 1];
-          edge |= dt[u] <= kEdge || nx[u] - fx[u] <= kEdge;
-        }
-        float4 c[kVox];
-#pragma unroll
-        for (int u = 0; u < kVox; ++u) c[u] = __ldg(T + (size_t)(unsigned)(e[u] - 1) * B + b);
-#pragma unroll
-        for (int u = 0; u < kVox; ++u) {
-          const float d = (float)dt[u];
-          acc[u] += fmaf(d, fmaf(d, fmaf(d, c[u].w, c[u].z), c[u].y), c[u].x);
-        }
-        if (edge) {
-#pragma unroll
-          for (int u = 0; u < kVox; ++u)
-            if (dt[u] <= kEdge || nx[u] - fx[u] <= kEdge) {
-              const int v = min(v0 + u * kGatherThreads + tid, n2 - 1);
-              tot[u] += edge_terms(s, zi, pos, e[u], fx[u], v / n, v % n, b);
-            }
-        }
+      for (int u = 0; u < kVox; ++u) {
+        const double p = fma(x[u], cs.x, fma(y[u], cs.y, kTMax * kPerT));
+        fx[u] = (unsigned)__double2loint(__dadd_rd(p, 4503599627370496.0));  // floor, + 2^52
+        e[u] = start[fx[u] >> shift];
       }
 #pragma unroll
-      for (int u = 0; u < kVox; ++u) tot[u] += (double)acc[u];
+      for (int h = 8; h > 0; h >>= 1)
+#pragma unroll
+        for (int u = 0; u < kVox; ++u)
+          if (pos[e[u] + h - 1] <= fx[u]) e[u] += h;
+#pragma unroll
+      for (int u = 0; u < kVox; ++u) {
+        nx[u] = pos[e[u]];
+        more |= nx[u] <= fx[u] && e[u] < total;
+      }
+      if (more) {
+#pragma unroll 1
+        for (int u = 0; u < kVox; ++u) {
+          int q = u == 0 ? e[0] : u == 1 ? e[1] : u == 2 ? e[2] : e[3];
+          const unsigned f = u == 0 ? fx[0] : u == 1 ? fx[1] : u == 2 ? fx[2] : fx[3];
+          while (q < total && pos[q] <= f) ++q;
+          if (u == 0) e[0] = q;
+          else if (u == 1) e[1] = q;
+          else if (u == 2) e[2] = q;
+          else e[3] = q;
+        }
+#pragma unroll
+        for (int u = 0; u < kVox; ++u) nx[u] = pos[e[u]];
+      }
+#pragma unroll
+      for (int u = 0; u < kVox; ++u) {
+        dt[u] = fx[u] - pos[e[u] - 1];
+        edge |= dt[u] <= kEdge || nx[u] - fx[u] <= kEdge;
+      }
+      float4 c[kVox];
+#pragma unroll
+      for (int u = 0; u < kVox; ++u) c[u] = __ldg(T + (size_t)(unsigned)(e[u] - 1) * B + b);
+#pragma unroll
+      for (int u = 0; u < kVox; ++u) {
+        const float d = (float)dt[u];
+        acc[u] += fmaf(d, fmaf(d, fmaf(d, c[u].w, c[u].z), c[u].y), c[u].x);
+      }
+      if (edge) {
+#pragma unroll
+        for (int u = 0; u < kVox; ++u)
+          if (dt[u] <= kEdge || nx[u] - fx[u] <= kEdge) {
+            const int v = min(v0 + u * kGatherThreads + tid, n2 - 1);
+            tot[u] += edge_terms(s, zi, pos, e[u], fx[u], v / n, v % n, b);
+          }
+      }
+      // FP32 over two longitudes (over eight, the error against FP64 was a fifth larger)
+      if ((b & 1) | (b + 1 == B)) {
+#pragma unroll
+        for (int u = 0; u < kVox; ++u) {
+          tot[u] += (double)acc[u];
+          acc[u] = 0.0f;
+        }
+      }
     }
 #pragma unroll
     for (int u = 0; u < kVox; ++u) {
@@ -515,11 +542,7 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
   r.M = reinterpret_cast<double *>(at + p.data);
   r.D = reinterpret_cast<double *>(at + 2 * p.data);
   at += 3 * p.data;
-  const dim3 grid((p.nbase + 31) / 32, (r.ntheta + 31) / 32, r.ns);
-  back_merge_kernel<<<grid, kThreads, 0, stream>>>(r);
-  back_solve_kernel<<<(r.ntheta * p.nbase + 63) / 64, 64, 0, stream>>>(r);
-  ctx->launches += 2;
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = cudaSuccess;
   // ---- z planes, dealt in groups to the lanes
   char *lists = at;
   at += (size_t)r.n * p.list();
@@ -551,14 +574,25 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
   s0.ids = s0.pos + (size_t)(p.cap + 16) * r.n;
   s0.start = reinterpret_cast<unsigned *>(lists + (size_t)r.n * (p.rec + p.pos));
   s0.keys = reinterpret_cast<unsigned long long *>(lists + (size_t)r.n * (p.rec + p.pos + p.start));
-  if (e == cudaSuccess) {
-    back_sort_kernel<<<r.n, kSortThreads, sm_sort, stream>>>(s0);
-    ctx->launches++;
-    e = cudaGetLastError();
-  }
   if (nl > 1) {
     int st = profile_lanes_init(ctx, lanes);
     if (st) return st;
+    // the lists do not depend on the data: beside the splines
+    if (e == cudaSuccess) e = cudaEventRecord(lanes->fork, stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(lanes->stream[0], lanes->fork, 0);
+  }
+  if (e == cudaSuccess) {
+    const cudaStream_t ls = nl > 1 ? lanes->stream[0] : stream;
+    back_sort_kernel<<<r.n, kSortThreads, sm_sort, ls>>>(s0);
+    const dim3 grid((p.nbase + 31) / 32, (r.ntheta + 31) / 32, r.ns);
+    back_merge_kernel<<<grid, kThreads, 0, stream>>>(r);
+    back_solve_kernel<<<(r.ntheta * p.nbase + 63) / 64, 64, 0, stream>>>(r);
+    ctx->launches += 3;
+    e = cudaGetLastError();
+  }
+  if (nl > 1) {
+    if (e == cudaSuccess) e = cudaEventRecord(lanes->done[0], lanes->stream[0]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, lanes->done[0], 0);
     if (e == cudaSuccess) e = cudaEventRecord(lanes->fork, stream);
     for (int k = 1; k < nl && e == cudaSuccess; ++k)
       e = cudaStreamWaitEvent(lanes->stream[k - 1], lanes->fork, 0);
