@@ -354,17 +354,14 @@ def other_paths(wrt, ctx, phantom, steps, warmup, smem_bw, with_cpu):
     # what binds each kernel, from its committed ncu capture (a profiler cannot
     # run inside the timed bench): the byte figure above is the algorithmic
     # gather, not always the limit
-    for k, b in (("nearest", "issue: 79 % of issue slots, 3.15 instructions per clock; a 4-byte "
-                             "warp load is one shared wavefront, so the byte figure is not the "
-                             "limit (profiles/plane_staged_nearest_128cubed.md)"),
-                 ("ray", "L1 gathers: 64 % of L1 throughput, 20 of 32 lanes busy (parallel rays "
-                         "of different chord lengths) (profiles/ray_kernel_128cubed.md)"),
+    for k, b in (("nearest", "gathers of the row tables from L2, late blocks of dependent launches; "
+                             "samples share table entries, so the byte figure is not the limit"),
+                 ("ray", "column loads along z, shared by all slices of a (shift, angle)"),
                  ("ray_rotated", "L1 gathers: 82 % of L1 throughput "
                                  "(profiles/ray_kernel_128cubed.md)"),
-                 ("reduction", "L1 sectors: 97.5 % of L1 throughput at ~30 sectors per request "
-                               "(profiles/reduction_kernel_128cubed.md)"),
-                 ("adjoint", "latency of the record gathers: long-scoreboard stalls, 68 % issue, "
-                             "59 % of the L1 data pipe (profiles/adjoint_kernel_128cubed.md)")):
+                 ("reduction", "shared-memory wavefronts: 90 % of the peak"),
+                 ("adjoint", "L1 tag lookups of the record gathers; evaluations share merged "
+                             "splines, so the byte figure is not the limit")):
         res[k]["roofline"]["limit_measured"] = b
     if with_cpu:
         import oracle as O
@@ -567,20 +564,6 @@ def batch_vs_one_per_launch(wrt, ctx, steps, count=64, edges=(48, 64, 96, 128, 1
 
 
 # ------------------------------------------------------------ our arm
-def traffic_from_profiles():
-    """DRAM bytes per launch of the plane kernel from the committed ncu summary."""
-    f = ROOT / "profiles" / "plane_staged_kernel_128cubed.md"
-    if not f.exists():
-        return None
-    for ln in f.read_text().splitlines():
-        if ln.strip().startswith("dram_bytes_per_launch:"):
-            try:
-                return float(ln.split(":", 1)[1].split()[0])
-            except ValueError:
-                return None
-    return None
-
-
 def served_stream(wrt, srv, pin_vol, pin_outs, steps):
     """K requests of the workload through the serving loop, each with its FP32
     volume in pinned host memory and its FP64 result copied back to pinned
@@ -981,8 +964,8 @@ def run_ours(args, dist):
     lat = np.array([i.done_ms - i.submit_ms for i in infos])
     served_equal = bool(np.array_equal(served_res, result_dev))
 
-    # roofline of the plane kernel: 32 B of staged voxel reads per sample
-    # against the measured shared-memory bandwidth of this device
+    # compulsory HBM bytes, and the lattice's samples at 32 B each against the
+    # measured shared-memory bandwidth of this device
     smem_bw = ctx.smem_bandwidth()
     per_launch_s = ms_per_step * 1e-3
     achieved = samples * BYTES_PER_SAMPLE / per_launch_s / 1e9
@@ -1007,17 +990,17 @@ def run_ours(args, dist):
         "samples_per_step": samples,
         "samples_per_s": samples * args.steps * dist.world / (total_ms * 1e-3),
         "gpu_launches": launches,
-        "roofline": {"bound": "l1tex", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                     "frac": achieved / peak if peak else None, "traffic": traffic_from_profiles(),
-                     "traffic_source": "dram__bytes_read.sum + dram__bytes_write.sum per launch "
-                                       "from the committed ncu capture of this workload "
-                                       "(profiles/plane_staged_kernel_128cubed.md), not "
-                                       "measured in this run",
-                     "peak_source": "shared-memory read bandwidth measured in this run "
-                                    "(wrt_measure_smem_bandwidth); 32 B per trilinear sample",
-                     "hbm": {"achieved": hbm_bytes / per_launch_s / 1e9, "peak": hbm_peak,
-                             "unit": "GB/s", "frac": hbm_bytes / per_launch_s / 1e9 / hbm_peak,
-                             "note": "compulsory bytes only; the volume is re-read from L2"}},
+        "roofline": {"bound": "latency", "achieved": hbm_bytes / per_launch_s / 1e9,
+                     "peak": hbm_peak, "unit": "GB/s",
+                     "frac": hbm_bytes / per_launch_s / 1e9 / hbm_peak,
+                     "note": "compulsory HBM bytes (volume in, results out); the kernel reads its "
+                             "row sums from tables in L2 and waits for those gathers",
+                     "lattice": {"achieved": achieved, "peak": peak, "unit": "GB/s",
+                                 "note": "32 B per trilinear sample of the lattice against the "
+                                         "shared-memory read bandwidth measured in this run "
+                                         "(wrt_measure_smem_bandwidth): what evaluating every "
+                                         "sample would have to read.  The samples of a row share "
+                                         "its table entry, so this may exceed the peak"}},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": N ** 3 * 4,
                 "d2h_bytes_per_step": nplanes * 8,
                 "path": "wrt_server: one request per step, pinned FP32 volume in, pinned FP64 "

@@ -62,7 +62,8 @@ typedef enum wrt_kernel {
                             else the plain one */
   WRT_KERNEL_PLAIN = 1,  /* one warp per plane, gathers through L1 */
   WRT_KERNEL_STAGED = 2  /* the row-sum profiles where they cover and suit the request
-                            (working memory of up to ~750 MB in the context), else
+                            (working memory of up to 3 GB in the context, less
+                            where its budget or the device has less), else
                             volume layers staged in shared memory, persistent CTAs:
                             trilinear from the layer pairs (FP32 or BF16 storage),
                             nearest from the z-major cell layers (FP32 storage) */
@@ -386,7 +387,10 @@ typedef struct wrt_server_opts {
   int max_inflight;    /* launches on the device at once (0: 2; at most 8) */
   int queue_capacity;  /* requests waiting for admission (0: 65536) */
   size_t hbm_budget;   /* device memory for request state and grid tables
-                          (0: 60 GiB or 3/4 of the free memory, whichever is less) */
+                          (0: 60 GiB or 3/4 of the free memory, whichever is less);
+                          tables that only make requests faster come beside it,
+                          where there is room: an eighth of it, at most 3 GB,
+                          per launch in flight */
   int reserved[8];
 } wrt_server_opts;
 

@@ -87,7 +87,7 @@ struct Request {
   bool has_frame = false;
 };
 
-constexpr size_t kServerProfBytes = (size_t)1536 << 20;
+constexpr size_t kServerProfBytes = (size_t)3072 << 20;
 constexpr size_t kServerProfLeast = (size_t)16 << 20;
 
 struct Slot {
@@ -681,15 +681,27 @@ int wrt_server_create(const wrt_server_opts *opts, wrt_server **out) {
       break;
     }
     st = wrt::batch_slot_init(ctx, &sl->batch, sl->stream);
-    // working memory of the row-sum profiles, beside the arena: a sixteenth of
+    // working memory of the row-sum profiles, beside the arena: an eighth of
     // the budget per slot, at most kServerProfBytes; without it (small budgets,
-    // no memory left) the plane transforms take the staged kernel
-    const size_t want = std::min(budget / 16, kServerProfBytes) & ~(size_t)0xffff;
+    // no memory left) the plane transforms take the staged kernel.  The host does not
+    // know a volume's support, so units have room for all of the cube and fewer fit a
+    // step (128^3, 64 x 128 x 256, ten requests at once: 13.5 ms each with 256 MB a
+    // slot, 9.4 with 512, 7.6 with 1 GB, 7.0 with 1.5, 6.7 with 3)
+    const size_t want = std::min(budget / 8, kServerProfBytes) & ~(size_t)0xffff;
     if (!st && want >= kServerProfLeast &&
         wrt::ctx_alloc(ctx, &sl->batch.prof_ws, want) == WRT_OK)
       sl->batch.prof_bytes = want;
     s->slots.push_back(std::move(sl));
   }
+  // every slot or none: a request's kernel must not depend on the slot it gets
+  bool every = true;
+  for (auto &sl : s->slots) every = every && sl->batch.prof_bytes > 0;
+  if (!every)
+    for (auto &sl : s->slots) {
+      wrt::ctx_free(ctx, sl->batch.prof_ws, sl->batch.prof_bytes);
+      sl->batch.prof_ws = nullptr;
+      sl->batch.prof_bytes = 0;
+    }
   if (st) {
     s->stop = true;
     wrt_server_destroy(s);
