@@ -128,6 +128,20 @@ def test_backprojection_matches_oracle(ctx, n, nphi, ntheta, nshift):
     assert rel_l2(got[pick[:, 0], pick[:, 1], pick[:, 2]], ref) < TOL_L2
 
 
+# the spline solve takes 16 elements at a time: the shortest line, and lines of one
+# element less than a whole number of groups, of a whole number and of one more
+@pytest.mark.parametrize("n,nphi,ntheta,nshift", [
+    (9, 300, 300, 3), (9, 98, 160, 17), (10, 96, 160, 18), (11, 96, 160, 19), (12, 96, 90, 34),
+])
+def test_backprojection_short_lines_match_oracle(ctx, n, nphi, ntheta, nshift):
+    radon = np.random.default_rng(n).standard_normal((nshift, nphi, ntheta))
+    got = ctx.radon3d_adjoint(radon, n)
+    x = -1.0 + (2.0 * np.arange(n) + 1.0) / n
+    pick = np.random.default_rng(2).integers(0, n, (200, 3))
+    ref = O.adjoint_points(radon, x[pick[:, 1]], x[pick[:, 2]], x[pick[:, 0]])
+    assert rel_l2(got[pick[:, 0], pick[:, 1], pick[:, 2]], ref) < TOL_L2
+
+
 def test_tables_make_room():
     # the tables' buffer may fill the budget; what is allocated next still fits
     with wrt.Context(0, budget_bytes=96 << 20) as c:
