@@ -41,7 +41,7 @@
 // launch waits for its gathers (random 32-byte reads, mostly from L2) and FP64
 // geometry, the build for its node loads.  128^3, 64 x 128 directions x 256
 // shifts, lattice [-n, n)^2: 53.7 ms by the staged kernel (lattice samples
-// through shared memory), 4.6 ms here; 256^3 BF16, 96 x 192 x 384: 750 and 44
+// through shared memory), 4.6-4.9 ms here; 256^3 BF16, 96 x 192 x 384: 750 and 44
 // ms; error against FP64 6.5e-8 (staged 8.9e-8).  Small requests wait for the four
 // launches one after another (24^3, 8 x 16 x 32: 109 and 80 us).
 #include <math.h>
