@@ -62,9 +62,7 @@ constexpr unsigned kAll = 0xffffffffu;
 constexpr int kThreads = 256;
 constexpr int kSortThreads = 1024;
 constexpr int kMaxChunks = 6;  // ranges of t of one phi in a step
-constexpr double kMagicPos = 6442450944.0;            // 1.5 * 2^32: 20 fraction bits
 constexpr double kMagicInt = 6755399441055744.0;      // 1.5 * 2^52
-constexpr unsigned kBoundary = 2;  // 2^-20 bins: rows this near a piece end go exact
 using namespace wrtp;
 
 __device__ __forceinline__ float crop_of(const ProfReq &r) {
@@ -85,7 +83,15 @@ __device__ __forceinline__ Geo geo_of_unit(const ProfSeg &s, int unit) {
 // One block (of 1024 threads: few blocks, on which the whole step waits) finds the
 // unit's piece boundaries, counts them per bin, and writes
 // them in order of (position, identity): a bin's few entries are ranked by
-// counting, so the order does not depend on the atomics.
+// counting, so the order does not depend on the atomics.  The identities of
+// boundaries just beyond the unit's ends go behind the list, kMaxWindow on each side
+// (more are only counted, after start[kUnitBins]).
+constexpr int kMaxWindow = 8;  // more boundaries than this at one t: whole row by the warp
+
+__device__ __forceinline__ unsigned boundary_id(int kind, int li, int m) {
+  return ((unsigned)kind << 29 | (unsigned)li << 13 | (unsigned)m) + 1u;
+}
+
 __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
   const Geo g = geo_of_unit(s, unit);
   unsigned *pos = s.pos + (size_t)unit * (s.cap + 16);
@@ -93,10 +99,11 @@ __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
   unsigned *start = s.start + (size_t)unit * (kUnitBins + 8);
   int *cnt = reinterpret_cast<int *>(smem);           // [kUnitBins]
   int *cur = cnt + kUnitBins;                         // [kUnitBins]
-  __shared__ int s_warp[kSortThreads / 32];
+  __shared__ int s_warp[kSortThreads / 32], s_beyond[2];
   const int tid = threadIdx.x;
   const bool skip = s.r.nearest && on_axis(g);
   for (int b = tid; b < kUnitBins; b += kSortThreads) cnt[b] = 0;
+  if (tid < 2) s_beyond[tid] = 0;
   __syncthreads();
   if (!skip)
     each_boundary(g, s.nsub, s.sub_bins, (int)threadIdx.x, kSortThreads,
@@ -131,15 +138,30 @@ __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
   if (tid == 0) start[kUnitBins] = total;
   unsigned long long *keys = s.keys + (size_t)unit * s.cap;
   if (!skip)
-    each_boundary(g, s.nsub, s.sub_bins, (int)threadIdx.x, kSortThreads, [&](unsigned p, int kind, int li, int m) {
-      const int slot = atomicAdd(&cur[p >> 20], 1);
-      // the sub-range's start precedes everything at its position
-      const unsigned id = kind == K_NULL ? 0u
-                                         : ((unsigned)kind << 29 | (unsigned)li << 13 |
-                                            (unsigned)m) + 1u;
-      if (slot < s.cap) keys[slot] = (unsigned long long)p << 32 | id;
-    });
+    each_boundary(g, s.nsub, s.sub_bins, (int)threadIdx.x, kSortThreads,
+                  [&](unsigned p, int kind, int li, int m) {
+                    const int slot = atomicAdd(&cur[p >> 20], 1);
+                    // the sub-range's start precedes everything at its position
+                    const unsigned id = kind == K_NULL ? 0u : boundary_id(kind, li, m);
+                    if (slot < s.cap) keys[slot] = (unsigned long long)p << 32 | id;
+                  },
+                  [&](bool after, int kind, int li, int m) {
+                    const int slot = atomicAdd(&s_beyond[after], 1);
+                    if (slot < kMaxWindow)
+                      ids[s.cap + after * kMaxWindow + slot] = boundary_id(kind, li, m);
+                  });
   __syncthreads();
+  if (tid < 2) {  // in order of identity
+    const int m = s_beyond[tid];
+    unsigned *list = ids + s.cap + tid * kMaxWindow;
+    start[kUnitBins + 1 + tid] = m;
+    for (int a = 1; a < min(m, kMaxWindow); ++a)
+      for (int b = a; b > 0 && list[b] < list[b - 1]; --b) {
+        const unsigned t = list[b];
+        list[b] = list[b - 1];
+        list[b - 1] = t;
+      }
+  }
   PieceRec *rec = static_cast<PieceRec *>(s.rec) + (size_t)unit * s.cap;
   for (int e = tid; e < total; e += kSortThreads) {
     const unsigned long long key = keys[e];
@@ -156,7 +178,8 @@ __device__ void role_sort(const ProfSeg &s, int unit, char *smem) {
                              s.sub_bins, s.r.nearest)
                   : make_rec(g, p, K_NULL, 0, 0, s.sub_bins, s.r.nearest);
   }
-  if (tid < 16) pos[total + tid] = 0xffffffffu;
+  // no row is past the unit's end; one next to it is not decided by the table
+  if (tid < 16) pos[total + tid] = kUnitEnd;
 }
 
 // ----------------------------------------------------------------- build role
@@ -442,23 +465,23 @@ __device__ __noinline__ double exact_row(const ProfReq &r, int d, int is, int i,
 }
 
 // What is missing from the table's value of a row that lies within kBoundary
-// of the piece boundaries [q0, q1): for each sample they belong to, its value
+// of `count` piece boundaries: for each sample they belong to, its value
 // by the reference's arithmetic minus the value it has in the table's piece.
 __device__ __noinline__ double boundary_terms(const ProfReq &r, const Geo &g, const unsigned *ids,
-                                              int q0, int q1, unsigned fx, double t, int iz,
-                                              double tz, int d, int is, int i, bool mirrored) {
+                                              int count, unsigned fx, double t, int iz, double tz,
+                                              int d, int is, int i, bool mirrored) {
   double sum = 0.0;
   const int n = r.n;
   const float *v = static_cast<const float *>(r.vol);
   const __nv_bfloat16 *bv = static_cast<const __nv_bfloat16 *>(r.vol);
   const bool bf = r.storage == WRT_STORAGE_BF16;
   auto f = [&](int x) { return (double)(bf ? ld_node(bv, x) : ld_node(v, x)); };
-  for (int q = q0; q < q1; ++q) {
+  for (int q = 0; q < count; ++q) {
     const unsigned id = ids[q];
     if (!id) continue;
     const unsigned line = (id - 1u) >> 13 & 0xffffu;
     bool seen = false;
-    for (int x = q0; x < q; ++x) seen |= ids[x] && ((ids[x] - 1u) >> 13 & 0xffffu) == line;
+    for (int x = 0; x < q; ++x) seen |= ids[x] && ((ids[x] - 1u) >> 13 & 0xffffu) == line;
     if (seen) continue;
     const int j = g.jlo + (int)line;
     const Line l = make_line(g, j);
@@ -485,8 +508,6 @@ __device__ __noinline__ double boundary_terms(const ProfReq &r, const Geo &g, co
   return sum;
 }
 
-constexpr int kMaxWindow = 8;  // more boundaries than this at one t: whole row by the warp
-
 // First piece boundary past fx (binary steps while many share the bin: phis on
 // or near an axis, where whole columns of samples cross together).
 template <typename S>
@@ -502,23 +523,6 @@ __device__ __forceinline__ int find_piece(const unsigned *pos, const S *start, u
   return lo;
 }
 
-// Bin and z cell of the rows of one (phi, theta): row i of shift s lies at
-// u = s ub + uo + i u1 bins of the unit and at z cell s wb + h + i w1.
-struct RowGeo {
-  double ub, uo, u1, wb, wo, w1;
-};
-__device__ __forceinline__ RowGeo row_geo(const ProfReq &r, const Geo &g, int d) {
-  const double *D = r.dir + 9 * (size_t)d;
-  RowGeo q;
-  q.ub = (__ldg(D) * g.cu + __ldg(D + 1) * g.su) * g.h * g.n;
-  q.uo = g.toff * g.n - g.tfirst;
-  q.u1 = (__ldg(D + 3) * g.cu + __ldg(D + 4) * g.su) * g.dl * g.n;
-  q.wb = __ldg(D + 2) * g.h;
-  q.wo = g.h;
-  q.w1 = __ldg(D + 5) * g.dl;
-  return q;
-}
-
 // Where a row lies: position in the unit, z cell and fraction.  layer: within
 // 1e-9 cells of a node layer (or rounding to one).
 struct RowAt {
@@ -527,14 +531,15 @@ struct RowAt {
   float tz;
   bool in, layer;  // in: in the unit; layer rows are not read from the table
 };
-__device__ __forceinline__ RowAt row_at(double di, double u0, double u1, double w0, double w1) {
+__device__ __forceinline__ RowAt row_at(double di, double u0, double u1, double w0, double w1,
+                                        double tfirst) {
   RowAt a;
-  a.fx = (unsigned)__double2loint(__dadd_rd(fma(di, u1, u0), kMagicPos));
+  a.fx = row_pos(fma(di, u1, u0), tfirst);
   const double w = fma(di, w1, w0);
   const double mz = __dadd_rd(w, kMagicInt);
   a.iz = __double2loint(mz);
   a.tz = (float)(w - (mz - kMagicInt));
-  a.in = a.fx < (unsigned)kUnitBins << 20;
+  a.in = a.fx < kUnitEnd;
   a.layer = a.tz < 1e-9f || a.tz >= 1.0f;
   return a;
 }
@@ -563,8 +568,8 @@ __device__ __noinline__ bool settle_layer(const ProfReq &r, int d, double sh, do
 // Rows lo .. lo + len - 1 of shift sh that can lie in the unit, the cube and the
 // crop ball.
 __device__ __forceinline__ int row_range(const ProfReq &r, const Geo &g, const RowGeo &w,
-                                         double crop, double sh, double u0, double w0, int *lo_out) {
-  const double rem = crop - sh * sh;
+                                         double crop, double sh, double u, double w0, int *lo_out) {
+  const double rem = crop - sh * sh, u0 = u - g.tfirst;
   *lo_out = 1;
   if (!(rem >= 0.0)) return 0;
   const int im = (int)(sqrt(rem) * r.n);
@@ -597,7 +602,7 @@ __device__ __forceinline__ double slow_rows(const ProfSeg &s, const Geo &g, cons
   const unsigned *ids = s.ids + (size_t)unit * (s.cap + 16);
   const unsigned *start = s.start + (size_t)unit * (kUnitBins + 8);
   const int total = start[kUnitBins], lane = threadIdx.x & 31, n = r.n;
-  RowAt a = row_at((double)i, u0, q.u1, w0, q.w1);
+  RowAt a = row_at((double)i, u0, q.u1, w0, q.w1, g.tfirst);
   act = act && a.in;
   // a settled row is read here, the others' table values the fast pass has added
   const bool settled = r.nearest && act && a.layer && settle_layer(r, d, __ldg(r.shift + is), (double)i, &a);
@@ -608,7 +613,11 @@ __device__ __forceinline__ double slow_rows(const ProfSeg &s, const Geo &g, cons
     int q0 = e, q1 = e;
     while (q0 > 0 && a.fx - pos[q0 - 1] <= kBoundary && e - q0 <= kMaxWindow) --q0;
     while (q1 < total && pos[q1] - a.fx <= kBoundary && q1 - e <= kMaxWindow) ++q1;
-    if (q1 - q0 > kMaxWindow || settled) {
+    // the neighbouring units' boundaries next to this one's ends
+    const int before = a.fx <= kBoundary ? (int)start[kUnitBins + 1] : 0;
+    const int after = kUnitEnd - a.fx <= kBoundary ? (int)start[kUnitBins + 2] : 0;
+    const int count = q1 - q0 + before + after;
+    if (count > kMaxWindow || settled) {
       const size_t o = ((size_t)unit * s.cap + (e - 1)) * n + a.iz;
       if (r.nearest) {
         val = (double)__ldg(static_cast<const float *>(s.table) + o);
@@ -621,12 +630,17 @@ __device__ __forceinline__ double slow_rows(const ProfSeg &s, const Geo &g, cons
         val = (double)fmaf(a.tz, vb - va, va);
       }
     }
-    if (q1 - q0 > kMaxWindow) {
+    if (count > kMaxWindow) {
       whole = true;
-    } else if (q1 > q0) {
+    } else if (count > 0) {
+      unsigned win[kMaxWindow];
+      int m = 0;
+      for (int k = 0; k < before; ++k) win[m++] = ids[s.cap + k];
+      for (int k = q0; k < q1; ++k) win[m++] = ids[k];
+      for (int k = 0; k < after; ++k) win[m++] = ids[s.cap + kMaxWindow + k];
       const double t = (fma((double)i, q.u1, u0) - q.uo) / n;
       const double w = fma((double)i, q.w1, w0);
-      add = boundary_terms(r, g, ids, q0, q1, a.fx, t, a.iz, w - (double)a.iz, d, is, i, mirrored);
+      add = boundary_terms(r, g, win, m, a.fx, t, a.iz, w - (double)a.iz, d, is, i, mirrored);
     }
     if (settled) {
       add += val;
@@ -681,7 +695,7 @@ __global__ void __launch_bounds__(kSlowThreads)
       for (int c = 0; c < s.nchunk; ++c) {
         if (!(item >> (kMarkChunk + c) & 1u)) continue;
         const Geo g = geo_of(r, s.base0 + phi, s.chunk + c);
-        const RowGeo q = row_geo(r, g, d);
+        const RowGeo q = row_geo(r.dir + 9 * (size_t)d, g);
         const double u0 = fma(sh, q.ub, q.uo), w0 = fma(sh, q.wb, q.wo);
         int lo;
         const int len = row_range(r, g, q, crop, sh, u0, w0, &lo);
@@ -718,14 +732,14 @@ template <bool NEAR>
 __device__ __forceinline__ bool rows4(const void *table, const unsigned *pos,
                                       const unsigned short *start, int n, int W, double di,
                                       double step, double u0, double u1, double w0, double w1,
-                                      int m, double *sum) {
+                                      double tfirst, int m, double *sum) {
   constexpr int P = 4;
   RowAt a[P];
   int e[P];
   bool ok[P], flag = false;
 #pragma unroll
   for (int u = 0; u < P; ++u) {
-    a[u] = row_at(di + step * u, u0, u1, w0, w1);
+    a[u] = row_at(di + step * u, u0, u1, w0, w1, tfirst);
     const bool act = u < m && a[u].in;
     flag |= act && a[u].layer;
     ok[u] = act && !a[u].layer && (unsigned)a[u].iz < (unsigned)W;
@@ -790,9 +804,8 @@ __device__ __forceinline__ bool rows4(const void *table, const unsigned *pos,
 
 // Lattice samples of a row inside the crop ball (measurement only).
 __device__ __noinline__ int row_samples(const ProfReq &r, int is, int i, double u0, double a1,
-                                        double crop) {
-  const double ul = fma((double)i, a1, u0);
-  if (ul < 0.0 || ul >= kUnitBins) return 0;
+                                        double tfirst, double crop) {
+  if (row_pos(fma((double)i, a1, u0), tfirst) >= kUnitEnd) return 0;
   const double sq = r.shift[is], di = (double)i / r.n;
   const double r2 = crop - sq * sq - di * di;
   const int jm = r2 > 0.0 ? (int)(sqrt(r2) * r.n) : 0;
@@ -845,7 +858,7 @@ __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long
     const int W = g.W;
     const char *table = static_cast<const char *>(s.table) +
                         (size_t)unit * s.cap * n * (NEAR ? 4 : 16);
-    const RowGeo w = row_geo(r, g, d);
+    const RowGeo w = row_geo(r.dir + 9 * (size_t)d, g);
     // ---- row ranges, lane = plane
     int lo = 1, len = 0;
     double u0 = 0.0, w0 = 0.0;
@@ -864,7 +877,8 @@ __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long
     if ((most + 3) >> 2 <= wide) {
       double di = (double)lo;
       for (int x = 0; x < most; x += 4, di += 4.0)
-        flag |= rows4<NEAR>(table, pos, start, n, W, di, 1.0, u0, w.u1, w0, w.w1, len - x, &mine);
+        flag |= rows4<NEAR>(table, pos, start, n, W, di, 1.0, u0, w.u1, w0, w.w1, g.tfirst, len - x,
+                            &mine);
     } else {
       for (int p = 0; p < np; ++p) {
         const int lenp = __shfl_sync(kAll, len, p);
@@ -873,7 +887,7 @@ __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long
         double di = (double)(__shfl_sync(kAll, lo, p) + lane), acc = 0.0;
         bool mark = false;
         for (int x = lane; x - lane < lenp; x += 128, di += 128.0)
-          mark |= rows4<NEAR>(table, pos, start, n, W, di, 32.0, up, w.u1, wp, w.w1,
+          mark |= rows4<NEAR>(table, pos, start, n, W, di, 32.0, up, w.u1, wp, w.w1, g.tfirst,
                               (lenp - x + 31) >> 5, &acc);
         acc = wrtd::warp_sum(acc);
         mark = __any_sync(kAll, mark);
@@ -887,7 +901,7 @@ __device__ void role_rows(const ProfSeg &s, int seg, int blk, unsigned long long
     if (r.counter) {
       unsigned long long counted = 0;
       for (int x = 0; x < len; ++x)
-        counted += row_samples(r, is0 + lane, lo + x, u0, w.u1, crop);
+        counted += row_samples(r, is0 + lane, lo + x, u0, w.u1, g.tfirst, crop);
       if (counted) atomicAdd(r.counter, counted);
     }
   }

@@ -20,16 +20,20 @@ PROF_FN double prof_mul(double a, double b) { return __dmul_rn(a, b); }
 PROF_FN double prof_add(double a, double b) { return __dadd_rn(a, b); }
 PROF_FN double prof_sub(double a, double b) { return __dsub_rn(a, b); }
 PROF_FN long long prof_floor(double a) { return __double2ll_rd(a); }
+PROF_FN double prof_ld(const double *p) { return __ldg(p); }
 #else
 PROF_FN double prof_mul(double a, double b) { return a * b; }
 PROF_FN double prof_add(double a, double b) { return a + b; }
 PROF_FN double prof_sub(double a, double b) { return a - b; }
 PROF_FN long long prof_floor(double a) { return (long long)floor(a); }
+PROF_FN double prof_ld(const double *p) { return *p; }
 #endif
 PROF_FN int imax(int a, int b) { return a > b ? a : b; }
 PROF_FN int imin(int a, int b) { return a < b ? a : b; }
 
 constexpr int kUnitBins = 2048;  // bins of t per unit of work
+constexpr unsigned kUnitEnd = (unsigned)kUnitBins << 20;  // its length in positions
+constexpr unsigned kBoundary = 2;  // 2^-20 bins: rows this near a piece end go exact
 // A horizontal axis component below this is a rounding of zero (phi on an
 // axis): samples then never cross that axis' cell boundaries.
 constexpr double kAxis = 1e-9;
@@ -177,15 +181,22 @@ PROF_FN int ycell(const Geo &g, double jd, double t, Passed p) {
 
 PROF_FN float clamp01(double x) { return (float)fmin(fmax(x, 0.0), 1.0); }
 
-// Calls f(pos, kind, line index, m) for every piece boundary of the unit, the
-// tasks dealt to `step` callers (this one is number `first`).
+// Calls f(pos, kind, line index, m) for every piece boundary of the unit, and
+// beyond(after, kind, line index, m) for those up to kBoundary before its start
+// and after its end (pieces of the units next to it, which a row at this one's end
+// may lie on), the tasks dealt to `step` callers (this one is number `first`).
 // Tasks 0 .. 3 nl - 1: per line its x crossings, its y crossings, its entry
 // and exit; then the sub-range starts.
-template <class F>
-PROF_FN void each_boundary(const Geo &g, int nsub, int sub_bins, int first, int step, F f) {
+template <class F, class B>
+PROF_FN void each_boundary(const Geo &g, int nsub, int sub_bins, int first, int step, F f,
+                           B beyond) {
   const int nl = imax(0, g.jhi - g.jlo + 1);
   const double ta = g.tfirst / g.n - g.toff, tb = (g.tfirst + kUnitBins) / g.n - g.toff;
-  const long long end = (long long)kUnitBins << 20;
+  const long long end = kUnitEnd, near = kBoundary;
+  auto at = [&](long long p, int kind, int li, int m) {
+    if (p >= 0 && p < end) f((unsigned)p, kind, li, m);
+    else if (p >= -near && p < end + near) beyond(p >= end, kind, li, m);
+  };
   for (int k = first; k < 3 * nl + nsub; k += step) {
     if (k >= 3 * nl) {
       const int sub = k - 3 * nl;
@@ -204,8 +215,7 @@ PROF_FN void each_boundary(const Geo &g, int nsub, int sub_bins, int first, int 
       for (int e = 0; e < 2; ++e) {
         const double t = e ? l.tout : l.tin;
         if (fabs(t) > tc) continue;
-        const long long p = pos_of(g, t);
-        if (p >= 0 && p < end) f((unsigned)p, e ? K_OUT : K_IN, li, 0);
+        at(pos_of(g, t), e ? K_OUT : K_IN, li, 0);
       }
       continue;
     }
@@ -220,10 +230,13 @@ PROF_FN void each_boundary(const Geo &g, int nsub, int sub_bins, int first, int 
     for (int m = m0; m <= m1; ++m) {
       const double t = what ? ty_of(g, l.jd, m) : tx_of(g, l.jd, m);
       if (!(t > l.tin && t < l.tout) || fabs(t) > tc) continue;
-      const long long p = pos_of(g, t);
-      if (p >= 0 && p < end) f((unsigned)p, what ? K_Y : K_X, li, m);
+      at(pos_of(g, t), what ? K_Y : K_X, li, m);
     }
   }
+}
+template <class F>
+PROF_FN void each_boundary(const Geo &g, int nsub, int sub_bins, int first, int step, F f) {
+  each_boundary(g, nsub, sub_bins, first, step, f, [](bool, int, int, int) {});
 }
 
 PROF_FN PieceRec make_rec(const Geo &g, unsigned pos, int kind, int li, int m,
@@ -268,5 +281,35 @@ PROF_FN PieceRec make_rec(const Geo &g, unsigned pos, int kind, int li, int m,
   return r;
 }
 
+// Where the rows of one (phi, theta) lie: row i of shift s at bin u = s ub + uo +
+// i u1, counted from bin 0 of t for every unit alike, and at z cell s wb + wo + i w1.
+struct RowGeo {
+  double ub, uo, u1, wb, wo, w1;
+};
+PROF_FN RowGeo row_geo(const double *D, const Geo &g) {  // D: the direction's nine numbers
+  RowGeo q;
+  // (roundings spelled out: every kernel has to find the same u)
+  q.ub = prof_mul(fma(prof_ld(D), g.cu, prof_mul(prof_ld(D + 1), g.su)), prof_mul(g.h, g.n));
+  q.uo = prof_mul(g.toff, g.n);
+  q.u1 = prof_mul(fma(prof_ld(D + 3), g.cu, prof_mul(prof_ld(D + 4), g.su)), prof_mul(g.dl, g.n));
+  q.wb = prof_ld(D + 2) * g.h;
+  q.wo = g.h;
+  q.w1 = prof_ld(D + 5) * g.dl;
+  return q;
+}
+
+// Position of bin u in the unit that starts at bin tfirst, from kUnitEnd up outside
+// it.  Rounded down once, in units that all units share (tfirst is a whole number
+// and the sum stays within one binade): a row is in exactly one unit, also where its
+// u is within rounding of the border of two.  u - tfirst from -kUnitBins up
+// to twice that (positions wrap beyond).
+PROF_FN unsigned row_pos(double u, double tfirst) {
+#ifdef __CUDACC__
+  constexpr double kMagicPos = 6442450944.0;  // 1.5 * 2^32: 20 fraction bits
+  return (unsigned)__double2loint(__dadd_rd(u, kMagicPos - tfirst));
+#else
+  return (unsigned)prof_floor((u - tfirst) * 1048576.0);
+#endif
+}
 
 }  // namespace wrtp
