@@ -62,7 +62,9 @@ template <bool VEC>
 __global__ void __launch_bounds__(32 * kWarps)
     ray_slices_kernel(wrt::RayJob job, int groups, int step, int pairs) {
   __shared__ float4 s_w[kWarps][32];
-  __shared__ int s_off[kWarps][32];
+  // columns, as a volume may have more than 2^31 nodes (their 64-bit offsets here: 228
+  // us at 128^3 instead of 223)
+  __shared__ int s_col[kWarps][32];
   __shared__ double s_g[kWarps][kSlots];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = job.n;
   const int ts = (job.nshift + kWarps - 1) / kWarps;
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(32 * kWarps)
       const double x = __dadd_rn(p0x, __dmul_rn(ax, (double)k));
       const double y = __dadd_rn(p0y, __dmul_rn(ay, (double)k));
       float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-      int off = 0;
+      int col = 0;
       if (k <= khi && fabs(x) <= 1.0 && fabs(y) <= 1.0) {
         int ix, iy;
         double cx, cy;
@@ -129,19 +131,19 @@ __global__ void __launch_bounds__(32 * kWarps)
         cell_of(y, n, &iy, &cy);
         w = make_float4((float)((1.0 - cx) * (1.0 - cy)), (float)((1.0 - cx) * cy),
                         (float)(cx * (1.0 - cy)), (float)(cx * cy));
-        off = (ix * n + iy) * n;
+        col = ix * n + iy;
         ++taken;
       }
       __syncwarp();
       s_w[warp][lane] = w;
-      s_off[warp][lane] = off;
+      s_col[warp][lane] = col;
       __syncwarp();
       float a[4] = {0.f, 0.f, 0.f, 0.f};
       const int m = min(32, khi - k0 + 1);
 #pragma unroll 4
       for (int j = 0; j < m; ++j) {
         const float4 c = s_w[warp][j];
-        const float *v = job.vol + s_off[warp][j];
+        const float *v = job.vol + (size_t)s_col[warp][j] * n;
         if (VEC) {
           const float *q = v + layer[0];
           const float4 f0 = __ldg(reinterpret_cast<const float4 *>(q));
