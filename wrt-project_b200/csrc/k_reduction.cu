@@ -11,10 +11,11 @@
 // spline is linear in its data), then (a, -ab(1+a)) and (b, -ab(1+b)) weigh the
 // (y, m) pairs of the two knots.
 //
-// Positions along a line advance in 32.32 fixed point (layers, knots): integer
+// Positions along a line advance in 16.48 fixed point (layers, knots): integer
 // part = layer or knot, fraction = 23 bits by a mantissa insert; no conversions
-// and no FP64 in the loop.  The error is below 200 steps x 2^-33 + 2^-24.  The
-// reference's layer index and knot interval are not reproduced at a layer or
+// and no FP64 in the loop.  The error is below (2 ngrid + 1) x 2^-49 + 2^-24
+// (reduction_dev.cuh; with 32.32 positions the steps' rounding passed 2^-24 from 256
+// layers up).  The reference's layer index and knot interval are not reproduced at a layer or
 // knot: the interpolant is continuous there (two zero layers and a zero knot
 // beyond the ends stand for slicing.c:62-74's zero third value).  Which samples
 // belong to a line (tau^2 + p^2 <= 1, slicing.c:110, |z|, |s| <= 1) is decided in
@@ -28,9 +29,12 @@
 #include <algorithm>
 #include <vector>
 
+#include "reduction_dev.cuh"
 #include "wrt_internal.cuh"
 
 namespace {
+
+using namespace wrtr;
 
 typedef unsigned long long u64;
 __device__ __forceinline__ u64 pk(float lo, float hi) {
@@ -53,11 +57,6 @@ __device__ __forceinline__ u64 lds64(unsigned a) {
   asm("ld.shared.b64 %0, [%1];" : "=l"(v) : "r"(a));
   return v;
 }
-// Upper 23 bits of a 32-bit fraction as a float in [0, 1).
-__device__ __forceinline__ float fraction(unsigned lo) {
-  return __uint_as_float(0x3f800000u | lo >> 9) - 1.0f;
-}
-
 // m_{i-1} + 4 m_i + m_{i+1} = y_{i+1} - 2 y_i + y_{i-1}, m_0 = m_{ns-1} = 0, one
 // thread per line (iz, iphi), element i at [(iz*ns + i)*nphi + iphi]: every access
 // of a warp is one row of consecutive phis.  d: forward pass, m: result.
@@ -98,15 +97,6 @@ struct RedJob {
   int ngrid, ns, nphi, nshift, ntheta, pitch;
 };
 
-// Whether sample k of a line belongs to it (slicing.c:105-110).
-__device__ __forceinline__ bool on_line(int k, double dtau, double p, double ct, double st) {
-  const double tau = __dmul_rn((double)k, dtau);
-  const double z = __dadd_rn(__dmul_rn(p, ct), __dmul_rn(tau, st));
-  const double s = __dsub_rn(__dmul_rn(p, st), __dmul_rn(tau, ct));
-  return !(fabs(__dadd_rn(__dmul_rn(tau, tau), __dmul_rn(p, p))) > 1.0) && !(fabs(z) > 1.0) &&
-         !(fabs(s) > 1.0);
-}
-
 template <int T>
 __global__ void __launch_bounds__(T, 1) reduction_staged_kernel(const RedJob job) {
   extern __shared__ __align__(16) float2 ym[];  // [ngrid + 2][pitch]
@@ -120,7 +110,6 @@ __global__ void __launch_bounds__(T, 1) reduction_staged_kernel(const RedJob job
   const unsigned base = (unsigned)__cvta_generic_to_shared(ym);
   const unsigned row = (unsigned)pitch * 8u;
   const double dtau = (2.0 / (ngrid - 1)) / (2.0);  // slicing.c:88
-  const double per_z = 0.5 * (ngrid - 1), per_s = 0.5 * (ns - 1);
   unsigned long long counted = 0;
   int staged = -1;
   for (long long item = i0; item < i1; ++item) {
@@ -142,33 +131,23 @@ __global__ void __launch_bounds__(T, 1) reduction_staged_kernel(const RedJob job
     const int line0 = (int)(item % per) * T + tid, line = min(line0, lines - 1);
     const int it = line / job.nshift, is = line - it * job.nshift;
     const double p = job.shift[is], ct = job.cs[2 * it], st = job.cs[2 * it + 1];
-    int khi = -1;
-    const double r = 1.0 - p * p;
-    if (r >= 0.0) khi = min(2 * ngrid, (int)floor(sqrt(r) / dtau) + 1);
-    int klo = -khi;
-    while (khi >= klo && !on_line(khi, dtau, p, ct, st)) --khi;
-    while (klo <= khi && !on_line(klo, dtau, p, ct, st)) ++klo;
+    int klo, khi;
+    line_range(ngrid, dtau, p, ct, st, &klo, &khi);
     // the warp's lanes keep the same tau: their cells then lie half a cell apart
     // along one short line, and neighbours share them
     const int k0 = __reduce_min_sync(0xffffffffu, klo), k1 = __reduce_max_sync(0xffffffffu, khi);
-    // 32.32 positions of sample k0, 2^-24 above the exact ones: the truncated
-    // fraction is then centred, and a position just below 0 does not leave the
-    // first cell
-    const double tau = (double)k0 * dtau;
-    long long zp = __double2ll_rn(((p * ct + tau * st + 1.0) * per_z + 0x1p-24) * 4294967296.0);
-    long long sp = __double2ll_rn(((p * st - tau * ct + 1.0) * per_s + 0x1p-24) * 4294967296.0);
-    const long long dz = __double2ll_rn(dtau * st * per_z * 4294967296.0);
-    const long long ds = __double2ll_rn(-dtau * ct * per_s * 4294967296.0);
+    LinePos at = line_pos(ngrid, ns, dtau, p, ct, st, k0);
     double acc = 0.0;
     for (int k = k0; k <= k1; k += 8) {
       float part = 0.0f;
 #pragma unroll 4
       for (int j = 0; j < 8; ++j) {
         const bool on = k + j >= klo && k + j <= khi;
-        const int iz = on ? (int)(zp >> 32) : 0, i = on ? (int)(sp >> 32) : 0;
-        const float f = fraction((unsigned)zp), b = fraction((unsigned)sp);
-        zp += dz;
-        sp += ds;
+        const int iz = on ? cell_of(at.z) : 0, i = on ? cell_of(at.s) : 0;
+        const float f = __uint_as_float(one_plus_fraction(at.z)) - 1.0f,
+                    b = __uint_as_float(one_plus_fraction(at.s)) - 1.0f;
+        at.z += at.dz;
+        at.s += at.ds;
         const unsigned a0 = base + (unsigned)iz * row + (unsigned)i * 8u;
         const unsigned a1 = a0 + row, a2 = a1 + row;
         const u64 l00 = lds64(a0), l01 = lds64(a0 + 8), l10 = lds64(a1), l11 = lds64(a1 + 8),
