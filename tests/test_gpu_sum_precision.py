@@ -23,3 +23,18 @@ def test_reduction(ctx, ngrid, nsr, nphi, nshift, ntheta, bound):
     err = rel_l2(got, O.reduction_forward(rays, nshift, ntheta))
     print(f"reduction {err:.2e}")
     assert err < bound
+
+
+def test_backprojection(ctx):
+    n, nphi, ntheta, nshift = 32, 128, 64, 256
+    r = np.random.default_rng(4)
+    s = np.linspace(-1.0, 1.0, nshift)[:, None, None]
+    radon = np.clip(1.0 - ((s - r.uniform(-0.3, 0.3, (1, nphi, ntheta))) / 0.7) ** 2, 0.0, None)
+    radon = np.ascontiguousarray(radon + 0.05 * r.standard_normal((nshift, nphi, ntheta)))
+    got = ctx.radon3d_adjoint(radon, n)
+    x = -1.0 + (2.0 * np.arange(n) + 1.0) / n
+    pick = r.integers(0, n, (4000, 3))
+    ref = O.adjoint_points(radon, x[pick[:, 1]], x[pick[:, 2]], x[pick[:, 0]])
+    err = rel_l2(got[pick[:, 0], pick[:, 1], pick[:, 2]], ref)
+    print(f"backprojection {err:.2e}")
+    assert err < 6.4e-9

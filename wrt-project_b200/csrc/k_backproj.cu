@@ -23,8 +23,8 @@
 //           range's start from the lines directly, then one knot after another,
 //           each piece's coefficients at its own start rounded once to FP32
 //   gather: threads on voxels of one z, the list's positions in shared memory,
-//           one 16-byte record per (voxel, longitude); FP32 over 2 longitudes,
-//           FP64 beyond, every voxel in a fixed order by one thread
+//           one 16-byte record per (voxel, longitude); FP64 sums, every voxel
+//           in a fixed order by one thread
 //
 // A voxel within 2 positions (1.3e-9 in t) of the end of a line, where S jumps to
 // zero, is decided by the FP64 position of the direction itself, as in the
@@ -34,8 +34,8 @@
 // What bounds it: the gather's L1 tag lookups (32 lanes, 32 lines, 32 cycles per
 // request: 0.5 ms of the 128^3 case if every SM were busy), the build's latency.
 // 128^3 from 64 x 128 directions x 256 shifts: 15.9 ms by the direct kernel (16
-// bytes and ~7 instructions per voxel and direction), 1.87 here; 256^3 from 96 x
-// 192 x 384: 237 and 20 ms; error against FP64 5.4e-8 both.
+// bytes and ~7 instructions per voxel and direction), 1.77 here; 256^3 from 96 x
+// 192 x 384: 237 and 20 ms; error against FP64 (128^3) 6.5e-9 and 4.8e-9.
 #include <math.h>
 
 #include <algorithm>
@@ -400,9 +400,6 @@ __global__ void __launch_bounds__(kGatherThreads, 2) back_gather_kernel(const Ba
       y[u] = z_of(n, v % n);
       tot[u] = 0.0;
     }
-    float acc[kVox];
-#pragma unroll
-    for (int u = 0; u < kVox; ++u) acc[u] = 0.0f;
     for (int b = 0; b < B; ++b) {
       const double2 cs = dir[b];
       unsigned fx[kVox], nx[kVox], dt[kVox];
@@ -449,7 +446,9 @@ __global__ void __launch_bounds__(kGatherThreads, 2) back_gather_kernel(const Ba
 #pragma unroll
       for (int u = 0; u < kVox; ++u) {
         const float d = (float)dt[u];
-        acc[u] += fmaf(d, fmaf(d, fmaf(d, c[u].w, c[u].z), c[u].y), c[u].x);
+        // FP64 at once: two longitudes in FP32 first were 7.5e-9 from FP64 at 128^3 (the
+        // direct kernel 6.5e-9, this 4.8e-9) and 1.85 ms instead of 1.77
+        tot[u] += (double)fmaf(d, fmaf(d, fmaf(d, c[u].w, c[u].z), c[u].y), c[u].x);
       }
       if (edge) {
 #pragma unroll
@@ -458,14 +457,6 @@ __global__ void __launch_bounds__(kGatherThreads, 2) back_gather_kernel(const Ba
             const int v = min(v0 + u * kGatherThreads + tid, n2 - 1);
             tot[u] += edge_terms(s, zi, pos, e[u], fx[u], v / n, v % n, b);
           }
-      }
-      // FP32 over two longitudes (over eight, the error against FP64 was a fifth larger)
-      if ((b & 1) | (b + 1 == B)) {
-#pragma unroll
-        for (int u = 0; u < kVox; ++u) {
-          tot[u] += (double)acc[u];
-          acc[u] = 0.0f;
-        }
       }
     }
 #pragma unroll
