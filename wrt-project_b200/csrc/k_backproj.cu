@@ -498,6 +498,10 @@ Plan plan_of(int nphi, int ntheta, int ns) {
 size_t gather_smem(const Plan &p) {
   return 16 * (size_t)p.nbase + 4 * (size_t)(p.cap + 16) + 2 * ((size_t)1 << p.nb_log2);
 }
+size_t build_smem(int ntheta) {
+  return kRecTile * sizeof(KnotRec) + sizeof(StartLat) * (size_t)ntheta;
+}
+constexpr size_t kMostSmem = 220 * 1024;
 
 }  // namespace
 
@@ -505,14 +509,14 @@ namespace wrt {
 
 bool backproj_covers(int nphi, int ntheta, int ns, int n) {
   const long long knots = (long long)ntheta * ns;
-  // the list's positions fit shared memory; larger than the allocation-free
+  // the list's positions and the latitudes fit shared memory; larger than the allocation-free
   // path takes, whose volume is the direct kernel's bit for bit.  Measured beyond
   // that (n 16 .. 256, 41 .. 96 latitudes): never slower than the direct kernel,
   // which takes at least 0.43 us per direction, e.g. 33^3 from 64 x 128 x 256 in
   // 3.6 ms against 0.7 here
   if (knots > 50000 || ns < 3 || n > 2048 || (long long)nphi * knots <= 262144) return false;
   if ((long long)nphi * knots > (1LL << 30)) return false;
-  return gather_smem(plan_of(nphi, ntheta, ns)) <= 220 * 1024;
+  return gather_smem(plan_of(nphi, ntheta, ns)) <= kMostSmem && build_smem(ntheta) <= kMostSmem;
 }
 
 // Working memory: the lines' Y, M and D, the sorted lists of every z plane, and
@@ -541,7 +545,7 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
   const int nz = (int)std::max<size_t>(1, std::min<size_t>(r.n, left / p.table));
   const int nl = nz >= kProfLanes && r.n >= 2 * kProfLanes ? kProfLanes : 1;
   const size_t sm_sort = 4 * ((size_t)1 << p.nb_log2);
-  const size_t sm_build = kRecTile * sizeof(KnotRec) + sizeof(StartLat) * (size_t)r.ntheta;
+  const size_t sm_build = build_smem(r.ntheta);
   const size_t sm_gather = gather_smem(p);
   if (e == cudaSuccess && sm_sort > 48 * 1024)
     e = cudaFuncSetAttribute(back_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
