@@ -1,12 +1,13 @@
-"""Sums of the staged reduction (and of the merged backprojection) against the FP64
-oracle: no further from it than the kernels that took every sample and direction on
+"""Sums of the staged reduction, of the merged backprojection and of the plane
+transforms against the FP64 oracle: no further from it than the kernels that took every sample and direction on
 its own, whose errors on this data are the bounds (FP64 sums of FP32 samples; adding
 up to eight samples in FP32 first was 1.2 to 1.5 times as far off)."""
 import numpy as np
 import pytest
 
 import oracle as O
-from conftest import rel_l2
+from conftest import rel_l2, wrt  # noqa: F401 (loads the package)
+from wrt_b200.phantom import ellipsoid_phantom
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,14 @@ def test_backprojection(ctx):
     err = rel_l2(got[pick[:, 0], pick[:, 1], pick[:, 2]], ref)
     print(f"backprojection {err:.2e}")
     assert err < 6.4e-9
+
+
+@pytest.mark.parametrize("sampler,n,grid,bound", [
+    (O.NEAREST, 24, (16, 8, 32), 1.86e-8), (O.TRILINEAR, 16, (16, 12, 40), 3.96e-8),
+    (O.TRILINEAR, 64, (32, 16, 64), 1.2e-8)])
+def test_planes(ctx, sampler, n, grid, bound):
+    vol = ellipsoid_phantom(n, 12, 0, dtype=np.float32).astype(np.float64)
+    got = ctx.radon_grid(vol, *grid, sampler=sampler, half_extent=n)
+    err = rel_l2(got, O.radon_forward(vol, *grid, sampler=sampler, half_extent=n))
+    print(f"planes {n} {err:.2e}")
+    assert err < bound

@@ -207,14 +207,17 @@ __device__ __forceinline__ Quad start_sum(const Geo &g, const StartLine *lines, 
   Quad q = {0.0, 0.0, 0.0};
   const float cu = (float)g.cu, su = (float)g.su, cusu = (float)(g.cu * g.su);
   const int sx = g.n * g.n, sy = g.n;
-  // FP32 over eight lines, FP64 beyond (lines[] is padded with empty ones)
+  // slopes in FP32 over eight lines, FP64 beyond (lines[] is padded with empty ones);
+  // values in FP64 at once: where many of them are equal, FP32 sums of eight are all off
+  // the same way, and with them every row of the range (24^3 nearest 2.1e-8 from FP64
+  // instead of 1.3e-8, 96^3 trilinear 1.6e-8 instead of 8e-9; less than 1 % of the time)
   for (int j0 = 0; j0 < nl; j0 += 8) {
-    float v = 0.0f, sl = 0.0f, cc = 0.0f;
+    float sl = 0.0f, cc = 0.0f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const StartLine l = lines[j0 + j];
       if (NEAR) {
-        v = fmaf(l.w, ld_node(vol, l.off), v);
+        q.a0 += (double)(l.w * ld_node(vol, l.off));
         continue;
       }
       const float x = l.tx, y = l.ty;
@@ -222,11 +225,10 @@ __device__ __forceinline__ Quad start_sum(const Geo &g, const StartLine *lines, 
                   f10 = ld_node(vol, l.off + sx), f11 = ld_node(vol, l.off + sx + sy);
       const float dx0 = f10 - f00, dx1 = f11 - f01, dy = f01 - f00, dxy = dx1 - dx0;
       const float fx = fmaf(y, dxy, dx0), fy = fmaf(x, dxy, dy);
-      v = fmaf(l.w, fmaf(x, fx, fmaf(y, dy, f00)), v);
+      q.a0 += (double)(l.w * fmaf(x, fx, fmaf(y, dy, f00)));
       sl = fmaf(l.w, fmaf(cu, fx, su * fy), sl);
       cc = fmaf(l.w, dxy, cc);
     }
-    q.a0 += (double)v;
     if (!NEAR) {
       q.a1 += (double)sl;
       q.a2 += (double)(cusu * cc);
@@ -1370,6 +1372,11 @@ bool profile_covers(int n, int nphi, int ntheta, int nshift) {
 bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift) {
   if (!profile_covers(n, nphi, ntheta, nshift)) return false;
   if (ctx->staged_config >= 0) return ctx->staged_config == kNumStagedConfigs - 1;
+  // A position is rounded to 2^-20 bins, n bins a cell, and a small volume's rows have
+  // few samples: below 20 the error against FP64 passes the staged kernel's (phantoms,
+  // trilinear, means of 4 to 8: 12^3 5.5e-8 and 3.9e-8, 16^3 3.6 and 3.7, 20^3 2.8 and 3.1,
+  // 24^3 2.3 and 3.1; 32 volumes of 16^3 .. 48^3 1.34 ms, 1.28 with those below 20 too).
+  if (n < 20) return false;
   const double rows = (double)ntheta * nshift;
   if (rows * nphi < 4000) return false;
   const bool paired = nphi % 2 == 0;
