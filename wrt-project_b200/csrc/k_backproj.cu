@@ -547,15 +547,9 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
   const size_t sm_sort = 4 * ((size_t)1 << p.nb_log2);
   const size_t sm_build = build_smem(r.ntheta);
   const size_t sm_gather = gather_smem(p);
-  if (e == cudaSuccess && sm_sort > 48 * 1024)
-    e = cudaFuncSetAttribute(back_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sm_sort);
-  if (e == cudaSuccess && sm_build > 48 * 1024)
-    e = cudaFuncSetAttribute(back_build_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sm_build);
-  if (e == cudaSuccess && sm_gather > 48 * 1024)
-    e = cudaFuncSetAttribute(back_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sm_gather);
+  if (e == cudaSuccess && sm_sort > 48 * 1024) e = allow_smem(back_sort_kernel, kMostSmem);
+  if (e == cudaSuccess && sm_build > 48 * 1024) e = allow_smem(back_build_kernel, kMostSmem);
+  if (e == cudaSuccess && sm_gather > 48 * 1024) e = allow_smem(back_gather_kernel, kMostSmem);
   // ---- the lists of all z planes
   BackStep s0 = {};
   s0.r = r;

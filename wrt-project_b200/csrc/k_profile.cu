@@ -1313,6 +1313,9 @@ void chunk_range(const ProfReq &r, float crop, int *c0, int *c1) {
   *c1 = (int)std::floor((toff + tmax) * r.n / kUnitBins) + 1;
 }
 
+// Dynamic shared memory of the build and the rows at the largest edge (70 KB each).
+constexpr size_t kMostSmem = 96 * 1024;
+
 template <bool NEAR, int S>
 cudaError_t launch_step(wrt_ctx *ctx, cudaStream_t stream, const std::vector<ProfSeg> &segs,
                         unsigned long long *list) {
@@ -1335,12 +1338,9 @@ cudaError_t launch_step(wrt_ctx *ctx, cudaStream_t stream, const std::vector<Pro
   const size_t sm_rows = 4 * (size_t)(cap + 16) + 2 * (size_t)(kUnitBins + 8);
   cudaError_t e = cudaSuccess;
   // beyond 48 KB of dynamic shared memory a kernel has to be told
-  if (sm_build > 48 * 1024)
-    e = cudaFuncSetAttribute(profile_build_kernel<NEAR, S>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_build);
+  if (sm_build > 48 * 1024) e = wrt::allow_smem(profile_build_kernel<NEAR, S>, kMostSmem);
   if (e == cudaSuccess && sm_rows > 48 * 1024)
-    e = cudaFuncSetAttribute(profile_rows_kernel<NEAR, S>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_rows);
+    e = wrt::allow_smem(profile_rows_kernel<NEAR, S>, kMostSmem);
   if (e != cudaSuccess) return e;
   profile_sort_kernel<S><<<(unsigned)sort, kSortThreads, kUnitBins * 8, stream>>>(st);
   profile_build_kernel<NEAR, S><<<(unsigned)build, th_build, sm_build, stream>>>(st);

@@ -216,10 +216,8 @@ int reduction_staged(wrt_ctx *ctx, cudaStream_t stream, const double *rays, int 
   const unsigned grid = (unsigned)std::min<long long>(items, (long long)ctx->sm_count * per_sm);
   cudaError_t e = cudaSuccess;
   if (smem > 48 * 1024)
-    e = big ? cudaFuncSetAttribute(reduction_staged_kernel<1024>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-            : cudaFuncSetAttribute(reduction_staged_kernel<512>,
-                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = big ? allow_smem(reduction_staged_kernel<1024>, kMostSmem)
+            : allow_smem(reduction_staged_kernel<512>, kMostSmem);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "reduction kernel attribute");
   if (big)
     reduction_staged_kernel<1024><<<grid, 1024, smem, stream>>>(j);

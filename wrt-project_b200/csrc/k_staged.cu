@@ -764,7 +764,8 @@ int launch_cfg(wrt_ctx *ctx, cudaStream_t stream, const StagedReq *d_reqs,
   auto kern = count ? plane_staged_kernel<T, G, K, true, NEAR>
                     : plane_staged_kernel<T, G, K, false, NEAR>;
   max_smem += (T / 32) * wrt::kStagedWarpSmemQuads * 16;  // per-warp row tables and queues
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem);
+  cudaError_t e = wrt::allow_smem(
+      kern, wrt::kStagedSmemMax + (T / 32) * wrt::kStagedWarpSmemQuads * 16);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "staged kernel smem attribute");
   e = cudaMemsetAsync(d_next, 0, sizeof(int), stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "staged counter reset");

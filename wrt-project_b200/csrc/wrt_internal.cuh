@@ -93,6 +93,14 @@ int cuda_fail(wrt_ctx *ctx, cudaError_t e, const char *what);
 int ctx_alloc(wrt_ctx *ctx, void **p, size_t bytes);
 void ctx_free(wrt_ctx *ctx, void *p, size_t bytes);
 int check_launch(wrt_ctx *ctx, const char *what);
+// Lets a kernel be launched with up to `most` bytes of dynamic shared memory.  The limit
+// belongs to the kernel, not to a call or a context: two threads that set what their own
+// launches need can lower it under one another, so each kernel has one constant that
+// all its callers set.
+template <typename K>
+inline cudaError_t allow_smem(K kernel, size_t most) {
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
 // Working buffer of a role, at least `bytes` long (grown after the context's
 // stream has drained; contents are not kept).
 enum WsRole { WS_STAGE, WS_IN, WS_OUT, WS_LINES, WS_SPLINE, WS_COEF, WS_TABLE, WS_FFT, WS_PROFILE,
