@@ -150,6 +150,8 @@ void spline_coefficients(int ns, double *cp, double *den) {
   }
 }
 
+static size_t ws_rounded(size_t bytes) { return (bytes + 0xffff) & ~(size_t)0xffff; }
+
 int ws_get(wrt_ctx *ctx, int role, size_t bytes, void **p) {
   if (role < 0 || role >= WS_ROLES) return fail(ctx, WRT_ERR_INTERNAL, "workspace role %d", role);
   if (bytes <= ctx->ws_bytes[role] && ctx->ws[role]) {
@@ -162,7 +164,7 @@ int ws_get(wrt_ctx *ctx, int role, size_t bytes, void **p) {
     ctx->ws[role] = nullptr;
     ctx->ws_bytes[role] = 0;
   }
-  const size_t want = (bytes + (1 << 16) - 1) & ~(size_t)((1 << 16) - 1);
+  const size_t want = ws_rounded(bytes);
   int st = ctx_alloc(ctx, &ctx->ws[role], want);
   if (st) return st;
   ctx->ws_bytes[role] = want;
@@ -747,19 +749,25 @@ struct TablesHeld {
   ~TablesHeld() { ctx->tables_held = false; }
 };
 
-// The profiles' working memory of these requests in the context's workspace:
-// what they ask for, or as much of it as the context's budget and the device hold,
-// halving down to the least that serves them; an error (cleared) below that.
-int profile_ws(wrt_ctx *ctx, const ProfReq *reqs, const float *crop, int nreq, void **ws,
-               size_t *bytes) {
-  size_t want = profile_workspace_want(reqs, crop, nreq), least = 0;
-  for (int q = 0; q < nreq; ++q)
-    least = std::max(least, profile_workspace_least(reqs[q], crop[q]));
-  auto half = [&] { return std::max(want / 2 & ~(size_t)255, least); };
-  while (want > least && want >= ctx->tables_refused) want = half();
+// Working memory that only makes a call faster, in the context's workspace: `want`
+// bytes, or as much of it as the context's budget and the device hold now, halving down
+// to the least that serves; an error (cleared) below that.  What a budget leaves is known
+// exactly; of the device it is asked only after it has refused or taken back as much.
+int tables_get(wrt_ctx *ctx, size_t want, size_t least, void **ws, size_t *bytes) {
+  const size_t have = ctx->ws_bytes[WS_PROFILE], others = ctx->in_use - have;
+  size_t room = ~(size_t)0;
+  if (ctx->budget) room = ctx->budget > others ? ctx->budget - others : 0;
+  if (want > have && want >= ctx->tables_refused) {
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) cudaGetLastError();
+    if (free_b + have >= want) ctx->tables_refused = ~(size_t)0;  // there again
+    else room = std::min(room, free_b + have);
+  }
+  auto half = [&] { return std::max(want / 2 & ~(size_t)0xffff, least); };
+  while (want > least && want > have && ws_rounded(want) > room) want = half();
   int st = ws_get(ctx, WS_PROFILE, want, ws);
   while (st && want > least) {
-    ctx->tables_refused = want;
+    ctx->tables_refused = std::min(ctx->tables_refused, want);
     want = half();
     st = ws_get(ctx, WS_PROFILE, want, ws);
   }
@@ -769,6 +777,14 @@ int profile_ws(wrt_ctx *ctx, const ProfReq *reqs, const float *crop, int nreq, v
   }
   *bytes = std::min(want, ctx->ws_bytes[WS_PROFILE]);
   return WRT_OK;
+}
+
+int profile_ws(wrt_ctx *ctx, const ProfReq *reqs, const float *crop, int nreq, void **ws,
+               size_t *bytes) {
+  size_t least = 0;
+  for (int q = 0; q < nreq; ++q)
+    least = std::max(least, profile_workspace_least(reqs[q], crop[q]));
+  return tables_get(ctx, profile_workspace_want(reqs, crop, nreq), least, ws, bytes);
 }
 
 int radon_forward_profile(wrt_ctx *ctx, wrt_volume *vol, const wrt_grid *grid, int L,
@@ -1198,14 +1214,11 @@ int wrt_radon3d_adjoint_device(wrt_ctx *ctx, const double *dev_radon, const wrt_
   int st = set_device(ctx);
   if (st) return st;
   if (backproj_covers(grid->nphi, grid->ntheta, grid->nshift, ngrid)) {
-    const size_t want = backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, false);
     void *ws = nullptr, *cp = nullptr;
-    st = want < ctx->tables_refused ? ws_get(ctx, WS_PROFILE, want, &ws) : WRT_ERR_BUDGET;
-    if (st) {
-      ctx->tables_refused = std::min(ctx->tables_refused, want);
-      st = ws_get(ctx, WS_PROFILE,
-                  backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, true), &ws);
-    }
+    size_t bytes = 0;
+    st = tables_get(ctx, backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, false),
+                    backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, true), &ws,
+                    &bytes);
     const TablesHeld held(ctx);
     if (!st) st = ws_get(ctx, WS_COEF, sizeof(double) * 2 * grid->nshift, &cp);
     if (!st) {
@@ -1225,8 +1238,7 @@ int wrt_radon3d_adjoint_device(wrt_ctx *ctx, const double *dev_radon, const wrt_
       r.ntheta = grid->ntheta;
       r.ns = grid->nshift;
       r.n = ngrid;
-      return backproj_forward(ctx, ctx->stream, &ctx->prof_lanes, r, ws,
-                              std::min(want, ctx->ws_bytes[WS_PROFILE]));
+      return backproj_forward(ctx, ctx->stream, &ctx->prof_lanes, r, ws, bytes);
     }
     ctx->err[0] = 0;  // no room for the tables: the direct kernel
   }

@@ -519,11 +519,31 @@ bool backproj_covers(int nphi, int ntheta, int ns, int n) {
   return gather_smem(plan_of(nphi, ntheta, ns)) <= kMostSmem && build_smem(ntheta) <= kMostSmem;
 }
 
+// Streams of a backprojection with nz z planes in flight, planes on each.
+static int lanes_of(int n, int nz) { return nz >= kProfLanes && n >= 2 * kProfLanes ? kProfLanes : 1; }
+
+// The fewest planes in flight that are not slower than the direct kernel.  With few of
+// them a round is one long chain, up to 3.2 us a longitude tabulated; the direct kernel
+// takes 0.43 us a direction, or 0.93 ps a direction and voxel.  Planes in flight, merged
+// and direct: 128^3 from 64 x 128 x 256 1: 26.7 ms, 7: 7.2, 20: 2.0, direct 15.9; 64^3 from
+// 33 x 65 x 129 4: 2.5 ms, 13: 1.01, 30: 0.57, direct 0.94; 40^3 from 50 x 100 x 220 2: 2.9,
+// 7: 1.5, 18: 0.57, direct 2.2.
+static int least_planes(int nphi, int ntheta, int n, int nbase) {
+  const double voxels = (double)n * n * n;
+  const double direct = (double)nphi * ntheta * std::max(0.43, 0.93e-6 * voxels);
+  for (int nz = 1; nz < n; ++nz) {
+    const int nl = lanes_of(n, nz), in_flight = std::max(1, nz / nl) * nl;
+    if ((n + in_flight - 1) / in_flight * 3.2 * nbase <= 0.9 * direct) return nz;
+  }
+  return n;
+}
+
 // Working memory: the lines' Y, M and D, the sorted lists of every z plane, and
 // the tables of the planes in flight.
 size_t backproj_workspace(int nphi, int ntheta, int ns, int n, bool least) {
   const Plan p = plan_of(nphi, ntheta, ns);
-  const size_t z = least ? 1 : std::min<size_t>(n, std::max<size_t>(1, kBackTableBytes / p.table));
+  const size_t most = std::min<size_t>(n, std::max<size_t>(1, kBackTableBytes / p.table));
+  const size_t z = least ? std::min<size_t>(most, least_planes(nphi, ntheta, n, p.nbase)) : most;
   return 3 * p.data + n * p.list() + z * p.table + 4096;
 }
 
@@ -543,7 +563,7 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
   at += (size_t)r.n * p.list();
   const size_t left = ws_bytes - (at - static_cast<char *>(ws));
   const int nz = (int)std::max<size_t>(1, std::min<size_t>(r.n, left / p.table));
-  const int nl = nz >= kProfLanes && r.n >= 2 * kProfLanes ? kProfLanes : 1;
+  const int nl = lanes_of(r.n, nz);
   const size_t sm_sort = 4 * ((size_t)1 << p.nb_log2);
   const size_t sm_build = build_smem(r.ntheta);
   const size_t sm_gather = gather_smem(p);

@@ -71,7 +71,8 @@ struct wrt_ctx {
   size_t ws_bytes[10] = {};
   wrt::ProfLanes prof_lanes;  // side streams of the plane transform's profiles
   bool tables_held = false;   // a running call works in ws[WS_PROFILE]
-  size_t tables_refused = ~(size_t)0;  // a size that WS_PROFILE could not have or had to give up
+  size_t tables_refused = ~(size_t)0;  // a size that WS_PROFILE could not have or had to give
+                                       // up: asked for again once the device has as much free
   void *fft_plans = nullptr;  // spectral Laplacian plans (k_laplace.cu)
   // the volume and sphere grid of the last drop-in (host-array) call, kept
   // for the next call of the same sizes
@@ -330,7 +331,7 @@ struct BackStep {        // a group of z planes
   int z0, cap, nb, nb_log2, nsub_log2, tiles;
 };
 // Whether a backprojection goes there (by sizes alone), its working memory (for
-// one z plane at a time, or what fills the device), and the launches.
+// the fewest z planes at a time that pay, or what fills the device), and the launches.
 bool backproj_covers(int nphi, int ntheta, int ns, int n);
 size_t backproj_workspace(int nphi, int ntheta, int ns, int n, bool least);
 int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackReq r, void *ws,
