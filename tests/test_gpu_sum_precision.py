@@ -42,7 +42,7 @@ def test_backprojection(ctx):
 
 
 @pytest.mark.parametrize("sampler,n,grid,bound", [
-    (O.NEAREST, 24, (16, 8, 32), 1.86e-8), (O.TRILINEAR, 16, (16, 12, 40), 3.96e-8),
+    (O.NEAREST, 24, (16, 8, 32), 1.86e-8), (O.TRILINEAR, 12, (16, 12, 40), 4.3e-8),
     (O.TRILINEAR, 64, (32, 16, 64), 1.2e-8)])
 def test_planes(ctx, sampler, n, grid, bound):
     vol = ellipsoid_phantom(n, 12, 0, dtype=np.float32).astype(np.float64)

@@ -1373,10 +1373,10 @@ bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift) 
   if (!profile_covers(n, nphi, ntheta, nshift)) return false;
   if (ctx->staged_config >= 0) return ctx->staged_config == kNumStagedConfigs - 1;
   // A position is rounded to 2^-20 bins, n bins a cell, and a small volume's rows have
-  // few samples: below 20 the error against FP64 passes the staged kernel's (phantoms,
-  // trilinear, means of 4 to 8: 12^3 5.5e-8 and 3.9e-8, 16^3 3.6 and 3.7, 20^3 2.8 and 3.1,
-  // 24^3 2.3 and 3.1; 32 volumes of 16^3 .. 48^3 1.34 ms, 1.28 with those below 20 too).
-  if (n < 20) return false;
+  // few samples: below 15 the error against FP64 passes the staged kernel's (24 phantoms
+  // and grids each, trilinear, means: 8^3 1.0e-7 here and 4.5e-8 there, 12^3 5.4 and 4.5,
+  // 14^3 4.3 and 4.3, 15^3 3.8 and 4.2, 16^3 3.7 and 3.9, 20^3 2.8 and 3.8).
+  if (n < 15) return false;
   const double rows = (double)ntheta * nshift;
   if (rows * nphi < 4000) return false;
   const bool paired = nphi % 2 == 0;
