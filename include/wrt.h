@@ -299,7 +299,9 @@ typedef struct wrt_forward_req {
  * request table; requests that suit the row-sum profiles share the launches of
  * those instead.  Asynchronous on the context's stream.  Each result is
  * bitwise identical to what wrt_radon_forward_device gives for the same
- * request alone.  Batch transforms of the reference's loop nest
+ * request alone (in a context whose budget or device has the least working
+ * memory of its row-sum profiles at both times, or at neither: the kernel is
+ * chosen request by request).  Batch transforms of the reference's loop nest
  * radon_grid/src/radon_grid.c:229-264, one per request. */
 int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq);
 

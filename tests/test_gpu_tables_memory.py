@@ -50,3 +50,22 @@ def test_tables_come_back(op, left):
         assert np.array_equal(first, out.download(np.empty(out.nbytes // 8)))
     assert rel_l2(first, ref.ravel()) < 1e-5
     assert rel_l2(tight, ref.ravel()) < 1e-5
+
+
+def test_batch_equals_alone_in_a_tight_budget():
+    # the large requests' tables do not fit, the small ones' do, whatever else is in the batch
+    sizes = [(64, (32, 16, 64)), (24, (16, 8, 40)), (16, (8, 4, 9)), (72, (30, 15, 70)), (30, (16, 8, 50))]
+    with wrt.Context(0, budget_bytes=28 << 20) as c:
+        reqs, keep = [], []
+        for n, grid in sizes:
+            v = wrt.Volume(c, n)
+            v.upload(np.random.default_rng(n).standard_normal((n, n, n)).astype(np.float32))
+            g = wrt.Grid(c, *grid)
+            out = wrt.DeviceBuffer(c, g.nplanes * 8)
+            keep.append((v, g, out))
+            reqs.append((v, g, out.ptr, n))
+        wrt.radon_forward_batch(c, reqs)
+        batched = [out.download(np.empty(g.nplanes)) for _, g, out in keep]
+        for (n, _), (v, g, out), got in zip(sizes, keep, batched):
+            wrt.radon_forward_device(c, v, g, out.ptr, half_extent=n)
+            assert np.array_equal(got, out.download(np.empty(g.nplanes))), n

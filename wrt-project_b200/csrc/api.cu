@@ -867,7 +867,8 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
   // requests for the row-sum profiles, FP32 and BF16 volumes together
   std::vector<ProfReq> prof;
   std::vector<float> prof_crop;
-  std::vector<char> routed(nreq, 0);
+  std::vector<int> routed;  // their places in reqs
+  std::vector<char> staged(nreq, 1);
   for (int r = 0; r < nreq; ++r) {
     const wrt_volume *vol = reqs[r].volume;
     const wrt_grid *grid = reqs[r].grid;
@@ -878,7 +879,8 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
       continue;  // refused below
     const int L = reqs[r].half_extent ? reqs[r].half_extent : 2 * vol->n;
     if (!profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift)) continue;
-    routed[r] = 1;
+    staged[r] = 0;
+    routed.push_back(r);
     prof.push_back(profile_request(ctx, vol, grid, L, false, reqs[r].dev_out));
     prof_crop.push_back(trilinear_crop_r2(vol->r2, vol->n));
   }
@@ -915,17 +917,46 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
     return WRT_OK;
   };
   for (int r = 0; r < nreq && !st; ++r)
-    if (!routed[r]) st = add_staged(r);
+    if (staged[r]) st = add_staged(r);
   if (st) return st;
-  // the tables after all that has to be there
+  auto slot_ready = [&]() -> int {
+    if (b.fwd.empty()) return WRT_OK;
+    if (!ctx->batch_slot) {
+      BatchSlot *s = new (std::nothrow) BatchSlot();
+      if (!s) return WRT_ERR_OUT_OF_MEMORY;
+      const int is = batch_slot_init(ctx, s, ctx->stream);
+      if (is) {
+        batch_slot_release(s);
+        delete s;
+        return is;
+      }
+      ctx->batch_slot = s;
+    }
+    return batch_slot_reserve(static_cast<BatchSlot *>(ctx->batch_slot), b);
+  };
+  // the tables after all that has to be there; a request that they have no room for
+  // (the one that needs most, as it would not have alone) takes the staged kernel
   void *prof_ws = nullptr;
   size_t prof_bytes = 0;
-  if (!prof.empty() && profile_ws(ctx, prof.data(), prof_crop.data(), (int)prof.size(), &prof_ws,
-                                  &prof_bytes)) {
-    prof.clear();
-    for (int r = 0; r < nreq && !st; ++r)
-      if (routed[r]) st = add_staged(r);
+  for (;;) {
+    st = slot_ready();
     if (st) return st;
+    if (prof.empty() || !profile_ws(ctx, prof.data(), prof_crop.data(), (int)prof.size(), &prof_ws,
+                                    &prof_bytes))
+      break;
+    size_t k = 0, most = 0;
+    for (size_t q = 0; q < prof.size(); ++q) {
+      const size_t least = profile_workspace_least(prof[q], prof_crop[q]);
+      if (least > most) {
+        most = least;
+        k = q;
+      }
+    }
+    st = add_staged(routed[k]);
+    if (st) return st;
+    prof.erase(prof.begin() + k);
+    prof_crop.erase(prof_crop.begin() + k);
+    routed.erase(routed.begin() + k);
   }
   const TablesHeld held(ctx);
   auto profiles = [&](ProfFork fork) {
@@ -935,17 +966,6 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
                                           fork);
   };
   if (b.fwd.empty()) return profiles(PROF_ALONE);
-  if (!ctx->batch_slot) {
-    BatchSlot *s = new (std::nothrow) BatchSlot();
-    if (!s) return WRT_ERR_OUT_OF_MEMORY;
-    st = batch_slot_init(ctx, s, ctx->stream);
-    if (st) {
-      batch_slot_release(s);
-      delete s;
-      return st;
-    }
-    ctx->batch_slot = s;
-  }
   if (!prof.empty()) {
     // beside the staged kernel, and before it: its blocks hold their SM until
     // the item list is empty, so they take what the profiles leave free
@@ -1216,11 +1236,12 @@ int wrt_radon3d_adjoint_device(wrt_ctx *ctx, const double *dev_radon, const wrt_
   if (backproj_covers(grid->nphi, grid->ntheta, grid->nshift, ngrid)) {
     void *ws = nullptr, *cp = nullptr;
     size_t bytes = 0;
-    st = tables_get(ctx, backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, false),
+    st = ws_get(ctx, WS_COEF, sizeof(double) * 2 * grid->nshift, &cp);
+    if (!st)
+      st = tables_get(ctx, backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, false),
                     backproj_workspace(grid->nphi, grid->ntheta, grid->nshift, ngrid, true), &ws,
                     &bytes);
     const TablesHeld held(ctx);
-    if (!st) st = ws_get(ctx, WS_COEF, sizeof(double) * 2 * grid->nshift, &cp);
     if (!st) {
       std::vector<double> coef(2 * (size_t)grid->nshift);
       spline_coefficients(grid->nshift, coef.data(), coef.data() + grid->nshift);

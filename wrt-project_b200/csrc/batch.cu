@@ -383,6 +383,10 @@ int capture(BatchSlot *s) {
 
 }  // namespace
 
+int batch_slot_reserve(BatchSlot *s, const BatchBuilder &b) {
+  return ensure_capacity(s, BatchLayout::bytes(b.items.size()));
+}
+
 int batch_slot_launch(BatchSlot *s, BatchBuilder &b) {
   wrt_ctx *ctx = s->ctx;
   if ((int)b.fwd.size() > kBatchMaxFwd || (int)b.adj.size() > kBatchMaxAdj ||

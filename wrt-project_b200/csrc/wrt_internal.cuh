@@ -453,6 +453,8 @@ void batch_add_forward(BatchBuilder &b, const StagedReq &req, const FwdAux &aux,
 int batch_slot_init(wrt_ctx *ctx, BatchSlot *slot, cudaStream_t stream);
 // Waits for the slot's previous launch, writes the table, launches the graph.
 int batch_slot_launch(BatchSlot *slot, BatchBuilder &b);
+// Room for the builder's table (which batch_slot_launch otherwise takes).
+int batch_slot_reserve(BatchSlot *slot, const BatchBuilder &b);
 void batch_slot_release(BatchSlot *slot);
 // Fills a StagedReq / FwdAux pair for a volume already on the device.
 void staged_request(int n, int pitch, int ndir, int nshift, int L, int storage,
