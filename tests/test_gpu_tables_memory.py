@@ -69,3 +69,14 @@ def test_batch_equals_alone_in_a_tight_budget():
         for (n, _), (v, g, out), got in zip(sizes, keep, batched):
             wrt.radon_forward_device(c, v, g, out.ptr, half_extent=n)
             assert np.array_equal(got, out.download(np.empty(g.nplanes))), n
+
+
+def test_nearest_bits_do_not_depend_on_the_memory():
+    n, grid = 45, (8, 33, 64)
+    vol = np.random.default_rng(n).standard_normal((n, n, n))
+    got = []
+    for mb in (0, 48, 32, 24, 20):  # all of them room for the least
+        with wrt.Context(0, budget_bytes=mb << 20) as c:
+            got.append(c.radon_grid(vol, *grid, sampler=wrt.NEAREST, half_extent=n))
+    for x in got[1:]:
+        assert np.array_equal(got[0], x)

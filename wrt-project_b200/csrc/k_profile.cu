@@ -1383,16 +1383,21 @@ bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift) 
   return rows * (paired ? 1.0 : 0.5) >= n * (7.0 + 0.4 * n / (paired ? nphi / 2 : nphi));
 }
 
-// The least workspace for nphis phis on an axis, and what holds their whole table.
-static size_t axis_workspace(const ProfReq &r, int nphis, int cells) {
-  return nphis * (axis_head_bytes(r.n, r.ntheta) + (size_t)kAxisSlots * cells * r.n * 4) + 256;
+// Cells of the fixed axis whose tables are made together, by the sizes alone: a plane's
+// sum is added up group by group.  All of them up to n = 512.
+static int axis_cells(int n) {
+  const size_t cell = 4 * (size_t)kAxisSlots * n * 4;  // of four phis
+  return (int)std::min<size_t>(n, std::max<size_t>(1, ((size_t)512 << 20) / cell));
+}
+static size_t axis_workspace(const ProfReq &r, int nphis) {
+  return nphis * (axis_head_bytes(r.n, r.ntheta) + (size_t)kAxisSlots * axis_cells(r.n) * r.n * 4) + 256;
 }
 
 // The least workspace a request can be computed in: that of one unit.
 size_t profile_workspace_least(const ProfReq &r, float crop) {
   size_t ws = 1 << 20;
   while (!Areas(ws).fits(unit_bytes(r, crop), chunk_group(r), UnitBytes())) ws += ws / 16;
-  if (r.nearest) ws = al(ws) + std::max(al(axis_workspace(r, 4, 1)), al(ws / 7));
+  if (r.nearest) ws = al(ws) + al(axis_workspace(r, 4));
   return ws;
 }
 
@@ -1411,14 +1416,13 @@ size_t profile_workspace_want(const ProfReq *reqs, const float *crop, int nreq) 
     least = std::max(least, profile_workspace_least(r, crop[q]));
   }
   const size_t ws = std::min(table, kProfTableBytes) / 176 * 256 + (4 << 20);
-  // (the nearest sampler's phis on an axis come first, in up to an eighth)
-  return std::max(least, reqs[0].nearest ? ws + ws / 7 : ws);
+  // (the tables of the nearest sampler's phis on an axis come first)
+  return std::max(least, reqs[0].nearest ? ws + al(axis_workspace(reqs[0], 4)) : ws);
 }
 
 static int axis_forward(wrt_ctx *ctx, cudaStream_t stream, const ProfReq &r, const int *phis, int nphis,
-                        void *ws, size_t ws_bytes) {
-  int cells = r.n;
-  while (cells > 1 && axis_workspace(r, nphis, cells) > ws_bytes) --cells;
+                        void *ws) {
+  const int cells = axis_cells(r.n);
   AxisJob a = {};
   a.r = r;
   for (int p = 0; p < nphis; ++p) a.phi[p] = phis[p];
@@ -1622,15 +1626,14 @@ int profile_forward_nearest(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes,
   if (st) return st;
   cudaError_t e = cudaEventRecord(lanes->fork, stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "profile fork");
-  const size_t part = al(std::min(axis_workspace(r, nphis, r.n),
-                                  std::max(axis_workspace(r, nphis, 1), ws_bytes / 8)));
+  const size_t part = al(axis_workspace(r, nphis));
   char *rest = static_cast<char *>(ws) + part;
   const bool small = unit_bytes(r, crop).table * (r.paired ? r.nphi / 2 : r.nphi) < kProfLaneBytes;
   if (small) {
     st = profile_forward(ctx, stream, lanes, &r, &crop, 1, rest, ws_bytes - part, PROF_BESIDE);
     if (st) return st;
   }
-  st = axis_forward(ctx, stream, r, phis, nphis, ws, part);
+  st = axis_forward(ctx, stream, r, phis, nphis, ws);
   if (!small)
     return st ? st : profile_forward(ctx, stream, lanes, &r, &crop, 1, rest, ws_bytes - part,
                                      PROF_FORKED);
