@@ -311,15 +311,19 @@ void *wrt_ctx_stream(wrt_ctx *ctx);
 
 /* Autotuner of the staged plane kernel's tile shape (CTA size, lattice rows
  * walked together per warp, shifts enumerated per lane): runs every
- * configuration on this request (dev_out receives the result), times each
- * with CUDA events and keeps the fastest in the context.  *best / *best_ms
- * (either may be NULL) receive the chosen index and its time per launch. */
+ * tile on this request (dev_out receives the result), times each
+ * with CUDA events and keeps the fastest in the context, for the requests that
+ * take the staged kernel (their sizes decide that as before; a forced
+ * configuration ends).  *best / *best_ms (either may be NULL) receive the
+ * chosen index and its time per launch. */
 int wrt_tune_plane_kernel(wrt_ctx *ctx, const wrt_volume *vol, const wrt_grid *grid,
                           const wrt_plane_opts *opts, double *dev_out, int *best,
                           float *best_ms);
-/* Number of tile configurations; their shapes; force one (-1: default, the
- * row-sum profiles or the staged kernel's default tile by the request's sizes).
- * The last one is the row-sum profiles, for every request they cover. */
+/* Number of configurations; their shapes; force one for every request (-1:
+ * none, the row-sum profiles or the staged kernel's default tile by the
+ * request's sizes).  All but the last are tiles of the staged kernel; the last
+ * one has no shape (zeros) and is the row-sum profiles, for every request they
+ * cover. */
 int wrt_plane_kernel_config_count(void);
 int wrt_plane_kernel_config_describe(int index, int *threads, int *rows_per_group,
                                      int *shifts_per_lane);

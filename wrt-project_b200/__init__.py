@@ -591,8 +591,9 @@ def radon3d_adjoint_static(ctx: Context, dev_radon: int, nphi: int, ntheta: int,
 
 
 def plane_kernel_configs():
-    """Tile shapes of the staged plane kernel: list of (threads, rows per
-    group, shifts per lane)."""
+    """Configurations of the plane transform: the staged kernel's tile shapes
+    (threads, rows per group, shifts per lane) and, last, the row-sum profiles
+    (zeros: no tile)."""
     out = []
     for k in range(lib().wrt_plane_kernel_config_count()):
         t, g, s = _i(), _i(), _i()
@@ -607,7 +608,9 @@ def set_plane_kernel_config(ctx: Context, index: int):
 
 def tune_plane_kernel(ctx: Context, vol: Volume, grid: Grid, dev_out: int, sampler=TRILINEAR,
                       half_extent=0):
-    """Run the autotuner on this request; returns (best index, ms per launch)."""
+    """Run the autotuner of the staged kernel's tile on this request; returns
+    (best index, ms per launch).  The tile serves the requests that take the
+    staged kernel by their sizes."""
     o = plane_opts(sampler, half_extent, KERNEL_STAGED)
     best, ms = _i(), C.c_float()
     ctx.check(lib().wrt_tune_plane_kernel(ctx.handle, vol.handle, grid.handle, C.byref(o),
@@ -616,9 +619,10 @@ def tune_plane_kernel(ctx: Context, vol: Volume, grid: Grid, dev_out: int, sampl
 
 
 def radon_forward_batch(ctx: Context, requests):
-    """One launch for many forward requests.  ``requests``: sequence of
+    """Many forward requests together.  ``requests``: sequence of
     (Volume, Grid, dev_out pointer, half_extent) tuples; asynchronous on the
-    context's stream (trilinear sampler, staged kernel)."""
+    context's stream (trilinear sampler; the row-sum profiles or the staged
+    kernel by each request's sizes)."""
     arr = (ForwardReq * max(1, len(requests)))()
     for k, (vol, grid, dev_out, half_extent) in enumerate(requests):
         arr[k].volume = vol.handle.value

@@ -998,6 +998,7 @@ int wrt_plane_kernel_config_describe(int index, int *threads, int *rows_per_grou
 int wrt_ctx_set_plane_kernel_config(wrt_ctx *ctx, int index) {
   if (!ctx || index < -1 || index >= kNumStagedConfigs) return WRT_ERR_INVALID_ARGUMENT;
   ctx->staged_config = index;
+  if (index < 0) ctx->staged_tile = 0;
   return WRT_OK;
 }
 
@@ -1013,7 +1014,8 @@ int wrt_tune_plane_kernel(wrt_ctx *ctx, const wrt_volume *vol, const wrt_grid *g
     return fail(ctx, WRT_ERR_CUDA, "tuner events");
   int st = WRT_OK, best_i = -1;
   float best_t = 0.0f;
-  for (int c = 0; c < kNumStagedConfigs && !st; ++c) {
+  // the staged kernel's tiles; whether a request takes that kernel is the sizes' matter
+  for (int c = 0; c < kNumStagedConfigs - 1 && !st; ++c) {
     ctx->staged_config = c;
     st = wrt_radon_forward_device(ctx, vol, grid, &o, dev_out);  // warm-up
     float tmin = 0.0f;
@@ -1033,7 +1035,8 @@ int wrt_tune_plane_kernel(wrt_ctx *ctx, const wrt_volume *vol, const wrt_grid *g
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
-  ctx->staged_config = st ? -1 : best_i;
+  ctx->staged_config = -1;
+  ctx->staged_tile = st ? 0 : best_i;
   if (!st) {
     if (best) *best = best_i;
     if (best_ms) *best_ms = best_t;

@@ -376,7 +376,7 @@ int capture(BatchSlot *s) {
   if (!s->copy_node) return fail(ctx, WRT_ERR_INTERNAL, "batch graph: no table upload node");
   e = cudaGraphInstantiate(&s->exec, graph, 0);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "batch graph instantiate");
-  s->config = ctx->staged_config;
+  s->config = plane_staged_tile(ctx);
   s->counting = ctx->d_counter != nullptr;
   return WRT_OK;
 }
@@ -402,7 +402,7 @@ int batch_slot_launch(BatchSlot *s, BatchBuilder &b) {
   const size_t bytes = BatchLayout::bytes(b.items.size());
   int st = ensure_capacity(s, bytes);
   if (st) return st;
-  if (!s->exec || s->config != ctx->staged_config || s->counting != (ctx->d_counter != nullptr)) {
+  if (!s->exec || s->config != plane_staged_tile(ctx) || s->counting != (ctx->d_counter != nullptr)) {
     st = capture(s);
     if (st) return st;
   }

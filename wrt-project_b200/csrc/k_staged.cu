@@ -782,18 +782,22 @@ int launch_cfg(wrt_ctx *ctx, cudaStream_t stream, const StagedReq *d_reqs,
 // was the fastest at 96^3, 128^3 and 256^3 on B200.
 const StagedConfig kStagedConfigs[] = {
     {1024, 8, 2}, {768, 8, 2}, {768, 4, 2}, {1024, 4, 2}, {768, 2, 2}, {1024, 1, 2}, {512, 8, 4},
-    // the row-sum profiles (k_profile.cu) where they cover the request, else the
-    // default tile: one row at a time per lane, lanes on shifts
-    {256, 32, 1},
+    // no tile: the row-sum profiles (k_profile.cu) where they cover the request, else
+    // the default tile
+    {0, 0, 0},
 };
 const int kNumStagedConfigs = sizeof(kStagedConfigs) / sizeof(kStagedConfigs[0]);
+
+int plane_staged_tile(const wrt_ctx *ctx) {
+  return ctx->staged_config < 0                        ? ctx->staged_tile
+         : ctx->staged_config < kNumStagedConfigs - 1 ? ctx->staged_config
+                                                       : 0;
+}
 
 int plane_staged_launch(wrt_ctx *ctx, cudaStream_t stream, const StagedReq *d_reqs,
                         const StagedItem *d_items, const int *d_nitems, int max_smem,
                         int *d_next) {
-  const int c = (ctx->staged_config >= 0 && ctx->staged_config < kNumStagedConfigs - 1)
-                    ? ctx->staged_config : 0;
-  switch (c) {
+  switch (plane_staged_tile(ctx)) {
     case 0: return launch_cfg<1024, 8, 2>(ctx, stream, d_reqs, d_items, d_nitems, max_smem, d_next);
     case 1: return launch_cfg<768, 8, 2>(ctx, stream, d_reqs, d_items, d_nitems, max_smem, d_next);
     case 2: return launch_cfg<768, 4, 2>(ctx, stream, d_reqs, d_items, d_nitems, max_smem, d_next);

@@ -63,7 +63,8 @@ struct wrt_ctx {
   size_t staged_req_bytes = 0;
   int *staged_next = nullptr;
   void *staged_cache = nullptr;
-  int staged_config = -1;  // tile configuration (-1: default), set by the autotuner
+  int staged_config = -1;  // configuration forced for every plane transform (-1: none)
+  int staged_tile = 0;     // the staged kernel's tile otherwise, set by the autotuner
   void *batch_slot = nullptr;  // BatchSlot of wrt_radon_forward_batch (batch.cu)
   // grow-only working buffers, one per role (wrt::ws_get), freed with the
   // context: warm calls of the same or smaller sizes allocate nothing
@@ -221,6 +222,7 @@ constexpr int kStagedDirChunk = 512;  // directions per work item
 // per warp, 48 KB at 1024 threads) and a few static words.
 constexpr int kStagedSmemMax = 168 * 1024;
 constexpr int kStagedWarpSmemQuads = 96;
+int plane_staged_tile(const wrt_ctx *ctx);  // the tile in effect
 int plane_staged_launch(wrt_ctx *ctx, cudaStream_t stream, const StagedReq *d_reqs,
                         const StagedItem *d_items, const int *d_nitems, int max_smem,
                         int *d_next);
