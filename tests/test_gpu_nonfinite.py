@@ -1,0 +1,55 @@
+"""Values that are no numbers: what does not touch them is as without them."""
+import numpy as np
+import pytest
+
+import oracle as O
+from conftest import rel_l2, wrt
+
+pytestmark = pytest.mark.gpu
+
+TOL_L2 = 1e-5  # the FP32 tolerance of every parity test
+
+
+def _volume(n, at):
+    v = np.random.default_rng(n).standard_normal((n, n, n)).astype(np.float32)
+    for x in at:
+        v[x] = np.nan
+    return v
+
+
+VOLUMES = [(40, [(20, 21, 5)]), (40, [(0, 0, 7)]), (33, [(3, 30, 16), (12, 2, 31)])]
+GRID = (20, 16, 60)
+
+
+@pytest.mark.parametrize("sampler", [O.TRILINEAR, O.NEAREST])
+@pytest.mark.parametrize("n,at", VOLUMES)
+def test_planes(ctx, sampler, n, at):
+    v = _volume(n, at).astype(np.float64)
+    ref = O.radon_forward(v, *GRID, sampler=sampler, half_extent=n)
+    clear = np.isfinite(ref)
+    assert 0.2 < clear.mean() < 1.0
+    got = ctx.radon_grid(v, *GRID, sampler=sampler, half_extent=n)
+    assert rel_l2(got[clear], ref[clear]) < TOL_L2
+
+
+def test_planes_batched_and_served_equal_alone(ctx):
+    n, at = VOLUMES[0]
+    vols = [_volume(n, a) for a in (at, [], [(0, 0, 7)])]
+    alone = []
+    for v in vols:
+        vol = wrt.Volume(ctx, n)
+        vol.upload(v)
+        g = wrt.Grid(ctx, *GRID)
+        out = wrt.DeviceBuffer(ctx, g.nplanes * 8)
+        wrt.radon_forward_device(ctx, vol, g, out.ptr, half_extent=n)
+        alone.append((vol, g, out, out.download(np.empty(g.nplanes))))
+    wrt.radon_forward_batch(ctx, [(v, g, o.ptr, n) for v, g, o, _ in alone])
+    for _, g, out, x in alone:
+        assert np.array_equal(x, out.download(np.empty(g.nplanes)), equal_nan=True)
+    with wrt.Server(0, budget_bytes=1 << 30) as srv:
+        outs = [np.zeros((GRID[2], GRID[0], GRID[1])) for _ in vols]
+        ids = [srv.submit_forward(v, *GRID, o, half_extent=n) for v, o in zip(vols, outs)]
+        for i in ids:
+            assert srv.wait(i, 120_000).status == 0
+    for (_, _, _, x), o in zip(alone, outs):
+        assert np.array_equal(x, o.ravel(), equal_nan=True)

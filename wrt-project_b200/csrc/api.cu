@@ -22,8 +22,10 @@ struct wrt_volume {
   wrt_ctx *ctx = nullptr;
   int n = 0;
   float *d_vol = nullptr;          // n^3, v[ix][iy][iz]
-  unsigned int *d_stats = nullptr; // [0] largest |x|^2 of a non-zero node, [1] max |v| (float bits)
+  unsigned int *d_stats = nullptr; // [0] largest |x|^2 of a non-zero node, [1] max |v| (float
+                                   // bits), [2] values that do not suit tables
   float r2 = 3.0f, maxabs = 0.0f;  // host copies of d_stats, read at upload
+  bool wild = false;
   float2 *d_pairs = nullptr;       // layer pairs for the staged kernel (built on first use)
   int pitch = 0;
   size_t vol_bytes = 0, pair_bytes = 0;
@@ -463,7 +465,7 @@ int wrt_volume_create_storage(wrt_ctx *ctx, int n, int storage, wrt_volume **out
     v->vol_bytes = sizeof(float) * count;
     st = ctx_alloc(ctx, (void **)&v->d_vol, v->vol_bytes);
   }
-  if (!st) st = ctx_alloc(ctx, (void **)&v->d_stats, 2 * sizeof(unsigned int));
+  if (!st) st = ctx_alloc(ctx, (void **)&v->d_stats, kVolumeStats * sizeof(unsigned int));
   if (st) {
     wrt_volume_destroy(v);
     return st;
@@ -476,11 +478,12 @@ namespace {
 // Waits for the upload and copies the volume statistics to the host.
 int volume_finish_upload(wrt_volume *v) {
   wrt_ctx *ctx = v->ctx;
-  unsigned int stats[2] = {0, 0};
+  unsigned int stats[kVolumeStats] = {};
   int st = d2h_sync(ctx, stats, v->d_stats, sizeof(stats), "volume statistics");
   if (st) return st;
   memcpy(&v->r2, &stats[0], sizeof(float));
   memcpy(&v->maxabs, &stats[1], sizeof(float));
+  v->wild = stats[2] != 0;
   v->pairs_valid = false;
   v->oct_valid = false;
   v->layers_valid = false;
@@ -569,7 +572,7 @@ int wrt_volume_upload_device(wrt_volume *v, const float *dev_f32) {
 
 size_t wrt_volume_bytes(const wrt_volume *v) {
   return v ? v->vol_bytes + v->pair_bytes + v->oct_bytes + (v->d_layers ? v->vol_bytes : 0) +
-                 2 * sizeof(unsigned int)
+                 kVolumeStats * sizeof(unsigned int)
            : 0;
 }
 
@@ -580,7 +583,7 @@ int wrt_volume_destroy(wrt_volume *v) {
   cudaStreamSynchronize(ctx->stream);
   ctx_free(ctx, v->d_vol, v->vol_bytes);
   ctx_free(ctx, v->d_vol16, v->vol_bytes);
-  ctx_free(ctx, v->d_stats, 2 * sizeof(unsigned int));
+  ctx_free(ctx, v->d_stats, kVolumeStats * sizeof(unsigned int));
   ctx_free(ctx, v->d_pairs, v->pair_bytes);
   ctx_free(ctx, v->d_pairs16, v->pair_bytes);
   ctx_free(ctx, v->d_oct, v->oct_bytes);
@@ -833,7 +836,7 @@ int wrt_radon_forward_device(wrt_ctx *ctx, const wrt_volume *cvol, const wrt_gri
   if (o.kernel == WRT_KERNEL_STAGED && !staged_ok)
     return fail(ctx, WRT_ERR_INVALID_ARGUMENT, "staged kernel: volume edge below 4");
   if (o.kernel != WRT_KERNEL_PLAIN && staged_ok) {
-    if (profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift)) {
+    if (!vol->wild && profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift)) {
       bool done = false;
       st = radon_forward_profile(ctx, vol, grid, L, dev_out, nearest, &done);
       if (st || done) return st;
@@ -878,7 +881,7 @@ int wrt_radon_forward_batch(wrt_ctx *ctx, const wrt_forward_req *reqs, int nreq)
         reqs[r].half_extent > 8 * vol->n)
       continue;  // refused below
     const int L = reqs[r].half_extent ? reqs[r].half_extent : 2 * vol->n;
-    if (!profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift)) continue;
+    if (vol->wild || !profile_route(ctx, vol->n, grid->nphi, grid->ntheta, grid->nshift)) continue;
     staged[r] = 0;
     routed.push_back(r);
     prof.push_back(profile_request(ctx, vol, grid, L, false, reqs[r].dev_out));

@@ -87,6 +87,7 @@ __global__ void batch_reset_kernel(char *t) {
     unsigned long long *acc = F[r].acc;
     for (long long k = tid; k < A[r].nout; k += nth) acc[k] = 0ull;
     if (A[r].prep && tid < 2) A[r].stats[tid] = 0u;
+    if (A[r].wild && tid == 2) *A[r].wild = 0u;
   }
 }
 
@@ -103,9 +104,11 @@ __global__ void batch_volume_kernel(char *t) {
     const float *v = A[r].vol;
     const long long total = (long long)n * n * n;
     float local = 0.0f, amax = 0.0f;
+    bool wild = false;
     for (long long k = tid; k < total; k += nth) {
       const float x = v[k];
       amax = fmaxf(amax, fabsf(x));
+      wild |= !(fabsf(x) <= wrt::kTableMost);
       if (x != 0.0f) {
         const int iz = (int)(k % n), iy = (int)((k / n) % n), ix = (int)(k / ((long long)n * n));
         local = fmaxf(local, wrtd::node_r2(ix, iy, iz, n));
@@ -115,7 +118,9 @@ __global__ void batch_volume_kernel(char *t) {
       local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, o));
       amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     }
+    wild = __any_sync(0xffffffffu, wild);
     if ((threadIdx.x & 31) == 0) {
+      if (wild && A[r].wild) atomicOr(A[r].wild, 1u);
       if (local > 0.0f) atomicMax(A[r].stats, __float_as_uint(local));
       if (amax > 0.0f) atomicMax(A[r].stats + 1, __float_as_uint(amax));
     }
@@ -445,6 +450,11 @@ int batch_slot_launch(BatchSlot *s, BatchBuilder &b) {
     st = profile_forward(ctx, s->stream, &s->prof_lanes, b.prof.data(), crop.data(),
                          (int)b.prof.size(), s->prof_ws, s->prof_bytes);
     if (st) return st;
+    if (s->d_wild) {
+      e = cudaMemcpyAsync(s->h_wild, s->d_wild, sizeof(unsigned) * b.fwd.size(),
+                          cudaMemcpyDeviceToHost, s->stream);
+      if (e != cudaSuccess) return cuda_fail(ctx, e, "batch flags");
+    }
   }
   for (const RedReq &q : b.staged_red) {
     st = reduction_staged(ctx, s->stream, q.rays, q.ngrid, q.ns_ray, q.nphi, q.shift, q.nshift, q.cs,
@@ -474,6 +484,8 @@ void batch_slot_release(BatchSlot *s) {
   if (s->launched) cudaEventSynchronize(s->done);
   drop_graph(s);
   ctx_free(s->ctx, s->prof_ws, s->prof_bytes);
+  ctx_free(s->ctx, s->d_wild, sizeof(unsigned) * kBatchMaxFwd);
+  if (s->h_wild) cudaFreeHost(s->h_wild);
   profile_lanes_release(&s->prof_lanes);
   if (s->h_table) cudaFreeHost(s->h_table);
   ctx_free(s->ctx, s->d_table, s->cap);

@@ -11,7 +11,10 @@
 //              max).  Every lattice sample farther than sqrt(r2) + sqrt(3)
 //              delta from the origin has only zero corners, so it contributes
 //              exactly 0; the kernels skip those samples.  This is exact for
-//              any input, not an assumption about the support.
+//              any input, not an assumption about the support;
+//   * stats[2] non-zero when some value is no number, infinite or beyond
+//              wrt::kTableMost: running sums would carry it past its cell, so
+//              such volumes take the kernels that read every sample on its own.
 //   * d_pairs  layer pairs for the staged plane kernel: pairs[iz][iy][ix] =
 //              (v[ix][iy][iz], v[ix][iy][iz+1]) for iz in [0, n-2], rows
 //              padded to `pitch` elements so every row starts 16-byte aligned;
@@ -28,11 +31,13 @@ __global__ void volume_convert_kernel(const T *__restrict__ src, int n, float *_
                                       unsigned int *__restrict__ stats) {
   const size_t total = (size_t)n * n * n;
   float local = 0.0f, amax = 0.0f;
+  bool wild = false;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total;
        k += (size_t)gridDim.x * blockDim.x) {
     float v = (float)src[k];
     dst[k] = v;
     amax = fmaxf(amax, fabsf(v));
+    wild |= !(fabsf(v) <= wrt::kTableMost);
     if (v != 0.0f) {
       const int iz = (int)(k % n), iy = (int)((k / n) % n), ix = (int)(k / ((size_t)n * n));
       local = fmaxf(local, wrtd::node_r2(ix, iy, iz, n));
@@ -43,7 +48,9 @@ __global__ void volume_convert_kernel(const T *__restrict__ src, int n, float *_
     local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, o));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   }
+  wild = __any_sync(0xffffffffu, wild);
   if ((threadIdx.x & 31) == 0) {
+    if (wild) atomicOr(stats + 2, 1u);
     if (local > 0.0f) atomicMax(stats, __float_as_uint(local));
     if (amax > 0.0f) atomicMax(stats + 1, __float_as_uint(amax));
   }
@@ -87,12 +94,14 @@ __global__ void volume_bf16_kernel(const float *__restrict__ src, int n,
                                    __nv_bfloat16 *__restrict__ dst, unsigned int *__restrict__ stats) {
   const size_t total = (size_t)n * n * n;
   float local = 0.0f, amax = 0.0f;
+  bool wild = false;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < total;
        k += (size_t)gridDim.x * blockDim.x) {
     const __nv_bfloat16 b = __float2bfloat16_rn(src[k]);
     dst[k] = b;
     const float v = __bfloat162float(b);
     amax = fmaxf(amax, fabsf(v));
+    wild |= !(fabsf(v) <= wrt::kTableMost);
     if (v != 0.0f) {
       const int iz = (int)(k % n), iy = (int)((k / n) % n), ix = (int)(k / ((size_t)n * n));
       local = fmaxf(local, wrtd::node_r2(ix, iy, iz, n));
@@ -102,7 +111,9 @@ __global__ void volume_bf16_kernel(const float *__restrict__ src, int n,
     local = fmaxf(local, __shfl_xor_sync(0xffffffffu, local, o));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
   }
+  wild = __any_sync(0xffffffffu, wild);
   if ((threadIdx.x & 31) == 0) {
+    if (wild) atomicOr(stats + 2, 1u);
     if (local > 0.0f) atomicMax(stats, __float_as_uint(local));
     if (amax > 0.0f) atomicMax(stats + 1, __float_as_uint(amax));
   }
@@ -126,7 +137,7 @@ __global__ void volume_pairs_bf16_kernel(const __nv_bfloat16 *__restrict__ v, in
 
 template <typename T>
 int convert(wrt_ctx *ctx, const T *d_src, int n, float *d_vol, unsigned int *d_stats) {
-  cudaError_t e = cudaMemsetAsync(d_stats, 0, 2 * sizeof(unsigned int), ctx->stream);
+  cudaError_t e = cudaMemsetAsync(d_stats, 0, wrt::kVolumeStats * sizeof(unsigned int), ctx->stream);
   if (e != cudaSuccess) return wrt::cuda_fail(ctx, e, "volume stats reset");
   int blocks = ctx->sm_count * 8;
   volume_convert_kernel<T><<<blocks, 256, 0, ctx->stream>>>(d_src, n, d_vol, d_stats);
@@ -145,7 +156,7 @@ int volume_from_f32(wrt_ctx *ctx, const float *d_src, int n, float *d_vol,
 
 int volume_to_bf16(wrt_ctx *ctx, const float *d_vol, int n, __nv_bfloat16 *d_vol16,
                    unsigned int *d_stats) {
-  cudaError_t e = cudaMemsetAsync(d_stats, 0, 2 * sizeof(unsigned int), ctx->stream);
+  cudaError_t e = cudaMemsetAsync(d_stats, 0, wrt::kVolumeStats * sizeof(unsigned int), ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "volume stats reset");
   volume_bf16_kernel<<<ctx->sm_count * 8, 256, 0, ctx->stream>>>(d_vol, n, d_vol16, d_stats);
   ctx->launches++;

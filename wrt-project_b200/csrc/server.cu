@@ -85,6 +85,10 @@ struct Request {
   void *d_tab = nullptr;
   double frame[9] = {};
   bool has_frame = false;
+  // a plane transform by the row-sum profiles: its entry in the batch; and whether it
+  // has to be done over by the staged kernel (its volume does not suit tables)
+  int wild_at = -1;
+  bool staged = false;
 };
 
 constexpr size_t kServerProfBytes = (size_t)3072 << 20;
@@ -430,11 +434,14 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
     p.nshift = r.nshift;
     p.storage = WRT_STORAGE_F32;
     p.paired = wrt::profile_paired(n, r.nphi, L);
-    if (wrt::profile_route(s->ctx, n, r.nphi, r.ntheta, r.nshift) &&
+    q->wild_at = -1;
+    if (!q->staged && wrt::profile_route(s->ctx, n, r.nphi, r.ntheta, r.nshift) &&
         slot.prof_bytes >= wrt::profile_workspace_least(p, 3.0f + 1e-5f)) {
       a.pairs = nullptr;
       a.nout = 0;
       sr.nshift = sr.ndir = 0;
+      q->wild_at = (int)b.fwd.size();
+      a.wild = slot.d_wild + q->wild_at;
       b.fwd.push_back(sr);
       b.aux.push_back(a);
       b.prof.push_back(p);
@@ -607,10 +614,14 @@ void complete_loop(wrt_server *s) {
     cudaError_t e = cudaEventSynchronize(slot->ev);
     if (e != cudaSuccess) st = WRT_ERR_CUDA;
     std::vector<int> per(slot->reqs.size(), st);
+    // the host does not look at the volumes: those that turn out not to suit the tables go
+    // to the front of the queue for the staged kernel
+    std::vector<char> again(slot->reqs.size(), 0);
     if (!st) {
       for (size_t k = 0; k < slot->reqs.size(); ++k) {
         Request *q = slot->reqs[k];
-        if (q->out_pinned) continue;
+        again[k] = q->wild_at >= 0 && slot->batch.h_wild[q->wild_at] != 0;
+        if (q->out_pinned || again[k]) continue;
         e = cudaMemcpyAsync(q->req.out, q->d_out, q->out_bytes, cudaMemcpyDeviceToHost,
                             s->copy_stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->copy_stream);
@@ -619,7 +630,16 @@ void complete_loop(wrt_server *s) {
     }
     const double t = s->now_ms();
     lk.lock();
-    for (size_t k = 0; k < slot->reqs.size(); ++k) finish(s, slot->reqs[k], per[k], t);
+    for (size_t k = slot->reqs.size(); k-- > 0;) {
+      Request *q = slot->reqs[k];
+      if (again[k] && !s->stop) {
+        q->staged = true;
+        unreserve(s, q);
+        s->arrivals.push_front(q);
+      } else {
+        finish(s, q, again[k] ? WRT_ERR_CANCELLED : per[k], t);
+      }
+    }
     slot->reqs.clear();
     slot->busy = false;
     s->inflight.pop_front();
@@ -691,6 +711,14 @@ int wrt_server_create(const wrt_server_opts *opts, wrt_server **out) {
     if (!st && want >= kServerProfLeast &&
         wrt::ctx_alloc(ctx, &sl->batch.prof_ws, want) == WRT_OK)
       sl->batch.prof_bytes = want;
+    if (sl->batch.prof_bytes) {
+      st = wrt::ctx_alloc(ctx, (void **)&sl->batch.d_wild, sizeof(unsigned) * wrt::kBatchMaxFwd);
+      if (!st && cudaMallocHost((void **)&sl->batch.h_wild,
+                                sizeof(unsigned) * wrt::kBatchMaxFwd) != cudaSuccess) {
+        cudaGetLastError();
+        st = WRT_ERR_OUT_OF_MEMORY;
+      }
+    }
     s->slots.push_back(std::move(sl));
   }
   // every slot or none: a request's kernel must not depend on the slot it gets

@@ -136,7 +136,11 @@ void adjoint_directions(int nphi, int ntheta, int nshift, const double *phi, con
                         const double *theta_w, double4 *dirw);
 
 // Volume preparation kernels (k_volume.cu).
-// d_stats[0]: largest |x|^2 of a non-zero node, d_stats[1]: max |v| (float bits)
+// d_stats[0]: largest |x|^2 of a non-zero node, d_stats[1]: max |v| (float bits),
+// d_stats[2]: some value is no number, infinite or beyond kTableMost (a row of 4096
+// samples of it, and its differences, stay finite in FP32)
+constexpr int kVolumeStats = 3;
+constexpr float kTableMost = 1e34f;
 int volume_from_f32(wrt_ctx *ctx, const float *d_src, int n, float *d_vol,
                     unsigned int *d_stats);
 int volume_pairs(wrt_ctx *ctx, const float *d_vol, int n, float2 *d_pairs, int pitch);
@@ -364,6 +368,7 @@ struct FwdAux {                    // per forward request, beside its StagedReq
   const float *vol;                // FP32 volume, reference order
   float2 *pairs;                   // layer pairs (built in the launch when prep)
   unsigned int *stats;             // [0] r2 bits, [1] max |v| bits (computed when prep)
+  unsigned int *wild;              // set when the values do not suit tables (or null)
   long long nout;                  // nshift * ndir
   double factor;                   // delta^2 / scale, written by the launch
   int n, pitch, L, prep;           // prep: build stats and pairs in this launch
@@ -446,6 +451,9 @@ struct BatchSlot {
   void *prof_ws = nullptr;
   size_t prof_bytes = 0;
   ProfLanes prof_lanes;
+  // per forward entry: its volume does not suit the tables (set by the owner, who reads
+  // h_wild once the launch has ended; null: not asked for)
+  unsigned *d_wild = nullptr, *h_wild = nullptr;
 };
 // Adds a forward request (staged kernel) to the builder: its descriptor, its
 // auxiliary record and its work items.  crop_items: crop radius^2 used to
