@@ -53,3 +53,13 @@ def test_planes_batched_and_served_equal_alone(ctx):
             assert srv.wait(i, 120_000).status == 0
     for (_, _, _, x), o in zip(alone, outs):
         assert np.array_equal(x, o.ravel(), equal_nan=True)
+
+
+@pytest.mark.parametrize("n,nslices", [(40, 40), (33, 33), (40, 7)])  # vector loads, scalar, layer pairs
+def test_rays(ctx, n, nslices):
+    v = _volume(n, [(0, 0, 3), (0, 0, n - 2)]).astype(np.float64)
+    ref = O.ray_forward(v, nslices, 41, 18)
+    clear = np.isfinite(ref)
+    assert 0.2 < clear.mean() < 1.0
+    got = ctx.ray_grid(v, nslices, 41, 18)
+    assert rel_l2(got[clear], ref[clear]) < TOL_L2

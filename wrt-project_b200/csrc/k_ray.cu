@@ -117,6 +117,13 @@ __global__ void __launch_bounds__(32 * kWarps)
       khi = min(2 * n, km);
       if (!(wrtd::clip_axis(p0x, ax, klo, khi) && wrtd::clip_axis(p0y, ay, klo, khi))) khi = klo - 1;
     }
+    // exactly the samples inside: their coordinates are monotone in k
+    auto inside = [&](int k) {
+      return fabs(__dadd_rn(p0x, __dmul_rn(ax, (double)k))) <= 1.0 &&
+             fabs(__dadd_rn(p0y, __dmul_rn(ay, (double)k))) <= 1.0;
+    };
+    while (klo <= khi && !inside(klo)) ++klo;
+    while (klo <= khi && !inside(khi)) --khi;
     int taken = 0;
     for (int k0 = klo; k0 <= khi; k0 += 32) {
       const int k = k0 + lane;
@@ -124,7 +131,7 @@ __global__ void __launch_bounds__(32 * kWarps)
       const double y = __dadd_rn(p0y, __dmul_rn(ay, (double)k));
       float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
       int col = 0;
-      if (k <= khi && fabs(x) <= 1.0 && fabs(y) <= 1.0) {
+      if (k <= khi) {
         int ix, iy;
         double cx, cy;
         cell_of(x, n, &ix, &cx);
