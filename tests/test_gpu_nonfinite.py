@@ -63,3 +63,29 @@ def test_rays(ctx, n, nslices):
     assert 0.2 < clear.mean() < 1.0
     got = ctx.ray_grid(v, nslices, 41, 18)
     assert rel_l2(got[clear], ref[clear]) < TOL_L2
+
+
+@pytest.mark.parametrize("n,nphi,ntheta,nshift,at", [
+    (20, 96, 47, 61, [(30, 7, 20)]), (20, 33, 31, 257, [(0, 4, 9), (200, 4, 9), (40, 5, 9)]),
+])
+def test_backprojection(ctx, n, nphi, ntheta, nshift, at):
+    # a line with such a value has none that is a number; voxels beyond its ends are free of it
+    radon = np.random.default_rng(n).standard_normal((nshift, nphi, ntheta))
+    for x in at:
+        radon[x] = np.nan
+    got = ctx.radon3d_adjoint(radon, n)
+    x = -1.0 + (2.0 * np.arange(n) + 1.0) / n
+    iz, ix, iy = (a.ravel() for a in np.meshgrid(np.arange(n), np.arange(n), np.arange(n), indexing="ij"))
+    phi, theta, _, _ = O.radon_grid(nphi, ntheta, nshift)
+    clear = np.ones(n ** 3, bool)
+    for _, ip, it in at:
+        s = (np.sin(theta[it]) * (np.cos(phi[ip]) * x[ix] + np.sin(phi[ip]) * x[iy])
+             + np.cos(theta[it]) * x[iz])
+        clear &= np.abs(s) > 1.0
+    assert 0.005 < clear.mean() < 1.0
+    assert np.isnan(got.ravel()[~clear]).all()
+    clean = radon.copy()
+    clean[:, [a[1] for a in at], [a[2] for a in at]] = 0.0
+    pick = np.flatnonzero(clear)
+    ref = O.adjoint_points(clean, x[ix[pick]], x[iy[pick]], x[iz[pick]])
+    assert rel_l2(got.ravel()[pick], ref) < TOL_L2

@@ -22,6 +22,9 @@
 //   build:  per z and range of t, lanes on longitudes: the cubic about the
 //           range's start from the lines directly, then one knot after another,
 //           each piece's coefficients at its own start rounded once to FP32
+//   (lines: one with a value that is no number has none that is, and a running sum
+//           would keep it beyond the line's end, so such lines are listed and zeroed by
+//           the solve and their voxels set once the sums are done)
 //   gather: threads on voxels of one z, the list's positions in shared memory,
 //           one 16-byte record per (voxel, longitude); FP64 sums, every voxel
 //           in a fixed order by one thread
@@ -75,6 +78,7 @@ __global__ void __launch_bounds__(kThreads) back_merge_kernel(const BackReq r) {
   __shared__ double tile[32][33];
   const int i = blockIdx.z, b0 = blockIdx.x * 32, t0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x) == 0) r.lost[0] = 0;
   for (int y = ty; y < 32; y += kThreads / 32) {
     const int b = b0 + y, th = t0 + tx;
     if (b < r.nbase && th < r.ntheta) {
@@ -129,6 +133,11 @@ __global__ void __launch_bounds__(64) back_solve_kernel(const BackReq r) {
       ya = yb;
       yb = v[u];
     }
+  }
+  if (!(fabs(prev) < 1e300)) {  // every y enters it
+    r.lost[1 + atomicAdd(r.lost, 1)] = L;
+    for (int i = 0; i < ns; ++i) r.Y[o + i * st] = m[i * st] = D[i * st] = 0.0;
+    return;
   }
   // from the end: mc = m_{i+1}, md = m_{i+2}
   double mc = 0.0, md = 0.0;
@@ -467,6 +476,26 @@ __global__ void __launch_bounds__(kGatherThreads, 2) back_gather_kernel(const Ba
   }
 }
 
+// The voxels on the lines that the solve has listed, as a rule none.
+__global__ void __launch_bounds__(kThreads) back_lost_kernel(const BackReq r) {
+  const int lost = r.lost[0], n = r.n, ns = r.ns;
+  if (!lost) return;
+  const long long total = (long long)n * n * n;
+  for (long long v = blockIdx.x * (long long)kThreads + threadIdx.x; v < total;
+       v += (long long)gridDim.x * kThreads) {
+    const double z = z_of(n, (int)(v / ((long long)n * n))), x = z_of(n, (int)(v / n % n)),
+                 y = z_of(n, (int)(v % n));
+    for (int k = 1; k <= lost; ++k) {
+      const int th = r.lost[k] / r.nbase, b = r.lost[k] % r.nbase;
+      const double4 g = r.dirw[(size_t)b * r.ntheta + th];
+      const double q = fma(x, g.x, fma(y, g.y, fma(z, g.z, 0.5 * (ns - 1))));
+      if (!(q >= 0.0 && q <= (double)(ns - 1))) continue;
+      r.out[v] = __longlong_as_double(0x7ff8000000000000ll);
+      break;
+    }
+  }
+}
+
 size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 int log2_up(int x) {
   int k = 0;
@@ -476,7 +505,7 @@ int log2_up(int x) {
 
 struct Plan {
   int cap, nb_log2, nsub_log2, nbase;
-  size_t data, table, rec, pos, start, keys;  // data: Y, M, D each; the rest per z
+  size_t data, lost, table, rec, pos, start, keys;  // data: Y, M, D each; from table on per z
   size_t list() const { return rec + pos + start + keys; }  // of one z plane
 };
 Plan plan_of(int nphi, int ntheta, int ns) {
@@ -488,6 +517,7 @@ Plan plan_of(int nphi, int ntheta, int ns) {
   // at least one bin per thread of the sort and per range
   p.nb_log2 = std::max({log2_up(knots) - 2, 9, p.nsub_log2});
   p.data = al(sizeof(double) * (size_t)knots * p.nbase);
+  p.lost = al(sizeof(int) * ((size_t)ntheta * p.nbase + 1));
   p.table = al(16 * (size_t)p.cap * p.nbase);
   p.rec = al(sizeof(KnotRec) * (size_t)p.cap);
   p.pos = al(2 * 4 * (size_t)(p.cap + 16));
@@ -544,7 +574,7 @@ size_t backproj_workspace(int nphi, int ntheta, int ns, int n, bool least) {
   const Plan p = plan_of(nphi, ntheta, ns);
   const size_t most = std::min<size_t>(n, std::max<size_t>(1, kBackTableBytes / p.table));
   const size_t z = least ? std::min<size_t>(most, least_planes(nphi, ntheta, n, p.nbase)) : most;
-  return 3 * p.data + n * p.list() + z * p.table + 4096;
+  return 3 * p.data + p.lost + n * p.list() + z * p.table + 4096;
 }
 
 int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackReq r, void *ws,
@@ -556,7 +586,8 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
   r.Y = reinterpret_cast<double *>(at);
   r.M = reinterpret_cast<double *>(at + p.data);
   r.D = reinterpret_cast<double *>(at + 2 * p.data);
-  at += 3 * p.data;
+  r.lost = reinterpret_cast<int *>(at + 3 * p.data);
+  at += 3 * p.data + p.lost;
   cudaError_t e = cudaSuccess;
   // ---- z planes, dealt in groups to the lanes
   char *lists = at;
@@ -630,6 +661,11 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
   for (int k = 1; k < nl && e == cudaSuccess; ++k) {
     e = cudaEventRecord(lanes->done[k - 1], lanes->stream[k - 1]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, lanes->done[k - 1], 0);
+  }
+  if (e == cudaSuccess) {
+    back_lost_kernel<<<ctx->sm_count * 2, kThreads, 0, stream>>>(r);
+    ctx->launches++;
+    e = cudaGetLastError();
   }
   return e == cudaSuccess ? WRT_OK : cuda_fail(ctx, e, "merged backprojection");
 }

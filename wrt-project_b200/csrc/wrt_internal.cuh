@@ -325,6 +325,7 @@ struct BackReq {
   // set by backproj_forward
   int nbase, paired;     // longitudes tabulated; phi + pi merged into phi
   double *Y, *M, *D;     // [theta][is][nbase]
+  int *lost;             // count, then the lines (theta nbase + phi) with no finite spline
 };
 constexpr size_t kBackTableBytes = (size_t)768 << 20;  // tables in flight
 struct BackStep {        // a group of z planes
