@@ -595,6 +595,12 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
   const size_t left = ws_bytes - (at - static_cast<char *>(ws));
   const int nz = (int)std::max<size_t>(1, std::min<size_t>(r.n, left / p.table));
   const int nl = lanes_of(r.n, nz);
+  // nothing may still use the workspace when a failed call returns
+  auto failed = [&](cudaError_t err) {
+    cudaStreamSynchronize(stream);
+    for (int k = 0; nl > 1 && k < kProfLanes - 1; ++k) cudaStreamSynchronize(lanes->stream[k]);
+    return cuda_fail(ctx, err, "merged backprojection");
+  };
   const size_t sm_sort = 4 * ((size_t)1 << p.nb_log2);
   const size_t sm_build = build_smem(r.ntheta);
   const size_t sm_gather = gather_smem(p);
@@ -667,7 +673,7 @@ int backproj_forward(wrt_ctx *ctx, cudaStream_t stream, ProfLanes *lanes, BackRe
     ctx->launches++;
     e = cudaGetLastError();
   }
-  return e == cudaSuccess ? WRT_OK : cuda_fail(ctx, e, "merged backprojection");
+  return e == cudaSuccess ? WRT_OK : failed(e);
 }
 
 }  // namespace wrt

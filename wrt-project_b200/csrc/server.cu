@@ -576,6 +576,8 @@ void dispatch_loop(wrt_server *s) {
       cudaError_t e = cudaEventRecord(slot->ev, slot->stream);
       if (e != cudaSuccess && !st) st = wrt::cuda_fail(s->ctx, e, "server event");
     }
+    // what a failed launch has queued still works in the requests' memory
+    if (st) cudaStreamSynchronize(slot->stream);
     lk.lock();
     if (st) {
       const double t = s->now_ms();
