@@ -35,6 +35,17 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (sm_100)")
 
 
+def pytest_collection_modifyitems(items):
+    # comparisons with the reference's own integrators need them built (oracle/_ref, which
+    # only happens where the reference's sources are); the other such tests say so themselves
+    import oracle
+
+    if not oracle.Reference.available():
+        for item in items:
+            if item.path.name == "test_gpu_analytic.py" and "match_the_reference" in item.name:
+                item.add_marker(pytest.mark.skip(reason="oracle/_ref not built"))
+
+
 def rel_l2(a, b):
     a, b = np.asarray(a, np.float64), np.asarray(b, np.float64)
     den = np.linalg.norm(b.ravel())
