@@ -392,11 +392,13 @@ typedef struct wrt_server_opts {
                           + 64 ray + 64 reduce) */
   int max_inflight;    /* launches on the device at once (0: 2; at most 8) */
   int queue_capacity;  /* requests waiting for admission (0: 65536) */
-  size_t hbm_budget;   /* device memory for request state and grid tables
-                          (0: 60 GiB or 3/4 of the free memory, whichever is less);
-                          tables that only make requests faster come beside it,
-                          where there is room: an eighth of it, at most 3 GB,
-                          per launch in flight */
+  size_t hbm_budget;   /* device memory for request state, grid tables and the
+                          working tables that only make requests faster (an
+                          eighth of it, at most 3 GB, per launch in flight; at
+                          most half of it in all) (0: 60 GiB or 3/4 of the free
+                          memory, whichever is less).  A request that has no
+                          room beside those tables runs alone, in their memory
+                          and without them */
   int reserved[8];
 } wrt_server_opts;
 

@@ -483,7 +483,6 @@ void batch_slot_release(BatchSlot *s) {
   if (!s->ctx) return;
   if (s->launched) cudaEventSynchronize(s->done);
   drop_graph(s);
-  ctx_free(s->ctx, s->prof_ws, s->prof_bytes);
   ctx_free(s->ctx, s->d_wild, sizeof(unsigned) * kBatchMaxFwd);
   if (s->h_wild) cudaFreeHost(s->h_wild);
   profile_lanes_release(&s->prof_lanes);

@@ -77,6 +77,10 @@ struct Request {
   bool out_pinned = false;
   // device pointers inside the block
   void *d_in = nullptr;
+  float2 *d_pairs = nullptr;
+  unsigned *d_stats = nullptr;
+  double *d_scratch = nullptr;
+  float4 *d_lines = nullptr;
   double *d_out = nullptr;
   size_t in_bytes = 0, out_bytes = 0;
   // ray and reduce requests: small host tables uploaded beside the input
@@ -85,8 +89,10 @@ struct Request {
   void *d_tab = nullptr;
   double frame[9] = {};
   bool has_frame = false;
-  // a plane transform by the row-sum profiles: its entry in the batch; and whether it
-  // has to be done over by the staged kernel (its volume does not suit tables)
+  // whether it works with the slot's tables; a plane transform that does: its entry in
+  // the batch; and whether it must not (its volume does not suit tables, or it needs
+  // their memory itself)
+  bool tables = false;
   int wild_at = -1;
   bool staged = false;
 };
@@ -118,6 +124,10 @@ struct wrt_server {
   std::deque<Slot *> inflight;
   std::thread dispatcher, completer;
   cudaStream_t copy_stream = nullptr;
+  // working memory of the row-sum profiles and merged backprojections: of each slot, in
+  // the arena (0: none), and whether a request that needs the room has it
+  size_t table_bytes = 0;
+  bool tables_given = false;
   bool stop = false;
   uint64_t next_id = 1, use_clock = 0;
   wrt_server_stats stats = {};
@@ -134,22 +144,43 @@ size_t forward_pitch(int n) { return (size_t)n + (n & 1); }
 
 size_t ray_table_len(const wrt_request &r) { return (size_t)r.nshift + 4 * (size_t)r.nphi; }
 
-size_t request_bytes(const wrt_request &r) {
+// The parts of a request's block, one behind the other.  tables: by the row-sum
+// profiles or merged splines, which need no layer pairs, spline scratch or lines.
+struct Parts {
+  size_t in = 0, pairs = 0, stats = 0, tab = 0, scratch = 0, lines = 0, out = 0;
+  size_t bytes() const { return in + pairs + stats + tab + scratch + lines + out; }
+};
+Parts parts_of(const wrt_request &r, bool tables) {
   const size_t nplanes = (size_t)r.nphi * r.ntheta * r.nshift;
   const size_t n = (size_t)r.ngrid;
-  const size_t vol_state = al(4 * n * n * n) + al(8 * (n - 1) * n * forward_pitch((int)n)) + al(8);
-  if (r.op == WRT_OP_FORWARD) return vol_state + al(8 * nplanes);
-  if (r.op == WRT_OP_RAY)
-    return vol_state + al(8 * ray_table_len(r)) +
-           al(8 * (size_t)r.nslices * r.nshift * r.nphi);
-  if (r.op == WRT_OP_REDUCE) {
+  Parts p;
+  if (r.op == WRT_OP_FORWARD || r.op == WRT_OP_RAY) {
+    p.in = al(4 * n * n * n);
+    p.stats = al(8);
+    if (r.op == WRT_OP_FORWARD) {
+      if (!tables) p.pairs = al(8 * (n - 1) * n * forward_pitch((int)n));
+      p.out = al(8 * nplanes);
+    } else {
+      p.tab = al(8 * ray_table_len(r));
+      p.out = al(8 * (size_t)r.nslices * r.nshift * r.nphi);
+    }
+  } else if (r.op == WRT_OP_REDUCE) {
     const size_t nlines = n * r.nphi, nsr = (size_t)r.nshift_ray;
-    return al(8 * nlines * nsr) + al(16 * nsr) + al(8 * nlines * nsr) +
-           al(16 * nlines * (nsr - 1)) + al(8 * nplanes);
+    p.in = al(8 * nlines * nsr);
+    p.tab = al(16 * nsr);
+    p.scratch = al(8 * nlines * nsr);
+    p.lines = al(16 * nlines * (nsr - 1));
+    p.out = al(8 * nplanes);
+  } else {
+    const size_t ndir = (size_t)r.nphi * r.ntheta;
+    p.in = al(8 * nplanes);
+    if (!tables) {
+      p.scratch = al(8 * ndir * r.nshift);
+      p.lines = al(16 * ndir * (r.nshift - 1));
+    }
+    p.out = al(8 * n * n * n);
   }
-  const size_t ndir = (size_t)r.nphi * r.ntheta;
-  return al(8 * nplanes) + al(8 * ndir * r.nshift) + al(16 * ndir * (r.nshift - 1)) +
-         al(8 * n * n * n);
+  return p;
 }
 
 size_t grid_bytes(int nphi, int ntheta, int nshift) {
@@ -258,13 +289,69 @@ GridTables *acquire_grid(wrt_server *s, const wrt_request &r, int *status) {
   return &it->second;
 }
 
+wrt::ProfReq table_request(const wrt_request &r) {  // its sizes
+  wrt::ProfReq p = {};
+  p.n = r.ngrid;
+  p.L = r.half_extent ? r.half_extent : 2 * r.ngrid;
+  p.nphi = r.nphi;
+  p.ntheta = r.ntheta;
+  p.nshift = r.nshift;
+  p.storage = WRT_STORAGE_F32;
+  p.paired = wrt::profile_paired(r.ngrid, r.nphi, p.L);
+  return p;
+}
+
+// Whether a request works with a slot's tables: by its sizes and the server's alone, so
+// that its result does not depend on what else is running.
+bool suits_tables(const wrt_server *s, const wrt_request &r) {
+  if (!s->table_bytes) return false;
+  if (r.op == WRT_OP_FORWARD)
+    return wrt::profile_route(s->ctx, r.ngrid, r.nphi, r.ntheta, r.nshift) &&
+           s->table_bytes >= wrt::profile_workspace_least(table_request(r), 3.0f + 1e-5f);
+  return r.op == WRT_OP_ADJOINT && wrt::backproj_covers(r.nphi, r.ntheta, r.nshift, r.ngrid) &&
+         s->table_bytes >= wrt::backproj_workspace(r.nphi, r.ntheta, r.nshift, r.ngrid, true);
+}
+
+// Whether a request has no room beside the tables of all slots.
+bool needs_tables_room(const wrt_server *s, const Request *q) {
+  const wrt_request &r = q->req;
+  const size_t need = parts_of(r, !q->staged && suits_tables(s, r)).bytes() +
+                      (r.op == WRT_OP_RAY ? 0 : grid_bytes(r.nphi, r.ntheta, r.nshift));
+  return need > s->arena.capacity() - s->slots.size() * s->table_bytes;
+}
+
+// The slots' tables, blocks of the arena; nothing is in flight.  Caller holds s->mu.
+void give_tables(wrt_server *s) {
+  for (auto &sl : s->slots) {
+    if (sl->batch.prof_ws) s->arena.release(static_cast<char *>(sl->batch.prof_ws) - s->arena_base);
+    sl->batch.prof_ws = nullptr;
+    sl->batch.prof_bytes = 0;
+  }
+  s->tables_given = true;
+}
+bool take_tables(wrt_server *s) {
+  evict_unused_grids(s);
+  for (auto &sl : s->slots) {
+    size_t off = 0;
+    if (!s->arena.alloc(s->table_bytes, &off)) {
+      give_tables(s);
+      return false;
+    }
+    sl->batch.prof_ws = s->arena_base + off;
+    sl->batch.prof_bytes = s->table_bytes;
+  }
+  s->tables_given = false;
+  return true;
+}
+
 // Reserves a request's state in the arena.  Caller holds s->mu.
 bool reserve(wrt_server *s, Request *q, int *status) {
   *status = WRT_OK;
   const bool needs_grid = q->req.op != WRT_OP_RAY;
   GridTables *g = needs_grid ? acquire_grid(s, q->req, status) : nullptr;
   if (needs_grid && !g) return false;
-  const size_t bytes = request_bytes(q->req);
+  const Parts parts = parts_of(q->req, q->tables);
+  const size_t bytes = parts.bytes();
   size_t off = 0;
   if (!s->arena.alloc(bytes, &off)) {
     if (g) g->refs--;
@@ -284,37 +371,34 @@ bool reserve(wrt_server *s, Request *q, int *status) {
   const size_t nplanes = (size_t)r.nphi * r.ntheta * r.nshift;
   const size_t n = (size_t)r.ngrid;
   char *b = s->arena_base + off;
-  const size_t vol_state = al(4 * n * n * n) + al(8 * (n - 1) * n * forward_pitch((int)n)) + al(8);
+  auto place = [&](size_t part) {
+    char *at = part ? b : nullptr;
+    b += part;
+    return at;
+  };
+  q->d_in = place(parts.in);
+  q->d_pairs = reinterpret_cast<float2 *>(place(parts.pairs));
+  q->d_stats = reinterpret_cast<unsigned *>(place(parts.stats));
+  q->d_tab = place(parts.tab);
+  q->d_scratch = reinterpret_cast<double *>(place(parts.scratch));
+  q->d_lines = reinterpret_cast<float4 *>(place(parts.lines));
+  q->d_out = reinterpret_cast<double *>(place(parts.out));
+  q->out_bytes = 8 * nplanes;
   if (r.op == WRT_OP_FORWARD) {
-    q->d_in = b;  // volume, then pairs, stats, output
     q->in_bytes = 4 * n * n * n;
-    q->out_bytes = 8 * nplanes;
-    q->d_out = reinterpret_cast<double *>(b + vol_state);
   } else if (r.op == WRT_OP_RAY) {
-    q->d_in = b;  // volume, then pairs, stats, tables, output
     q->in_bytes = 4 * n * n * n;
-    q->d_tab = b + vol_state;
     q->tab.resize(ray_table_len(r));
     wrt::ray_tables(r.nshift, r.nphi, q->tab.data());
     q->out_bytes = 8 * (size_t)r.nslices * r.nshift * r.nphi;
-    q->d_out = reinterpret_cast<double *>(b + vol_state + al(8 * ray_table_len(r)));
   } else if (r.op == WRT_OP_REDUCE) {
-    const size_t nlines = n * r.nphi, nsr = (size_t)r.nshift_ray;
-    q->d_in = b;  // ray data, then spline coefficients, scratch, lines, output
-    q->in_bytes = 8 * nlines * nsr;
-    q->d_tab = b + al(8 * nlines * nsr);
+    const size_t nsr = (size_t)r.nshift_ray;
+    q->in_bytes = 8 * n * r.nphi * nsr;
     q->tab.resize(2 * nsr);
     wrt::spline_coefficients((int)nsr, q->tab.data(), q->tab.data() + nsr);
-    q->out_bytes = 8 * nplanes;
-    q->d_out = reinterpret_cast<double *>(b + al(8 * nlines * nsr) + al(16 * nsr) +
-                                          al(8 * nlines * nsr) + al(16 * nlines * (nsr - 1)));
   } else {
-    const size_t ndir = (size_t)r.nphi * r.ntheta;
-    q->d_in = b;  // radon data, then spline scratch, lines, output
     q->in_bytes = 8 * nplanes;
     q->out_bytes = 8 * n * n * n;
-    q->d_out = reinterpret_cast<double *>(b + al(8 * nplanes) + al(8 * ndir * r.nshift) +
-                                          al(16 * ndir * (r.nshift - 1)));
   }
   return true;
 }
@@ -345,18 +429,14 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
   if (r.op == WRT_OP_RAY) {
     // the volume's statistics come from the batch's volume kernel through a
     // forward entry with no planes and no work items
-    const size_t nn = (size_t)n;
     float *vol = reinterpret_cast<float *>(base);
-    float2 *pairs = reinterpret_cast<float2 *>(base + al(4 * nn * nn * nn));
-    unsigned int *stats = reinterpret_cast<unsigned int *>(
-        base + al(4 * nn * nn * nn) + al(8 * (nn - 1) * nn * forward_pitch(n)));
     wrt::StagedReq sr;
-    wrt::staged_request(n, (int)forward_pitch(n), 0, 0, 2 * n, WRT_STORAGE_F32, pairs, vol,
+    wrt::staged_request(n, (int)forward_pitch(n), 0, 0, 2 * n, WRT_STORAGE_F32, nullptr, vol,
                         nullptr, nullptr, nullptr, nullptr, nullptr, &sr);
     wrt::FwdAux a = {};
     a.vol = vol;
     a.pairs = nullptr;
-    a.stats = stats;
+    a.stats = q->d_stats;
     a.nout = 0;
     a.n = n;
     a.pitch = (int)forward_pitch(n);
@@ -374,69 +454,52 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
     job.trig = static_cast<const double *>(q->d_tab) + r.nshift;
     job.has_frame = q->has_frame ? 1 : 0;
     for (int k = 0; k < 9; ++k) job.frame[k] = q->frame[k];
-    job.r2bits = stats;
+    job.r2bits = q->d_stats;
     job.margin = wrt::trilinear_margin(n);
     job.out = q->d_out;
     (q->has_frame ? b.ray : b.slices).push_back(job);
     return;
   }
   if (r.op == WRT_OP_REDUCE) {
-    const size_t nlines = (size_t)n * r.nphi, nsr = (size_t)r.nshift_ray;
     wrt::RedReq rq = {};
     rq.rays = reinterpret_cast<const double *>(base);
     rq.coef = static_cast<const double *>(q->d_tab);
-    rq.scratch = reinterpret_cast<double *>(base + al(8 * nlines * nsr) + al(16 * nsr));
-    rq.lines = reinterpret_cast<float4 *>(base + al(8 * nlines * nsr) + al(16 * nsr) +
-                                          al(8 * nlines * nsr));
+    rq.scratch = q->d_scratch;
+    rq.lines = q->d_lines;
     rq.shift = g->shift;
     rq.cs = g->cs;
     rq.out = q->d_out;
     rq.ngrid = n;
-    rq.ns_ray = (int)nsr;
+    rq.ns_ray = r.nshift_ray;
     rq.nphi = r.nphi;
     rq.nshift = r.nshift;
     rq.ntheta = r.ntheta;
-    (wrt::reduction_covers(n, (int)nsr) ? b.staged_red : b.red).push_back(rq);
+    (wrt::reduction_covers(n, r.nshift_ray) ? b.staged_red : b.red).push_back(rq);
     return;
   }
   if (r.op == WRT_OP_FORWARD) {
-    const size_t nn = (size_t)n;
     float *vol = reinterpret_cast<float *>(base);
-    float2 *pairs = reinterpret_cast<float2 *>(base + al(4 * nn * nn * nn));
-    unsigned int *stats = reinterpret_cast<unsigned int *>(
-        base + al(4 * nn * nn * nn) + al(8 * (nn - 1) * nn * forward_pitch(n)));
     const int L = r.half_extent ? r.half_extent : 2 * n;
     wrt::StagedReq sr;
-    wrt::staged_request(n, (int)forward_pitch(n), ndir, r.nshift, L, WRT_STORAGE_F32, pairs,
-                        vol, g->dir, g->dir32, g->shift, g->shift32, q->d_out, &sr);
+    wrt::staged_request(n, (int)forward_pitch(n), ndir, r.nshift, L, WRT_STORAGE_F32,
+                        q->d_pairs, vol, g->dir, g->dir32, g->shift, g->shift32, q->d_out, &sr);
     wrt::FwdAux a = {};
     a.vol = vol;
-    a.pairs = pairs;
-    a.stats = stats;
+    a.pairs = q->d_pairs;
+    a.stats = q->d_stats;
     a.nout = (long long)ndir * r.nshift;
     a.n = n;
     a.pitch = (int)forward_pitch(n);
     a.L = L;
     a.prep = 1;
-    // the row-sum profiles, where they cover the request and the slot has
-    // their working memory (decided by sizes alone: a request's result does not
-    // depend on what else is running)
-    wrt::ProfReq p = {};
-    p.vol = vol;
-    p.dir = g->dir;
-    p.shift = g->shift;
-    p.stats = stats;
-    p.out = q->d_out;
-    p.n = n;
-    p.L = L;
-    p.nphi = r.nphi;
-    p.ntheta = r.ntheta;
-    p.nshift = r.nshift;
-    p.storage = WRT_STORAGE_F32;
-    p.paired = wrt::profile_paired(n, r.nphi, L);
     q->wild_at = -1;
-    if (!q->staged && wrt::profile_route(s->ctx, n, r.nphi, r.ntheta, r.nshift) &&
-        slot.prof_bytes >= wrt::profile_workspace_least(p, 3.0f + 1e-5f)) {
+    if (q->tables) {
+      wrt::ProfReq p = table_request(r);
+      p.vol = vol;
+      p.dir = g->dir;
+      p.shift = g->shift;
+      p.stats = q->d_stats;
+      p.out = q->d_out;
       a.pairs = nullptr;
       a.nout = 0;
       sr.nshift = sr.ndir = 0;
@@ -449,9 +512,7 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
     }
     wrt::batch_add_forward(b, sr, a, 3.0f + 1e-5f);
   } else {
-    const size_t nplanes = (size_t)ndir * r.nshift;
-    if (wrt::backproj_covers(r.nphi, r.ntheta, r.nshift, n) &&
-        slot.prof_bytes >= wrt::backproj_workspace(r.nphi, r.ntheta, r.nshift, n, true)) {
+    if (q->tables) {
       wrt::BackReq q2 = {};
       q2.radon = reinterpret_cast<const double *>(base);
       q2.cs = g->cs;
@@ -468,8 +529,8 @@ void add_to_batch(wrt_server *s, Request *q, const wrt::BatchSlot &slot, wrt::Ba
     }
     wrt::AdjReq j = {};
     j.radon = reinterpret_cast<const double *>(base);
-    j.scratch = reinterpret_cast<double *>(base + al(8 * nplanes));
-    j.lines = reinterpret_cast<float4 *>(base + al(8 * nplanes) + al(8 * (size_t)ndir * r.nshift));
+    j.scratch = q->d_scratch;
+    j.lines = q->d_lines;
     j.out = q->d_out;
     j.dirw = g->dirw;
     j.h_dirw = g->h_dirw.data();
@@ -524,7 +585,21 @@ void dispatch_loop(wrt_server *s) {
           (op == WRT_OP_REDUCE && nred >= wrt::kBatchMaxRed))
         break;
       int st = WRT_OK;
-      if (!reserve(s, q, &st)) {
+      // a request that has no room beside the tables has their memory, and the device, to
+      // itself, and works without them
+      const bool alone = s->table_bytes && needs_tables_room(s, q);
+      if (alone || s->tables_given) {
+        if (!batch.empty() || !s->inflight.empty()) break;
+        if (alone) {
+          evict_unused_grids(s);
+          if (!s->tables_given) give_tables(s);
+          q->staged = true;
+        } else if (!take_tables(s)) {
+          st = WRT_ERR_INTERNAL;  // (an empty arena has room for them)
+        }
+      }
+      q->tables = !q->staged && suits_tables(s, q->req);
+      if (st || !reserve(s, q, &st)) {
         if (st == WRT_OK && (!batch.empty() || !s->inflight.empty())) break;  // wait for memory
         s->arrivals.pop_front();
         finish(s, q, st ? st : WRT_ERR_BUDGET, s->now_ms());
@@ -536,6 +611,7 @@ void dispatch_loop(wrt_server *s) {
       if (op == WRT_OP_RAY) ++nray;
       if (op == WRT_OP_REDUCE) ++nred;
       batch.push_back(q);
+      if (alone) break;
     }
     if (batch.empty()) {
       s->cv.notify_all();  // failed requests wake their waiters
@@ -695,6 +771,15 @@ int wrt_server_create(const wrt_server_opts *opts, wrt_server **out) {
   s->stats.budget = budget;
   st = cudaStreamCreateWithFlags(&s->copy_stream, cudaStreamNonBlocking) == cudaSuccess
            ? WRT_OK : WRT_ERR_CUDA;
+  // working memory of the row-sum profiles and merged backprojections, for each slot the
+  // same (a request's kernel must not depend on the slot it gets): an eighth of the budget,
+  // with many slots less, so that half the budget is left, at most kServerProfBytes; with
+  // little (small budgets) the requests take the staged and direct kernels.  The host does
+  // not know a volume's support, so units have room for all of the cube and fewer fit a
+  // step (128^3, 64 x 128 x 256, ten requests at once: 13.5 ms each with 256 MB a
+  // slot, 9.4 with 512, 7.6 with 1 GB, 7.0 with 1.5, 6.7 with 3)
+  size_t table_bytes = std::min({budget / 8, budget / 2 / o.max_inflight, kServerProfBytes});
+  table_bytes = table_bytes >= kServerProfLeast ? table_bytes & ~(size_t)0xffff : 0;
   for (int k = 0; k < o.max_inflight && !st; ++k) {
     auto sl = std::make_unique<Slot>();
     if (cudaStreamCreateWithFlags(&sl->stream, cudaStreamNonBlocking) != cudaSuccess ||
@@ -703,17 +788,7 @@ int wrt_server_create(const wrt_server_opts *opts, wrt_server **out) {
       break;
     }
     st = wrt::batch_slot_init(ctx, &sl->batch, sl->stream);
-    // working memory of the row-sum profiles, beside the arena: an eighth of
-    // the budget per slot, at most kServerProfBytes; without it (small budgets,
-    // no memory left) the plane transforms take the staged kernel.  The host does not
-    // know a volume's support, so units have room for all of the cube and fewer fit a
-    // step (128^3, 64 x 128 x 256, ten requests at once: 13.5 ms each with 256 MB a
-    // slot, 9.4 with 512, 7.6 with 1 GB, 7.0 with 1.5, 6.7 with 3)
-    const size_t want = std::min(budget / 8, kServerProfBytes) & ~(size_t)0xffff;
-    if (!st && want >= kServerProfLeast &&
-        wrt::ctx_alloc(ctx, &sl->batch.prof_ws, want) == WRT_OK)
-      sl->batch.prof_bytes = want;
-    if (sl->batch.prof_bytes) {
+    if (!st && table_bytes) {
       st = wrt::ctx_alloc(ctx, (void **)&sl->batch.d_wild, sizeof(unsigned) * wrt::kBatchMaxFwd);
       if (!st && cudaMallocHost((void **)&sl->batch.h_wild,
                                 sizeof(unsigned) * wrt::kBatchMaxFwd) != cudaSuccess) {
@@ -723,15 +798,8 @@ int wrt_server_create(const wrt_server_opts *opts, wrt_server **out) {
     }
     s->slots.push_back(std::move(sl));
   }
-  // every slot or none: a request's kernel must not depend on the slot it gets
-  bool every = true;
-  for (auto &sl : s->slots) every = every && sl->batch.prof_bytes > 0;
-  if (!every)
-    for (auto &sl : s->slots) {
-      wrt::ctx_free(ctx, sl->batch.prof_ws, sl->batch.prof_bytes);
-      sl->batch.prof_ws = nullptr;
-      sl->batch.prof_bytes = 0;
-    }
+  s->table_bytes = table_bytes;
+  if (!st && table_bytes && !take_tables(s)) st = WRT_ERR_INTERNAL;
   if (st) {
     s->stop = true;
     wrt_server_destroy(s);
@@ -767,8 +835,11 @@ int wrt_server_submit(wrt_server *s, const wrt_request *r, uint64_t *id) {
   } else {
     if (!r->radon || r->ngrid < 1 || r->ngrid > 2048 || r->nshift < 3) return WRT_ERR_INVALID_ARGUMENT;
   }
-  const size_t need = request_bytes(*r) +
-                      (r->op == WRT_OP_RAY ? 0 : grid_bytes(r->nphi, r->ntheta, r->nshift));
+  // (rays need no layer pairs; what is accepted does not hang on it)
+  const size_t nr = (size_t)r->ngrid;
+  const size_t need = parts_of(*r, false).bytes() +
+                      (r->op == WRT_OP_RAY ? al(8 * (nr - 1) * nr * forward_pitch(r->ngrid))
+                                           : grid_bytes(r->nphi, r->ntheta, r->nshift));
   auto q = std::make_unique<Request>();
   q->req = *r;
   if (r->op == WRT_OP_RAY && r->frame && !wrt::identity_frame(r->frame)) {
