@@ -271,12 +271,13 @@ def timed_device_calls(ctx, call, steps, warmup):
     return times
 
 
-def other_paths(wrt, ctx, phantom, steps, warmup, smem_bw, with_cpu):
+def other_paths(wrt, ctx, phantom, steps, warmup, smem_bw, hbm_peak, with_cpu):
     """The ray transform (reference frame and one rotated frame), the
     reduction of ray data to Radon data, and the backprojection, at 128^3,
     through their device-resident entry points: device time per call, units/s,
-    the gather roofline of the dominant kernel (bytes per counted unit against
-    the measured shared-memory/L1 bandwidth) and, in the CPU leg, the
+    a roofline -- where every counted sample is read on its own, its bytes against
+    the measured shared-memory/L1 bandwidth; where samples share what is read, the
+    compulsory HBM bytes, with the samples' figure beside it -- and, in the CPU leg, the
     reference's own code on a bounded seeded sample of the same units, timed
     on the host cores and compared with the GPU's values there."""
     n = N
@@ -299,16 +300,25 @@ def other_paths(wrt, ctx, phantom, steps, warmup, smem_bw, with_cpu):
         ctx.count_samples(False)
         return c
 
-    def entry(name, call, units, unit, bytes_per_sample, samples, sample_unit, download):
+    def entry(name, call, units, unit, bytes_per_sample, samples, sample_unit, download,
+              shared_hbm=None):
         times = timed_device_calls(ctx, call, steps, warmup)
         ms = statistics.mean(times)
-        achieved = samples * bytes_per_sample / (ms * 1e-3) / 1e9
+        gather = {"achieved": samples * bytes_per_sample / (ms * 1e-3) / 1e9, "peak": smem_bw / 1e9,
+                  "unit": "GB/s", "algorithmic_bytes": f"{bytes_per_sample} B per {sample_unit}",
+                  "samples_per_call": samples}
+        if shared_hbm is None:
+            roof = {"bound": "l1tex", **gather, "frac": gather["achieved"] / gather["peak"]}
+        else:
+            achieved = shared_hbm / (ms * 1e-3) / 1e9
+            roof = {"bound": "latency", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
+                    "frac": achieved / hbm_peak,
+                    "note": "compulsory HBM bytes (inputs once, results once)",
+                    "samples": {**gather, "note": "what reading every sample on its own would take; "
+                                                  "samples share what is read, so no roofline"}}
         res[name] = {"value": units / (ms * 1e-3), "unit": unit, "ms_per_call": ms,
                      "ms_median": statistics.median(times), "gpu_launches_per_call": None,
-                     "roofline": {"bound": "l1tex", "achieved": achieved, "peak": smem_bw / 1e9,
-                                  "unit": "GB/s", "frac": achieved / (smem_bw / 1e9),
-                                  "algorithmic_bytes": f"{bytes_per_sample} B per {sample_unit}",
-                                  "samples_per_call": samples}}
+                     "roofline": roof}
         return download()
 
     ray_call = lambda fr=None: wrt.ray_forward_device(ctx, vol, RAY_SLICES, RAY_SHIFTS, RAY_PHIS,
@@ -316,7 +326,7 @@ def other_paths(wrt, ctx, phantom, steps, warmup, smem_bw, with_cpu):
     dl_rays = lambda: rays_d.download(np.empty((RAY_SLICES, RAY_SHIFTS, RAY_PHIS)))
     l0 = ctx.launches
     rays = entry("ray", ray_call, nrays, "rays/s", BYTES_PER_SAMPLE, counted(ray_call),
-                 "trilinear sample (8 FP32 corners)", dl_rays)
+                 "trilinear sample (8 FP32 corners)", dl_rays, shared_hbm=4 * n ** 3 + 8 * nrays)
     res["ray"]["gpu_launches_per_call"] = (ctx.launches - l0) // (steps + max(warmup, 3) + 1)
     rc = lambda: ray_call(frame)
     rays_rot = entry("ray_rotated", rc, nrays, "rays/s", BYTES_PER_SAMPLE, counted(rc),
@@ -325,7 +335,7 @@ def other_paths(wrt, ctx, phantom, steps, warmup, smem_bw, with_cpu):
     ray_call()
     red = lambda: wrt.radon_reduction_device(ctx, rays_d.ptr, n, RAY_SHIFTS, grid, radon_d.ptr)
     radon = entry("reduction", red, grid.nplanes, "plane integrals/s", 48, counted(red),
-                  "slice sample (3 spline records of 16 B)",
+                  "slice sample (6 shared loads of 8 B)",
                   lambda: radon_d.download(np.empty((NSHIFT, NPHI, NTHETA))))
     gauss_d = wrt.DeviceBuffer(ctx, gauss.nbytes)
     gauss_d.upload(gauss)
@@ -333,12 +343,14 @@ def other_paths(wrt, ctx, phantom, steps, warmup, smem_bw, with_cpu):
     evals = n ** 3 * NPHI * NTHETA
     adjoint = entry("adjoint", adj, n ** 3, "voxels/s", 16, evals,
                     "spline evaluation (one 16 B record)",
-                    lambda: adj_d.download(np.empty((n, n, n))))
+                    lambda: adj_d.download(np.empty((n, n, n))),
+                    shared_hbm=8 * grid.nplanes + 8 * n ** 3)
     # the reference's default sampler: nearest cell on the 4n x 4n lattice
     near = lambda: wrt.radon_forward_device(ctx, vol, grid, radon_d.ptr, sampler=wrt.NEAREST)
     nearest = entry("nearest", near, grid.nplanes, "plane integrals/s", 4, counted(near),
                     "nearest sample (one FP32 cell value)",
-                    lambda: radon_d.download(np.empty((NSHIFT, NPHI, NTHETA))))
+                    lambda: radon_d.download(np.empty((NSHIFT, NPHI, NTHETA))),
+                    shared_hbm=4 * n ** 3 + 8 * grid.nplanes)
     plain_near = lambda: wrt.radon_forward_device(ctx, vol, grid, radon_d.ptr, sampler=wrt.NEAREST,
                                                   kernel=wrt.KERNEL_PLAIN)
     pt = timed_device_calls(ctx, plain_near, 2, 1)
@@ -354,14 +366,14 @@ def other_paths(wrt, ctx, phantom, steps, warmup, smem_bw, with_cpu):
     # what binds each kernel, from its committed ncu capture (a profiler cannot
     # run inside the timed bench): the byte figure above is the algorithmic
     # gather, not always the limit
-    for k, b in (("nearest", "gathers of the row tables from L2, late blocks of dependent launches; "
-                             "samples share table entries, so the byte figure is not the limit"),
-                 ("ray", "column loads along z, shared by all slices of a (shift, angle)"),
+    cap = "(profiles/table_kernels_128cubed.md)"
+    for k, b in (("nearest", "gathers of the row tables with few warps resident, late blocks of "
+                             f"dependent launches {cap}"),
+                 ("ray", f"L1: 87 % of its throughput, column loads along z {cap}"),
                  ("ray_rotated", "L1 gathers: 82 % of L1 throughput "
                                  "(profiles/ray_kernel_128cubed.md)"),
-                 ("reduction", "shared-memory wavefronts: 90 % of the peak"),
-                 ("adjoint", "L1 tag lookups of the record gathers; evaluations share merged "
-                             "splines, so the byte figure is not the limit")):
+                 ("reduction", f"shared-memory wavefronts: 90 % of the peak {cap}"),
+                 ("adjoint", f"record gathers: L1 at 81 % on the SMs that are busy {cap}")):
         res[k]["roofline"]["limit_measured"] = b
     if with_cpu:
         import oracle as O
@@ -984,7 +996,7 @@ def run_ours(args, dist):
                                "lattice step 1/n on [-n,n)^2",
                    "n": N, "sphere_grid": [NTHETA, NPHI], "shifts": NSHIFT,
                    "planes_per_step": nplanes, "kernel": args.kernel, "tile": tile,
-                   "path": "batched persistent kernel, graph launch (wrt_radon_forward_batch)",
+                   "path": "batch entry point (wrt_radon_forward_batch): row-sum profiles",
                    "l2": "flushed before every timed step (2x L2 memset)",
                    "parallelism": f"replicas x{dist.world}"},
         "samples_per_step": samples,
@@ -1015,7 +1027,7 @@ def run_ours(args, dist):
         result["served_over_plain"] = e2e_value / plain["value"]
     if not args.no_other_paths:
         result["paths"] = other_paths(wrt, ctx, phantom, max(3, min(args.steps, 10)), args.warmup,
-                                      smem_bw, dist.rank == 0 and not args.no_cpu_baseline)
+                                      smem_bw, hbm_peak, dist.rank == 0 and not args.no_cpu_baseline)
         result["batch_vs_one_per_launch"] = batch_vs_one_per_launch(wrt, ctx, 3)
         result["batch_vs_one_per_launch_small"] = batch_vs_one_per_launch(
             wrt, ctx, 3, count=256, edges=(16, 24, 32, 48), lat=(8, 17), shifts=(32, 65),
