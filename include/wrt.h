@@ -62,8 +62,10 @@ typedef enum wrt_kernel {
                             else the plain one */
   WRT_KERNEL_PLAIN = 1,  /* one warp per plane, gathers through L1 */
   WRT_KERNEL_STAGED = 2  /* the row-sum profiles where they cover and suit the request
-                            (working memory of up to 3 GB in the context, less
-                            where its budget or the device has less), else
+                            (working memory of up to 3 GB in the context, for
+                            the nearest sampler up to 3.5, less where its budget
+                            or the device has less; values that are no numbers do
+                            not suit them), else
                             volume layers staged in shared memory, persistent CTAs:
                             trilinear from the layer pairs (FP32 or BF16 storage),
                             nearest from the z-major cell layers (FP32 storage) */
@@ -273,8 +275,12 @@ int wrt_radon_reduction_device(wrt_ctx *ctx, const double *dev_rays, int ngrid, 
 
 /* Backprojection of device Radon data dev_radon[is][iphi][itheta] on a
  * resident sphere grid into dev_out, ngrid^3 doubles [iz][ix][iy].
- * Asynchronous; spline working memory lives in the context.  Device-resident
- * form of backprojection/C/src/radon3d_ajoint.c:221-260 with radon3d_adjoint
+ * Asynchronous; working memory lives in the context: with more than 262,144
+ * data half as much again as the data (odd nphi: three times), lists of every
+ * z plane and up to 768 MB of tables, less where the budget or the device has
+ * less; the direct kernel's three times the data where that does not fit or the
+ * data are few.  Device-resident form of
+ * backprojection/C/src/radon3d_ajoint.c:221-260 with radon3d_adjoint
  * (integral.c:6-24). */
 int wrt_radon3d_adjoint_device(wrt_ctx *ctx, const double *dev_radon, const wrt_grid *grid,
                                int ngrid, double *dev_out);

@@ -34,8 +34,9 @@
 // direct kernel (k_spline.cu).  That kernel stays for small direction sets and
 // for what has no working memory.
 //
-// What bounds it: the gather's L1 tag lookups (32 lanes, 32 lines, 32 cycles per
-// request: 0.5 ms of the 128^3 case if every SM were busy), the build's latency.
+// What bounds it: the gather's record loads (one line per lane; L1 at 81 % of its
+// throughput on the SMs that a launch keeps busy, more than half of a warp's cycles spent
+// waiting), the build's latency.
 // 128^3 from 64 x 128 directions x 256 shifts: 15.9 ms by the direct kernel (16
 // bytes and ~7 instructions per voxel and direction), 1.77 here; 256^3 from 96 x
 // 192 x 384: 237 and 20 ms; error against FP64 (128^3) 6.5e-9 and 4.8e-9.

@@ -38,12 +38,13 @@
 // alone or in any batch.
 //
 // What bounds it: nothing close to a byte or flop limit any more; the rows
-// launch waits for its gathers (random 32-byte reads, mostly from L2) and FP64
-// geometry, the build for its node loads.  128^3, 64 x 128 directions x 256
+// launch waits for its gathers (random 32-byte reads, mostly from L2: half of a warp's
+// cycles, with 22 % of the warps resident; FP64 7 % busy, DRAM 7 %), the build for its
+// node loads and its chain of sums.  128^3, 64 x 128 directions x 256
 // shifts, lattice [-n, n)^2: 53.7 ms by the staged kernel (lattice samples
-// through shared memory), 4.6-4.9 ms here; 256^3 BF16, 96 x 192 x 384: 750 and 44
-// ms; error against FP64 6.5e-8 (staged 8.9e-8).  Small requests wait for the four
-// launches one after another (24^3, 8 x 16 x 32: 109 and 80 us).
+// through shared memory), 5.0 ms here; 256^3 BF16, 96 x 192 x 384: 750 and 45
+// ms; error against FP64 (doubles, 96^3) 8e-9 (staged 5.1e-8).  Small requests wait for
+// the four launches one after another (24^3, 8 x 16 x 32: 109 and 82 us).
 #include <math.h>
 #include <string.h>
 
@@ -1368,7 +1369,11 @@ bool profile_covers(int n, int nphi, int ntheta, int nshift) {
 // 8 .. 256 shifts, 4000 planes up): 0.93 of its speed at worst, 1.05-2.5 times within a
 // fifth of the line, 2-4 times at twice; just below it 0.5-1.3 times for n > 100, up
 // to 2.5 for n < 60.  Nearest on 86 sizes past the line: 1.03 at worst, 1.3-9 as a
-// rule.  Below 4000 planes both are launches: 0.7-1.6 times.
+// rule.  Below 4000 planes both are launches; staged and tables by the number of planes,
+// trilinear, sizes past the line above: 2000 planes 20^3 66 and 75 us, 24^3 60 and 94;
+// 3000: 24^3 94 and 96, 32^3 87 and 100, 40^3 132 and 136; 4000: 24^3 129 and 80, 32^3 124
+// and 108, 40^3 115 and 128, 48^3 183 and 177; 5000: 155 and 123 (40^3), 155 and 147 (48^3);
+// 10,000: 276 and 93 (32^3), 366 and 187 (64^3).  (Nearest is ahead from 1000 planes up.)
 bool profile_route(const wrt_ctx *ctx, int n, int nphi, int ntheta, int nshift) {
   if (!profile_covers(n, nphi, ntheta, nshift)) return false;
   if (ctx->staged_config >= 0) return ctx->staged_config == kNumStagedConfigs - 1;

@@ -24,8 +24,9 @@
 //
 // 128 layers x 128 offsets, 64 x 128 directions x 256 shifts: 2.37 ms with three
 // 16-byte records per sample gathered through L1 (one request of up to 32 lines
-// each), 1.10 ms here (1.03 of it this kernel, at 90 % of the shared-memory
-// wavefronts; 1.45 with an odd pitch, 1.11 with every lane at its own line's start).
+// each), 1.12 ms here (1.04 of it this kernel, at 90 % of the shared-memory
+// wavefronts; 1.45 with an odd pitch; every lane at its own line's start: no faster).
+// Error against FP64 (doubles, 64 layers x 40 offsets) 7.5e-9, by records 1.2e-8.
 #include <algorithm>
 #include <vector>
 

@@ -3,8 +3,8 @@
 // The reference answers one request per process run (a CLI invocation that
 // reads text, transforms, writes text).  A wrt_server instead keeps a device
 // context, the sphere-grid tables of the shapes it has seen and one arena of
-// device memory (its HBM budget, reserved at start-up) resident, and runs two
-// threads:
+// device memory (its HBM budget, reserved at start-up; the launch slots' working
+// tables are blocks of it) resident, and runs two threads:
 //
 //   dispatcher  admits queued requests in arrival order while a launch slot is
 //               free and the arena has room for their state, uploads their
@@ -19,8 +19,9 @@
 // GPU are admitted as slots and memory free up, and consecutive launches
 // overlap on the device (the next graph's kernels start on SMs the previous
 // persistent kernel has left).  A request's result does not depend on its
-// batch: the plane sums are order-independent fixed-point integers and a
-// voxel's backprojection is one thread's sequential sum.
+// batch: its kernel follows from its sizes, the plane sums are order-independent
+// fixed-point integers or sums in an order that the sizes fix, and a voxel's
+// backprojection is one thread's sequential sum.
 #include <math.h>
 #include <string.h>
 
