@@ -367,6 +367,9 @@ __device__ __noinline__ double edge_terms(const BackStep &s, int zi, const unsig
     if (!id) continue;
     const int th = (int)((id - 1u) / ns), i = (int)((id - 1u) % ns);
     if (i != 0 && i != ns - 1) continue;
+    bool lost = false;  // not in the table
+    for (int k = r.lost[0]; k > 0; --k) lost |= r.lost[k] == th * r.nbase + b;
+    if (lost) continue;
     const bool model = (i == 0) == (pos[q] <= fx);
     for (int k = 0; k < (r.paired ? 2 : 1); ++k) {
       const int ph = b + k * r.nbase, t = k ? r.ntheta - 1 - th : th, j = k ? ns - 1 - i : i;
