@@ -768,6 +768,7 @@ int tables_get(wrt_ctx *ctx, size_t want, size_t least, void **ws, size_t *bytes
   }
   auto half = [&] { return std::max(want / 2 & ~(size_t)0xffff, least); };
   while (want > least && want > have && ws_rounded(want) > room) want = half();
+  if (want > have && ws_rounded(want) > room) return WRT_ERR_BUDGET;  // a smaller buffer stays
   int st = ws_get(ctx, WS_PROFILE, want, ws);
   while (st && want > least) {
     ctx->tables_refused = std::min(ctx->tables_refused, want);
